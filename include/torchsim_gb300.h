@@ -494,6 +494,14 @@ int tsg_gn_evaluate(const tsg_program* program, const tsg_tissue* tissue, int64_
                     int64_t state_count, const void* measured, const int64_t* measured_rows,
                     double* normal_equations, const tsg_launch* launch, void* stream);
 
+/* The launch shape tsg_gn_evaluate picks by itself for this many voxels of a
+ * plain recorded train (zeros: the general sweep's own choice). A solve asks
+ * once, at its first iteration, and passes the shape from then on: the order
+ * in which a voxel's samples are summed depends on the shape, and a solve
+ * whose pool shrinks should not change it on the way. */
+int tsg_gn_shape(const tsg_program* program, int64_t atom_count, int64_t state_count,
+                 tsg_launch* shape);
+
 enum { TSG_GN_FIRST = 0, TSG_GN_LIVE = 1, TSG_GN_DONE = 2 };
 
 /* Device-resident per-voxel Levenberg-Marquardt state (all DEVICE arrays of

@@ -147,6 +147,7 @@ SIGNATURES: dict[str, tuple] = {
                                        _int, _int, _vp]),
     "tsg_gn_evaluate": (_int, [_vp, ctypes.POINTER(Tissue), _i64, _i64, _vp, _vp, _vp,
                                ctypes.POINTER(Launch), _vp]),
+    "tsg_gn_shape": (_int, [_vp, _i64, _i64, ctypes.POINTER(Launch)]),
     "tsg_gn_step": (_int, [ctypes.POINTER(GNState), _i64, ctypes.POINTER(GNConfig), _vp]),
     "tsg_gn_judge": (_int, [ctypes.POINTER(GNState), _i64, ctypes.POINTER(GNConfig), _vp]),
     "tsg_gn_natural": (_int, [_vp, _i64, ctypes.POINTER(GNConfig), _vp, _vp]),

@@ -29,6 +29,17 @@ Table table_for(int mode) {
     return {nullptr, 0};
 }
 
+Table train_table_for(int mode) {
+    switch (mode) {
+        case MODE_FORWARD: return {kTrainForward, kTrainForwardCount};
+        case MODE_T12: return {kTrainT12, kTrainT12Count};
+        case MODE_T12B: return {kTrainT12B, kTrainT12BCount};
+        case MODE_T12BI: return {kTrainT12BI, kTrainT12BICount};
+        case MODE_GN: return {kTrainGN, kTrainGNCount};
+    }
+    return {nullptr, 0};
+}
+
 int sm_count() {
     static int count = [] {
         int dev = 0, n = 0;
@@ -106,6 +117,91 @@ const SweepEntry* choose(int mode, int states, int64_t work_items, const tsg_lau
     return best;
 }
 
+// Which shape of the recorded-train sweep runs: the first rule of the mode
+// whose states and voxel count (times trains) are above the call's. Few voxels
+// take many lanes each, since then the dependency chain of one op sets the
+// time and a lane's share of the orders is on it; many voxels take few lanes,
+// since every lane repeats an op's coefficient loads, record and shuffles. An
+// exact fit (lanes x orders = states) saves the truncation's selects. The
+// lines are where the two neighbours' times crossed on a GB300 (500 pulses;
+// us at the left shape / the right shape):
+//   forward 10 states:  8,192 (10,2) 84 / (5,2) 86; 24,576 (5,2) 177 / (1,10) 148
+//   forward 20 states: 16,384 (10,2) 135 / (5,4) 132; 24,576 (5,4) 182 / (2,10) 179;
+//                      65,536 (2,10) 367 / (1,20) 340
+//   forward 32 states:  8,192 (8,4) 97 / (4,8) 101; 65,536 (4,8) 476 / (1,32) 488
+//   T1, T2  10 states:  2,048 (10,2) 88 / (5,2) 92; 32,768 (5,2) 375 / (1,10) 352
+//   T1, T2  32 states: 32,768 (8,4) 664 / (4,8) 627, at 27 states 709 / 756
+//   T1, T2, B1  20 states: 8,192 (10,2) 212 / (5,4) 229; 24,576 534 / 485
+//   Gauss-Newton 10 states, 880 pulses: 4,096 (5,2) 158 / (1,10) 300;
+//                      16,384 (5,2) 378 / (1,10) 344
+struct TrainRule {
+    int mode, states, lanes, orders;
+    int64_t below;  // voxels x trains
+};
+constexpr int64_t kAny = INT64_MAX;
+const TrainRule kTrainRules[] = {
+    {MODE_FORWARD, 10, 10, 2, 8192},   {MODE_FORWARD, 10, 5, 2, 20480},
+    {MODE_FORWARD, 10, 1, 10, kAny},   {MODE_FORWARD, 16, 10, 2, 12288},
+    {MODE_FORWARD, 16, 4, 4, 24576},   {MODE_FORWARD, 16, 1, 16, kAny},
+    {MODE_FORWARD, 20, 10, 2, 12288},  {MODE_FORWARD, 20, 5, 4, 20480},
+    {MODE_FORWARD, 20, 2, 10, 40960},  {MODE_FORWARD, 20, 1, 20, kAny},
+    {MODE_FORWARD, 32, 16, 2, 3072},   {MODE_FORWARD, 32, 8, 4, 8192},
+    {MODE_FORWARD, 32, 4, 8, 73728},   {MODE_FORWARD, 32, 1, 32, kAny},
+    {MODE_FORWARD, 40, 10, 4, 32768},  {MODE_FORWARD, 40, 2, 20, kAny},
+    {MODE_FORWARD, 64, 16, 4, 8192},   {MODE_FORWARD, 64, 8, 8, kAny},
+    {MODE_FORWARD, 128, 32, 4, kAny},
+    {MODE_T12, 10, 10, 2, 2048},       {MODE_T12, 10, 5, 2, 28672},
+    {MODE_T12, 10, 1, 10, kAny},       {MODE_T12, 16, 10, 2, 4096},
+    {MODE_T12, 16, 4, 4, 98304},       {MODE_T12, 16, 1, 16, kAny},
+    {MODE_T12, 20, 10, 2, 10240},      {MODE_T12, 20, 5, 4, kAny},
+    {MODE_T12, 32, 16, 2, 2048},       {MODE_T12, 28, 8, 4, kAny},
+    {MODE_T12, 32, 8, 4, 28672},       {MODE_T12, 32, 4, 8, kAny},
+    {MODE_T12, 40, 10, 4, kAny},       {MODE_T12, 64, 16, 4, 8192},
+    {MODE_T12, 64, 8, 8, kAny},        {MODE_T12, 128, 32, 4, kAny},
+    {MODE_T12B, 10, 10, 2, 2048},      {MODE_T12B, 10, 5, 2, 28672},
+    {MODE_T12B, 10, 1, 10, kAny},      {MODE_T12B, 16, 10, 2, 4096},
+    {MODE_T12B, 16, 4, 4, kAny},       {MODE_T12B, 20, 10, 2, 10240},
+    {MODE_T12B, 20, 5, 4, kAny},       {MODE_T12B, 32, 16, 2, 4096},
+    {MODE_T12B, 32, 8, 4, kAny},       {MODE_T12B, 40, 10, 4, kAny},
+    {MODE_T12B, 64, 16, 4, kAny},      {MODE_T12B, 128, 32, 4, kAny},
+    {MODE_T12BI, 10, 10, 2, 2048},     {MODE_T12BI, 10, 5, 2, kAny},
+    {MODE_T12BI, 16, 10, 2, 4096},     {MODE_T12BI, 16, 4, 4, kAny},
+    {MODE_T12BI, 20, 10, 2, 10240},    {MODE_T12BI, 20, 5, 4, kAny},
+    {MODE_T12BI, 32, 16, 2, 4096},     {MODE_T12BI, 32, 8, 4, kAny},
+    {MODE_T12BI, 40, 10, 4, kAny},     {MODE_T12BI, 64, 16, 4, kAny},
+    {MODE_T12BI, 128, 32, 4, kAny},
+    {MODE_GN, 10, 5, 2, 12288},        {MODE_GN, 10, 1, 10, kAny},
+    {MODE_GN, 16, 10, 2, 3072},        {MODE_GN, 16, 4, 4, kAny},
+    {MODE_GN, 20, 10, 2, 8192},        {MODE_GN, 20, 2, 10, kAny},
+    {MODE_GN, 32, 16, 2, 2048},        {MODE_GN, 32, 8, 4, kAny},
+    {MODE_GN, 40, 10, 4, kAny},        {MODE_GN, 64, 16, 4, kAny},
+    {MODE_GN, 128, 32, 4, kAny},
+};
+
+// The kernel of a plain recorded train, or null where the general sweep runs:
+// a requested shape where it has an instantiation (a requested register budget
+// is the general sweep's and is not looked at), else the rules above.
+const SweepEntry* choose_train(int mode, int states, int64_t work_items, const tsg_launch* want,
+                               int* warps) {
+    const Table t = train_table_for(mode);
+    *warps = (want && want->warps_per_block > 0) ? want->warps_per_block : 4;
+    if (*warps > kTrainMaxWarps) return nullptr;
+    auto find = [&](int lanes, int orders) -> const SweepEntry* {
+        for (int i = 0; i < t.count; ++i)
+            if (t.entries[i].lanes_per_voxel == lanes && t.entries[i].orders_per_lane == orders)
+                return &t.entries[i];
+        return nullptr;
+    };
+    if (want && (want->lanes_per_voxel > 0 || want->orders_per_lane > 0)) {
+        if (want->lanes_per_voxel * want->orders_per_lane < states) return nullptr;
+        return find(want->lanes_per_voxel, want->orders_per_lane);
+    }
+    for (const TrainRule& r : kTrainRules)
+        if (r.mode == mode && states <= r.states && work_items < r.below)
+            return find(r.lanes, r.orders);
+    return nullptr;
+}
+
 int mode_for_mask(unsigned mask) {
     if (mask == 0) return MODE_FORWARD;
     if ((mask & ~3u) == 0) return MODE_T12;
@@ -117,7 +213,10 @@ int mode_for_mask(unsigned mask) {
 int launch(int mode, const tsg_program* prog, const SweepArgs& args, int64_t atoms, int states,
            const tsg_launch* want, cudaStream_t stream) {
     int warps = 4;
-    const SweepEntry* e = choose(mode, states, atoms * prog->host.trains, want, &warps);
+    const SweepEntry* e = nullptr;
+    if (prog->host.train_first >= 0 && !args.ckpt && !args.traj)
+        e = choose_train(mode, states, atoms * prog->host.trains, want, &warps);
+    if (!e) e = choose(mode, states, atoms * prog->host.trains, want, &warps);
     if (!e) return fail(TSG_ERR_UNSUPPORTED, "no sweep kernel for this state count / launch shape");
     if (warps < 1 || warps > 8) return fail(TSG_ERR_ARGUMENT, "warps_per_block must be 1..8");
     if (atoms == 0 || prog->host.ops == 0) return TSG_OK;
@@ -135,6 +234,7 @@ SweepArgs base_args(const tsg_program* prog, const tsg_tissue* tissue, int64_t a
                     int64_t states) {
     SweepArgs a{};
     a.ops = prog->d_ops;
+    a.train_first = prog->host.train_first;
     a.n_ops = int(prog->host.ops);
     a.atoms = atoms;
     a.states = int(states);
@@ -478,6 +578,23 @@ extern "C" int tsg_gn_evaluate(const tsg_program* program, const tsg_tissue* tis
     a.gn_out = normal_equations;
     return launch(MODE_GN, program, a, atom_count, int(state_count), launch_shape,
                   static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tsg_gn_shape(const tsg_program* program, int64_t atom_count, int64_t state_count,
+                            tsg_launch* shape) {
+    if (!program || !shape) return fail(TSG_ERR_ARGUMENT, "null argument");
+    if (atom_count < 0 || state_count < 1) return fail(TSG_ERR_ARGUMENT, "invalid EPG buffer dimensions");
+    *shape = tsg_launch{};
+    int warps = 4;
+    const SweepEntry* e = program->host.train_first < 0 || state_count > 256
+                              ? nullptr
+                              : choose_train(MODE_GN, int(state_count), atom_count, nullptr, &warps);
+    if (e) {
+        shape->lanes_per_voxel = e->lanes_per_voxel;
+        shape->orders_per_lane = e->orders_per_lane;
+        shape->warps_per_block = warps;
+    }
+    return TSG_OK;
 }
 
 namespace tsg {

@@ -108,6 +108,21 @@ struct Builder {
 
 }  // namespace
 
+int find_train(const HostProgram& program) {
+    if (program.ops == 0) return -1;
+    const int first = op_rf(program.op[0].code) == RF_INVERT ? 1 : 0;
+    for (int64_t t = 0; t < program.trains; ++t) {
+        const Op* ops = program.op.data() + t * program.ops;
+        if (first && ops[0].code != uint32_t(RF_INVERT) << OP_RF_SHIFT) return -1;
+        for (int64_t i = first; i < program.ops; ++i) {
+            // An op without a relaxation is one of zero duration.
+            if ((ops[i].code | OP_RELAX) != (kFastBits | OP_RECORD)) return -1;
+            if (ops[i].record != i - first) return -1;
+        }
+    }
+    return program.ops - first == program.outputs ? first : -1;
+}
+
 int compile_program(const float* duration, const int32_t* kind, const float* flip,
                     const uint8_t* action, const int32_t* output_index, int64_t trains,
                     int64_t events, bool unmerged, const float* duration_tangent,
@@ -187,6 +202,7 @@ int compile_program(const float* duration, const int32_t* kind, const float* fli
         for (int64_t t = 0; t < trains; ++t)
             std::copy(per_phase[t].begin(), per_phase[t].end(), out->phase.begin() + t * longest);
     }
+    out->train_first = find_train(*out);
     return TSG_OK;
 }
 

@@ -70,6 +70,9 @@ struct HostProgram {
     int64_t ops = 0;       // per train (trains padded to the longest)
     int64_t outputs = 0;   // recorded samples per train
     bool sequential_records = true;  // records appear as 0,1,2,... in op order
+    // A plain recorded train (find_train): the first op of the train, 0 or 1
+    // (after a leading inversion); -1 for any other program.
+    int train_first = -1;
     std::vector<Op> op;              // [train][ops]
     std::vector<OpSource> src;       // [train][ops]
     // With event phases (the complex path): per op the phase of its pulse
@@ -113,9 +116,13 @@ int compile_program(const float* duration, const int32_t* kind, const float* fli
                     int64_t events, bool unmerged, const float* duration_tangent,
                     HostProgram* out, const float* phase = nullptr);
 
+// Where the plain recorded train of a compiled program begins (0 or 1), or -1.
+int find_train(const HostProgram& program);
+
 // Arguments of one sweep launch (forward, fused tangents, general tangent).
 struct SweepArgs {
     const Op* ops;
+    int train_first;  // HostProgram::train_first
     const float2* op_dir;  // general tangent: (d dt, d flip) per op, [train][ops]
     int n_ops;
     int64_t atoms;
@@ -197,6 +204,20 @@ extern const SweepEntry kSweepGeneral[];
 extern const int kSweepGeneralCount;
 extern const SweepEntry kSweepGN[];
 extern const int kSweepGNCount;
+
+// The same modes' kernels for plain recorded trains (epg_train.cuh), for
+// blocks of up to kTrainMaxWarps warps.
+constexpr int kTrainMaxWarps = 4;
+extern const SweepEntry kTrainForward[];
+extern const int kTrainForwardCount;
+extern const SweepEntry kTrainT12[];
+extern const int kTrainT12Count;
+extern const SweepEntry kTrainT12B[];
+extern const int kTrainT12BCount;
+extern const SweepEntry kTrainT12BI[];
+extern const int kTrainT12BICount;
+extern const SweepEntry kTrainGN[];
+extern const int kTrainGNCount;
 
 constexpr int kOpChunk = 1024;  // ops staged in shared memory at a time
 

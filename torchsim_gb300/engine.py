@@ -418,14 +418,16 @@ def sweep_to_host(program: Program, tissue: TissueMaps, states: int, names: Sequ
 
 
 # (lanes per voxel, orders per lane) instantiated per kernel family, as in the
-# sweep tables of csrc/sweep_*.cu.
+# sweep tables of csrc/sweep_*.cu and csrc/train_*.cu (a shape of one table
+# only runs the programs of that table).
 FAMILY_SHAPES = {
     0: [(1, 10), (1, 20), (5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (4, 8), (8, 4), (8, 8),
-        (16, 4), (16, 8), (32, 4), (32, 8), (2, 10)],
+        (16, 4), (16, 8), (32, 4), (32, 8), (2, 10), (16, 2), (10, 4), (1, 16), (1, 32), (2, 20)],
     3: [(1, 10), (5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (4, 8), (8, 4), (8, 8), (16, 4),
-        (32, 4)],
-    7: [(5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (8, 4), (16, 4), (32, 4)],
-    15: [(5, 2), (5, 4), (10, 2), (4, 4), (8, 4), (16, 4), (32, 4)],
+        (32, 4), (16, 2), (10, 4), (1, 16)],
+    7: [(5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (8, 4), (16, 4), (32, 4), (16, 2), (10, 4),
+        (1, 10)],
+    15: [(5, 2), (5, 4), (10, 2), (4, 4), (8, 4), (16, 4), (32, 4), (16, 2), (10, 4)],
 }
 
 

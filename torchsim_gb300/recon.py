@@ -137,6 +137,18 @@ def config_of(bounds: Mapping[str, Any], tau: float, gradient_tolerance: float,
                             float(gradient_tolerance), float(step_tolerance), int(max_iterations))
 
 
+def pool_shape(program: Program, voxels: int, states: int) -> tuple[int, int, int] | None:
+    """The GN sweep's own launch shape for a solve that starts with
+    ``voxels`` voxels (``tsg_gn_shape``), or None for the general sweep's
+    choice."""
+    shape = _native.Launch()
+    _native.check(_native.library().tsg_gn_shape(program.handle, voxels, states,
+                                                 ctypes.byref(shape)))
+    if shape.lanes_per_voxel == 0:
+        return None
+    return shape.lanes_per_voxel, shape.orders_per_lane, shape.warps_per_block
+
+
 def fixed_shape(states: int) -> tuple[int, int, int]:
     """A (lanes per voxel, orders per lane, warps per CTA) of the GN sweep
     table that covers ``states``, chosen from the state count alone."""
@@ -689,10 +701,11 @@ class GaussNewton:
         steps = torch.zeros(V, dtype=torch.int32, device=device)
         limited = torch.zeros(V, dtype=torch.int32, device=device)
         history, weights = [], []
+        launch = self.launch if self.launch is not None else pool_shape(program, V, states)
         for it in range(self.max_iterations + 1):
             if it and pool.n:
                 weights.append(pool.t["damping"].mean())
-            pool.iterate(program, measured, states, config, self.launch)
+            pool.iterate(program, measured, states, config, launch)
             out = pool.retire()
             answer_u[out["owner"]] = out["u"]
             cost[out["owner"]] = out["cost"]
