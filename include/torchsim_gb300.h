@@ -549,6 +549,19 @@ int tsg_gn_step(const tsg_gn_state* state, int64_t voxel_count, const tsg_gn_con
  * and retirement on a short step or the step limit. */
 int tsg_gn_judge(const tsg_gn_state* state, int64_t voxel_count, const tsg_gn_config* config,
                  void* stream);
+/* A whole solve from the state's u (status, flags, iterations, cost and
+ * damping zero): max_iterations + 1 times step, evaluate, judge over the
+ * voxels still live, all queued on the stream with nothing read back. `b1` is
+ * nullable; `measured` has the voxels' rows in order. Scratch and results on
+ * the device: `lists` 2 * voxel_count entries; counts[it], the voxels live
+ * after iteration it (a solve is over where it is 0); totals[it][part][2],
+ * tsg_gn_total_parts() parts of the summed cost and of the live voxels' summed
+ * damping. Answers are in the state arrays. */
+int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* state, const float* b1,
+                 int64_t voxel_count, int64_t state_count, const void* measured,
+                 const tsg_gn_config* config, int32_t* lists, int32_t* counts, double* totals,
+                 const tsg_launch* launch, void* stream);
+int tsg_gn_total_parts(void);
 /* Natural parameters (voxel_count x 3 floats) of free variables. */
 int tsg_gn_natural(const double* free_variables, int64_t voxel_count, const tsg_gn_config* config,
                    float* natural, void* stream);

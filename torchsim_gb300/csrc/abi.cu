@@ -562,10 +562,12 @@ extern "C" int tsg_epg_forward_tangents(const tsg_program* program, const tsg_ti
                   static_cast<cudaStream_t>(stream));
 }
 
-extern "C" int tsg_gn_evaluate(const tsg_program* program, const tsg_tissue* tissue,
-                               int64_t atom_count, int64_t state_count, const void* measured,
-                               const int64_t* measured_rows, double* normal_equations,
-                               const tsg_launch* launch_shape, void* stream) {
+namespace tsg {
+
+int gn_evaluate_list(const tsg_program* program, const tsg_tissue* tissue, int64_t atom_count,
+                     int64_t state_count, const void* measured, const int64_t* measured_rows,
+                     const int32_t* voxel_list, const int32_t* voxel_list_count,
+                     double* normal_equations, const tsg_launch* launch_shape, void* stream) {
     int rc = check_common(program, tissue, atom_count, state_count);
     if (rc) return rc;
     if (atom_count == 0) return TSG_OK;
@@ -576,8 +578,20 @@ extern "C" int tsg_gn_evaluate(const tsg_program* program, const tsg_tissue* tis
     a.measured = static_cast<const float2*>(measured);
     a.measured_rows = measured_rows;
     a.gn_out = normal_equations;
+    a.voxel_list = voxel_list;
+    a.voxel_list_count = voxel_list_count;
     return launch(MODE_GN, program, a, atom_count, int(state_count), launch_shape,
                   static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace tsg
+
+extern "C" int tsg_gn_evaluate(const tsg_program* program, const tsg_tissue* tissue,
+                               int64_t atom_count, int64_t state_count, const void* measured,
+                               const int64_t* measured_rows, double* normal_equations,
+                               const tsg_launch* launch_shape, void* stream) {
+    return gn_evaluate_list(program, tissue, atom_count, state_count, measured, measured_rows,
+                            nullptr, nullptr, normal_equations, launch_shape, stream);
 }
 
 extern "C" int tsg_gn_shape(const tsg_program* program, int64_t atom_count, int64_t state_count,

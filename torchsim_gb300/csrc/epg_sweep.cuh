@@ -176,10 +176,18 @@ __global__ void __launch_bounds__(MINB > 1 ? 128 : 256, MINB) epg_sweep_kernel(c
     const int warp = threadIdx.x >> 5;
     const int q = lane % L;
     const int slot = lane / L;
-    const int64_t atom = (int64_t(blockIdx.x) * (blockDim.x >> 5) + warp) * VPW + slot;
+    int64_t atom = (int64_t(blockIdx.x) * (blockDim.x >> 5) + warp) * VPW + slot;
     const int64_t train = blockIdx.y;
     // Lanes past the last whole voxel of the warp (32 % L of them) idle.
-    const bool active = slot < VPW && atom < a.atoms;
+    bool active = slot < VPW && atom < a.atoms;
+    if constexpr (GN) {
+        if (a.voxel_list != nullptr) {
+            const int n = *a.voxel_list_count;
+            if (int64_t(blockIdx.x) * (blockDim.x >> 5) * VPW >= n) return;
+            active = slot < VPW && atom < n;
+            atom = a.voxel_list[active ? atom : 0];
+        }
+    }
     const int64_t ac = active ? atom : 0;
 
     const float t1 = a.t1[ac];

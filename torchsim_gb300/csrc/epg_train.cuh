@@ -90,9 +90,17 @@ __global__ void __launch_bounds__(128, MINB) epg_train_kernel(const SweepArgs a)
     const bool holds = slot < VPW;  // lanes past the last whole voxel idle
     const int vslot = holds ? slot : 0;
     const int64_t warp_atom = (int64_t(blockIdx.x) * (blockDim.x >> 5) + warp) * VPW;
-    const int64_t atom = warp_atom + slot;
     const int64_t train = blockIdx.y;
-    const bool active = holds && atom < a.atoms;
+    int64_t atom = warp_atom + slot;
+    bool active = holds && atom < a.atoms;
+    if constexpr (GN) {
+        if (a.voxel_list != nullptr) {
+            const int n = *a.voxel_list_count;
+            if (int64_t(blockIdx.x) * (blockDim.x >> 5) * VPW >= n) return;
+            active = holds && atom < n;
+            atom = a.voxel_list[active ? atom : 0];
+        }
+    }
     const int64_t ac = active ? atom : 0;
 
     float2* s_ops = reinterpret_cast<float2*>(s_raw);  // (dt, flip)

@@ -105,9 +105,21 @@ __device__ bool damped_solve(const double A[3][3], const double* g, double lambd
     return isfinite(d[0]) && isfinite(d[1]) && isfinite(d[2]);
 }
 
-__global__ void gn_step_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c) {
+// The voxels a launch works on: all n, or the first *count of a device list.
+struct VoxelList {
+    const int32_t* index;
+    const int32_t* count;
+};
+
+__device__ __forceinline__ int64_t listed_voxel(const VoxelList& list, int64_t n) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (list.index == nullptr) return i < n ? i : -1;
+    return i < *list.count ? list.index[i] : -1;
+}
+
+__global__ void gn_step_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c, VoxelList list) {
+    const int64_t i = listed_voxel(list, n);
+    if (i < 0) return;
     const int status = s.status[i];
     if (status == TSG_GN_DONE) return;
     double u[3] = {s.u[3 * i], s.u[3 * i + 1], s.u[3 * i + 2]};
@@ -153,9 +165,7 @@ __global__ void gn_step_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c) {
     s.m0[i] = float(x[2]);
 }
 
-__global__ void gn_judge_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__device__ void gn_judge(const tsg_gn_state& s, const tsg_gn_config& c, int64_t i) {
     const int status = s.status[i];
     if (status == TSG_GN_DONE) return;
     const double* tr = s.trial + 10 * i;
@@ -205,6 +215,70 @@ __global__ void gn_judge_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c) {
     }
 }
 
+__global__ void gn_judge_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c) {
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) gn_judge(s, c, i);
+}
+
+constexpr int kSolveThreads = 128;
+
+// The judgement of a solve's iteration, and the list of voxels for the next
+// one: a block's survivors keep their order, the blocks' runs come in the
+// order they reserve their places. A voxel's arithmetic does not depend on
+// its place.
+__global__ void __launch_bounds__(kSolveThreads)
+    gn_judge_list_kernel(tsg_gn_state s, int64_t n, tsg_gn_config c, VoxelList list,
+                         int32_t* next, int32_t* next_count) {
+    __shared__ int s_warp[kSolveThreads / 32];
+    __shared__ int s_base;
+    const int64_t i = listed_voxel(list, n);
+    bool live = false;
+    if (i >= 0) {
+        gn_judge(s, c, i);
+        live = s.status[i] != TSG_GN_DONE;
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned votes = __ballot_sync(0xffffffffu, live);
+    if (lane == 0) s_warp[warp] = __popc(votes);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+        for (int w = 0; w < kSolveThreads / 32; ++w) {
+            const int k = s_warp[w];
+            s_warp[w] = total;
+            total += k;
+        }
+        s_base = total > 0 ? atomicAdd(next_count, total) : 0;
+    }
+    __syncthreads();
+    if (live) next[s_base + s_warp[warp] + __popc(votes & ((1u << lane) - 1u))] = int32_t(i);
+}
+
+// Sums of the cost over all voxels and of the damping over the live ones, as
+// one pair per block, each over a fixed share of the voxels in a fixed order.
+constexpr int kTotalBlocks = 64;
+constexpr int kTotalThreads = 256;
+__global__ void __launch_bounds__(kTotalThreads)
+    gn_totals_kernel(tsg_gn_state s, int64_t n, double* out) {
+    __shared__ double s_part[2][kTotalThreads];
+    double cost = 0.0, damping = 0.0;
+    for (int64_t i = int64_t(blockIdx.x) * kTotalThreads + threadIdx.x; i < n;
+         i += int64_t(kTotalBlocks) * kTotalThreads) {
+        cost += s.cost[i];
+        if (s.status[i] == TSG_GN_LIVE) damping += s.damping[i];
+    }
+    s_part[0][threadIdx.x] = cost;
+    s_part[1][threadIdx.x] = damping;
+    for (int half = kTotalThreads / 2; half > 0; half >>= 1) {
+        __syncthreads();
+        if (threadIdx.x < half) {
+            s_part[0][threadIdx.x] += s_part[0][threadIdx.x + half];
+            s_part[1][threadIdx.x] += s_part[1][threadIdx.x + half];
+        }
+    }
+    if (threadIdx.x < 2) out[2 * blockIdx.x + threadIdx.x] = s_part[threadIdx.x][0];
+}
+
 __global__ void gn_natural_kernel(const double* u, int64_t n, tsg_gn_config c, float* out) {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -230,7 +304,7 @@ extern "C" int tsg_gn_step(const tsg_gn_state* state, int64_t voxel_count,
         return fail(TSG_ERR_ARGUMENT, "invalid Gauss-Newton state");
     if (voxel_count == 0) return TSG_OK;
     gn_step_kernel<<<unsigned((voxel_count + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(
-        *state, voxel_count, *config);
+        *state, voxel_count, *config, VoxelList{nullptr, nullptr});
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
 }
@@ -256,3 +330,44 @@ extern "C" int tsg_gn_natural(const double* free_variables, int64_t voxel_count,
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
 }
+
+// A whole solve queued on the stream: per iteration the step, the evaluation,
+// the judgement with the next voxel list, and the sums. Nothing is read back,
+// so the launches of all iterations are queued at once (a copy of the pool's
+// rows per iteration and one wait each took as long as the sweeps); the grids
+// cover every voxel and blocks past the live ones end at once.
+extern "C" int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* state,
+                            const float* b1, int64_t voxel_count, int64_t state_count,
+                            const void* measured, const tsg_gn_config* config, int32_t* lists,
+                            int32_t* counts, double* totals, const tsg_launch* launch_shape,
+                            void* stream) {
+    if (voxel_count < 0 || !config || (voxel_count > 0 && !valid(state)))
+        return fail(TSG_ERR_ARGUMENT, "invalid Gauss-Newton state");
+    if (config->max_iterations < 1) return fail(TSG_ERR_ARGUMENT, "max_iterations must be positive");
+    if (voxel_count > 0x7fffffffLL) return fail(TSG_ERR_CAPACITY, "too many voxels for one solve");
+    if (voxel_count == 0) return TSG_OK;
+    if (!lists || !counts || !totals) return fail(TSG_ERR_ARGUMENT, "null solve buffer");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const unsigned blocks = unsigned((voxel_count + kSolveThreads - 1) / kSolveThreads);
+    const int iterations = config->max_iterations + 1;
+    TSG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * iterations, s));
+    const tsg_tissue tissue{state->t1, state->t2, state->m0, b1, nullptr};
+    for (int it = 0; it < iterations; ++it) {
+        VoxelList list{nullptr, nullptr};
+        if (it > 0) list = {lists + (it & 1) * voxel_count, counts + it - 1};
+        gn_step_kernel<<<blocks, kSolveThreads, 0, s>>>(*state, voxel_count, *config, list);
+        TSG_CUDA(cudaGetLastError());
+        const int rc = gn_evaluate_list(program, &tissue, voxel_count, state_count, measured, nullptr,
+                                        list.index, list.count, state->trial, launch_shape, stream);
+        if (rc) return rc;
+        gn_judge_list_kernel<<<blocks, kSolveThreads, 0, s>>>(
+            *state, voxel_count, *config, list, lists + ((it + 1) & 1) * voxel_count, counts + it);
+        TSG_CUDA(cudaGetLastError());
+        gn_totals_kernel<<<kTotalBlocks, kTotalThreads, 0, s>>>(
+            *state, voxel_count, totals + int64_t(it) * 2 * kTotalBlocks);
+        TSG_CUDA(cudaGetLastError());
+    }
+    return TSG_OK;
+}
+
+extern "C" int tsg_gn_total_parts(void) { return kTotalBlocks; }

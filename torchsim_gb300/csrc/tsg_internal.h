@@ -168,6 +168,10 @@ struct SweepArgs {
     const float2* measured;
     const int64_t* measured_rows;
     double* gn_out;
+    // Optional, GN sweeps of one train: only the voxels of this device list,
+    // whose length is on the device too (blocks past it end at once).
+    const int32_t* voxel_list;
+    const int32_t* voxel_list_count;
 };
 
 using SweepLaunch = void (*)(const SweepArgs&, dim3 grid, dim3 block, size_t smem,
@@ -257,6 +261,12 @@ struct AdjointEntry {
     AdjointLaunch launch;
     const void* kernel;  // for the shared-memory attribute
 };
+
+// tsg_gn_evaluate over a device list of voxels (null: every voxel).
+int gn_evaluate_list(const tsg_program* program, const tsg_tissue* tissue, int64_t atom_count,
+                     int64_t state_count, const void* measured, const int64_t* measured_rows,
+                     const int32_t* voxel_list, const int32_t* voxel_list_count,
+                     double* normal_equations, const tsg_launch* launch_shape, void* stream);
 
 // The reverse-sweep kernels built for `warps` warps per block (2 or 4),
 // checkpointed or trajectory; null with *count = 0 for any other block size.

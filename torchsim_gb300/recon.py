@@ -688,36 +688,51 @@ class GaussNewton:
 
     def _pool_solve(self, program: Program, measured: torch.Tensor, u0: torch.Tensor,
                     b1: torch.Tensor | None, config: _native.GNConfig, states: int):
-        """The fused device loop over a voxel pool: (free variables in
-        T1, T2, M0 order, final cost, steps and limit flags per voxel, the
-        summed cost and mean damping after every iteration)."""
+        """The fused device loop: (free variables in T1, T2, M0 order, final
+        cost, steps and limit flags per voxel, the summed cost and mean
+        damping after every iteration). Every iteration is queued at once
+        (``tsg_gn_solve``); the one wait is for the counts of live voxels at
+        the end."""
         device = measured.device
         V = measured.shape[0]
-        pool = VoxelPool(device)
-        idx = torch.arange(V, device=device)
-        pool.add(u0, b1, idx, idx)
-        answer_u = u0.clone()
-        cost = torch.zeros(V, dtype=torch.float64, device=device)
-        steps = torch.zeros(V, dtype=torch.int32, device=device)
-        limited = torch.zeros(V, dtype=torch.int32, device=device)
-        history, weights = [], []
+        lib = _native.library()
+        parts = int(lib.tsg_gn_total_parts())
+        rounds = self.max_iterations + 1
+        if V == 0:
+            empty = torch.zeros(0, dtype=torch.float64, device=device)
+            none = torch.zeros(0, dtype=torch.int32, device=device)
+            return (u0.clone(), empty, none, none,
+                    torch.zeros(1, dtype=torch.float64, device=device), empty)
+        if b1 is not None:
+            b1 = b1.to(device, torch.float32).reshape(V).contiguous()
+        # Rows of the state that start at zero, then the ones written before
+        # they are read.
+        u = u0.to(device, torch.float64).expand(V, 3).clone()
+        zeroed = torch.zeros((3, V), dtype=torch.float64, device=device)
+        wide = torch.empty(V * 24, dtype=torch.float64, device=device)
+        cand, normal, trial, predicted = wide.split([3 * V, 10 * V, 10 * V, V])
+        whole = torch.zeros((3, V), dtype=torch.int32, device=device)
+        natural = torch.empty((3, V), dtype=torch.float32, device=device)
+        lists = torch.empty(2 * V + rounds, dtype=torch.int32, device=device)
+        totals = torch.empty((rounds, parts, 2), dtype=torch.float64, device=device)
+        cost, damping, rising = zeroed
+        status, flags, steps = whole
+        state = _native.GNState(*[t.data_ptr() for t in (
+            u, cand, cost, normal, trial, damping, rising, predicted, status, flags, steps,
+            *natural)])
         launch = self.launch if self.launch is not None else pool_shape(program, V, states)
-        for it in range(self.max_iterations + 1):
-            if it and pool.n:
-                weights.append(pool.t["damping"].mean())
-            pool.iterate(program, measured, states, config, launch)
-            out = pool.retire()
-            answer_u[out["owner"]] = out["u"]
-            cost[out["owner"]] = out["cost"]
-            steps[out["owner"]] = out["iterations"]
-            limited[out["owner"]] = out["limited"]
-            history.append(cost.sum() + pool.t["cost"].sum())
-            if pool.n == 0:
-                break
-        empty = torch.zeros(0, dtype=torch.float64, device=device)
-        return (answer_u, cost, steps, limited,
-                torch.stack(history) if history else empty,
-                torch.stack(weights) if weights else empty)
+        counts = lists[2 * V:]
+        _native.check(lib.tsg_gn_solve(
+            program.handle, ctypes.byref(state), None if b1 is None else b1.data_ptr(), V, states,
+            measured.data_ptr(), ctypes.byref(config), lists.data_ptr(), counts.data_ptr(),
+            totals.data_ptr(), _native.launch_shape(launch),
+            torch.cuda.current_stream(device).cuda_stream))
+        live = counts.cpu()
+        over = torch.nonzero(live == 0)
+        rounds = int(over[0]) + 1 if over.numel() else rounds
+        history, weights = totals[:rounds].sum(1).unbind(-1)
+        weights = weights[: rounds - 1] / counts[: rounds - 1]
+        return u, cost, steps, flags & 4, history.contiguous(), weights
 
     @torch.no_grad()
     def minimize_program(self, program: Program, measured: torch.Tensor, start: torch.Tensor,
