@@ -887,19 +887,23 @@ def match_section(torch, device, voxels: int = 65536, repeats: int = 3) -> dict:
     match_ms = timed(lambda: matcher.match(measured))
     # The screen kernel alone, for the roofline.
     s_hat = measured / torch.linalg.vector_norm(measured, dim=-1, keepdim=True)
-    queries = matcher._queries(s_hat)
-    k = matcher._screen_atoms.shape[1]
+    prepared = matcher._prepared()
     lib = _native.library()
-    cands = lib.tsg_match_candidates()
-    cand_s = torch.empty((voxels, cands), dtype=torch.float32, device=device)
-    cand_i = torch.empty((voxels, cands), dtype=torch.int32, device=device)
+    stream = torch.cuda.current_stream().cuda_stream
+    queries = torch.empty((2 * voxels, prepared.k), dtype=torch.float16, device=device)
+    _native.check(lib.tsg_match_queries(s_hat.data_ptr(), voxels, prepared.samples, prepared.k,
+                                        prepared.scale, int(prepared.axis == 0), queries.data_ptr(),
+                                        stream))
+    k = 2 * prepared.k
+    lists = (lib.tsg_match_lists(voxels, A, prepared.k), voxels, lib.tsg_match_candidates())
+    cand_s = torch.empty(lists, dtype=torch.float32, device=device)
+    cand_i = torch.empty(lists, dtype=torch.int32, device=device)
     err = torch.zeros(1, dtype=torch.int32, device=device)
 
     def screen():
-        _native.check(lib.tsg_match_screen(queries.data_ptr(), 2 * voxels,
-                                           matcher._screen_atoms.data_ptr(), A, k,
-                                           cand_s.data_ptr(), cand_i.data_ptr(), err.data_ptr(),
-                                           torch.cuda.current_stream().cuda_stream))
+        _native.check(lib.tsg_match_screen_lists(
+            queries.data_ptr(), 2 * voxels, prepared.screen_atoms, A, prepared.k, cand_s.data_ptr(),
+            cand_i.data_ptr(), err.data_ptr(), stream))
 
     screen_ms = timed(screen)
     # Executed tensor work: every query row against every atom's hi and lo

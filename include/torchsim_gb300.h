@@ -587,6 +587,49 @@ int tsg_match_screen(const void* queries, int64_t query_rows, const void* atoms,
 int tsg_match_rescore(const void* signals, int64_t voxels, const void* atoms, int64_t atom_count,
                       int64_t samples, const int32_t* candidate_index, int top_k, float* scores,
                       int64_t* index, void* stream);
+/* A dictionary prepared for tsg_match (DEVICE pointers). Each screen atom is
+ * two fp16 rows side by side along the contraction, its value and the rounding
+ * remainder: (tsg_match_screen_rows(atom_count) x 2 k), rows permuted, values
+ * times `scale`, k a multiple of 8 of at least the samples (twice that for
+ * complex atoms: real parts, then imaginary). `axis` 0: complex atoms,
+ * normalized_atoms complex64; 1 real or 2 on the imaginary axis,
+ * normalized_atoms their one float part; both (atom_count x samples).
+ * dictionary: the complex64 atoms as given, power their squared norms; table
+ * (nullable): `columns` floats per atom. */
+typedef struct {
+    const void* screen_atoms;
+    const void* normalized_atoms;
+    const void* dictionary;
+    const float* power;
+    const float* table;
+    int64_t atom_count;
+    int64_t samples;
+    int64_t k;
+    float scale;
+    int32_t axis;
+    int32_t columns;
+} tsg_match_dictionary;
+
+/* Candidate lists a voxel may have: with few voxels the atoms are shared among
+ * several CTAs, each of which keeps its own. */
+int tsg_match_lists(int64_t voxels, int64_t atom_count, int64_t k);
+/* The two fp16 rows (k wide, zero-padded) of each normalized complex64 signal. */
+int tsg_match_queries(const void* normalized, int64_t voxels, int64_t samples, int64_t k, float scale,
+                      int complex_atoms, void* queries, void* stream);
+/* The screen of tsg_match: queries (query_rows x k) against atoms (rows x 2 k)
+ * into lists x (query_rows / 2) x candidates scores and indices. */
+int tsg_match_screen_lists(const void* queries, int64_t query_rows, const void* atoms,
+                           int64_t atom_count, int64_t k, float* list_scores, int32_t* list_index,
+                           int* error, void* stream);
+/* A whole match of `voxels` complex64 signals, given as they are and
+ * normalized, with the norms: query rows (scratch, 2 voxels x k fp16, 16-byte
+ * aligned), screen (scratch lists, as tsg_match_screen_lists), exact FP32
+ * rescoring, and per voxel the top_k (1..8) scores, atom indices, complex
+ * least-squares scales, densities and table rows. */
+int tsg_match(const tsg_match_dictionary* dictionary, const void* signals, const void* normalized,
+              const float* norms, int64_t voxels, int top_k, void* queries, float* list_scores,
+              int32_t* list_index, int* error, float* scores, int64_t* index, void* scales,
+              float* densities, float* parameters, void* stream);
 /* Candidates the screen keeps per voxel (32). */
 int tsg_match_candidates(void);
 /* Rows of the atom matrix tsg_match_screen reads for atom_count atoms (a

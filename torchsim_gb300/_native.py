@@ -86,6 +86,13 @@ class GNConfig(ctypes.Structure):
                 ("step_tolerance", ctypes.c_double), ("max_iterations", ctypes.c_int32)]
 
 
+class MatchDictionary(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("screen_atoms", "normalized_atoms", "dictionary",
+                                               "power", "table")]
+    _fields_ += [("atom_count", ctypes.c_int64), ("samples", ctypes.c_int64), ("k", ctypes.c_int64),
+                 ("scale", ctypes.c_float), ("axis", ctypes.c_int32), ("columns", ctypes.c_int32)]
+
+
 class Launch(ctypes.Structure):
     _fields_ = [("lanes_per_voxel", ctypes.c_int), ("orders_per_lane", ctypes.c_int),
                 ("warps_per_block", ctypes.c_int), ("min_blocks_per_sm", ctypes.c_int)]
@@ -156,6 +163,11 @@ SIGNATURES: dict[str, tuple] = {
     "tsg_gn_natural": (_int, [_vp, _i64, ctypes.POINTER(GNConfig), _vp, _vp]),
     "tsg_match_screen": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "tsg_match_rescore": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _int, _vp, _vp, _vp]),
+    "tsg_match_lists": (_int, [_i64, _i64, _i64]),
+    "tsg_match_queries": (_int, [_vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp]),
+    "tsg_match_screen_lists": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
+    "tsg_match": (_int, [ctypes.POINTER(MatchDictionary), _vp, _vp, _vp, _i64, _int, _vp, _vp, _vp,
+                         _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
     "tsg_match_candidates": (_int, []),
     "tsg_match_screen_rows": (_int, [_i64]),
     "tsg_epg_simulate_vjp": (_int, [ctypes.POINTER(_vp), _i64, _i64, _i64, _i64, _i64, _i64,

@@ -5,7 +5,8 @@
 // through chunked FP32 matrix products (_grouped.py:212-240) and keeps the
 // top k. Here one kernel does the product and the selection without ever
 // writing the score matrix: queries (two rows per voxel) and atoms are fp16
-// K-major tiles brought by TMA into a 4-stage shared-memory ring;
+// K-major tiles brought by TMA into shared memory (the queries once per sweep
+// over the atoms where they fit, the atoms through a ring);
 // `tcgen05.mma` (issued by one thread) accumulates a 128 x 256 tile in tensor
 // memory, double-buffered so the epilogue of one atom tile overlaps the MMAs of
 // the next; eight epilogue warps (two per TMEM lane quarter, each taking every
@@ -24,9 +25,21 @@
 // complex atoms (Re s, Im s) and (Im s, -Re s) against (Re d, Im d), whose
 // products are the real and imaginary parts of <s, d>.
 //
+// Bound: the tensor pipe (60% active by ncu at 1.94 GHz, and with the scoring
+// left out no more than 1.45 to 1.6 PFLOP/s). Measured, 16,384 voxels x 65,536
+// atoms x 500 samples: 3.62 ms with one CTA per 128 rows in whole waves, 3.24
+// with row tiles in pairs, the last wave split and resident queries, 3.16 with
+// the pair's two SMs on one product, 2.95 (1.46 PFLOP/s) with the candidates
+// inserted a lane's best at a time; 1,024 voxels 2.0 -> 0.22 ms by the split.
+// The rescoring, bound by reading the candidates' atoms, 367 -> 219 us by
+// reading one part of atoms on an axis and four candidates at a time.
+//
 // Waits on mbarriers are bounded: a wait that runs out sets the error word
 // and the kernel winds down instead of hanging.
 #include <cuda.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
 
 #include "tsg_internal.h"
 
@@ -34,13 +47,25 @@ namespace tsg {
 
 namespace {
 
-constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
+constexpr int BM = 128, BN = 256, BK = 64;  // of one CTA's query rows; of a pair's atoms
 constexpr int kScreen = 8;           // per lane
 constexpr int kHalves = 2;            // epilogue warps per TMEM lane quarter
-constexpr int kCand = 2 * kHalves * kScreen;  // per voxel
+constexpr int kClasses = 2 * kHalves;
+constexpr int kCand = kClasses * kScreen;  // per voxel
 constexpr int SMEM_A = BM * BK * 2;
-constexpr int SMEM_B = BN * BK * 2;
-constexpr int STAGE_BYTES = SMEM_A + SMEM_B;
+constexpr int SMEM_B = BN / 2 * BK * 2;  // a CTA's half
+// CTAs come in pairs (a cluster, cta_group::2): 256 query rows against 256
+// atoms a tile, each CTA holding its 128 query rows, its half of the atom
+// tile and the accumulator of its rows. One CTA alone reads 96 bytes of
+// shared memory a cycle for its products while 64 or more are written, which
+// is past the 128 the memory has; half the atom tile makes it 64 and 32.
+constexpr int kPair = 2;
+// Shared-memory slots: query tiles resident for a whole sweep over the atoms
+// where the contraction has at most kResident tiles, else a short ring; atom
+// tiles in a ring.
+constexpr int kResident = 8;
+constexpr int kMaxA = 8, kMaxB = 10;
+constexpr int kTileBytes = 224 * 1024;  // of both
 constexpr int TMEM_COLS = 2 * BN;
 constexpr int kEpilogueThreads = 128 * kHalves;
 // warp 0 TMA, warp 1 MMA + TMEM, warps 2.. epilogue (each lane quarter twice:
@@ -56,7 +81,7 @@ __device__ __forceinline__ bool wait_parity(uint32_t bar, uint32_t parity) {
     for (long long i = 0; i < kWaitLimit; ++i) {
         uint32_t ok;
         asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
             "selp.u32 %0, 1, 0, p;\n}\n"
             : "=r"(ok)
             : "r"(bar), "r"(parity)
@@ -75,8 +100,23 @@ __host__ __device__ __forceinline__ int stored_atom(int pos) {
     return (pos & 1) | (((pos >> 5) & 1) << 1) | (((pos >> 1) & 15) << 2) | (pos & ~63);
 }
 
-__device__ __forceinline__ void arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+// The same place in the shared memory of the pair's first CTA.
+__device__ __forceinline__ uint32_t first_cta(uint32_t addr) {
+    uint32_t there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(there) : "r"(addr));
+    return there;
+}
+
+__device__ __forceinline__ void arrive_cluster(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
+// Both CTAs of a pair (every thread of each arrives, whatever happened).
+__device__ __forceinline__ void pair_sync() {
+    asm volatile(
+        "barrier.cluster.arrive.release;\n"
+        "barrier.cluster.wait.acquire;\n" ::
+            : "memory");
 }
 
 // Shared-memory matrix descriptor of a K-major 16-bit tile with 128-byte
@@ -92,17 +132,52 @@ __device__ __forceinline__ uint64_t tile_desc(uint32_t addr) {
 }
 
 // kind::f16 instruction descriptor: FP32 accumulate, fp16 A and B (format
-// 0), both K-major, M = BM, N = BN.
-constexpr uint32_t kInstr = (1u << 4) | (uint32_t(BN >> 3) << 17) | (uint32_t(BM >> 4) << 24);
+// 0), both K-major, M = 2 BM (the pair's rows), N = BN.
+constexpr uint32_t kInstr = (1u << 4) | (uint32_t(BN >> 3) << 17) | (uint32_t(kPair * BM >> 4) << 24);
 
+// The full and tempty barriers of the pair's first CTA serve both: it issues
+// the products. The others are each CTA's own, reached by multicast commits.
 struct ScreenShared {
-    uint64_t full[STAGES];
-    uint64_t empty[STAGES];
+    uint64_t a_full[kMaxA];
+    uint64_t a_empty[kMaxA];
+    uint64_t b_full[kMaxB];
+    uint64_t b_empty[kMaxB];
     uint64_t tfull[2];
     uint64_t tempty[2];
     uint32_t tmem_base;
     int abort;
 };
+
+// How the (pair of query row tiles) x (atom tile) plane is shared among the
+// CTA pairs: items 0 .. full-1 are row pairs with all their atom tiles; the
+// last `split` row pairs are cut into `pieces` runs of `run` atom tiles each,
+// items in order of the run first, so that CTAs working side by side read the
+// same few atom tiles. Pair c takes items c, c + pairs, ... A piece's
+// candidates go to its own list, merged before the rescoring.
+struct ScreenWork {
+    int n_tiles;  // atom tiles
+    int full, split, pieces, run;
+    int k_tiles;  // contraction tiles of one part
+    int parts;    // atom matrices side by side along the contraction (hi, lo)
+    int k_step;   // columns from one part to the next
+    int na, nb;   // slots
+    bool resident;
+};
+
+struct ScreenItem {
+    int row_pair, piece, begin, end;
+};
+
+__host__ __device__ __forceinline__ int screen_items(const ScreenWork& w) {
+    return w.full + w.split * w.pieces;
+}
+
+__device__ __forceinline__ ScreenItem screen_item(const ScreenWork& w, int i) {
+    if (i < w.full) return {i, 0, 0, w.n_tiles};
+    const int j = i - w.full, piece = j / w.split;
+    const int begin = piece * w.run;
+    return {w.full + j % w.split, piece, begin, min(begin + w.run, w.n_tiles)};
+}
 
 #define TSG_LD32(r, taddr)                                                                         \
     asm volatile(                                                                                  \
@@ -115,121 +190,190 @@ struct ScreenShared {
           "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])             \
         : "r"(taddr))
 
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
     screen_kernel(const __grid_constant__ CUtensorMap qmap, const __grid_constant__ CUtensorMap amap,
-                  int64_t rows, int64_t atoms, int64_t stored_rows, int k_tiles, float* cand_score,
-                  int32_t* cand_index, int* error) {
+                  const __grid_constant__ ScreenWork w, int64_t rows, int64_t atoms,
+                  float* cand_score, int32_t* cand_index, int* error) {
     extern __shared__ uint8_t s_raw[];
-    uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
-    ScreenShared* sh = reinterpret_cast<ScreenShared*>(tiles + STAGES * STAGE_BYTES);
+    uint8_t* a_tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
+    uint8_t* b_tiles = a_tiles + w.na * SMEM_A;
+    ScreenShared* sh = reinterpret_cast<ScreenShared*>(b_tiles + w.nb * SMEM_B);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
-    const int64_t row0 = int64_t(blockIdx.x) * BM;
-    const int n_tiles = int((stored_rows + BN - 1) / BN);
+    const int items = screen_items(w);
+    const int rank = int(blockIdx.x) % kPair;
+    const int first_item = int(blockIdx.x) / kPair, item_step = int(gridDim.x) / kPair;
+    constexpr uint16_t kBoth = (1u << kPair) - 1;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->full[s])));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->empty[s])));
+        for (int s = 0; s < w.na; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->a_full[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->a_empty[s])));
+        }
+        for (int s = 0; s < w.nb; ++s) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->b_full[s])));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->b_empty[s])));
         }
         for (int b = 0; b < 2; ++b) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&sh->tfull[b])));
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&sh->tempty[b])),
-                         "r"(kEpilogueThreads));
+                         "r"(kPair * kEpilogueThreads / 32));
         }
         sh->abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                          smem_u32(&sh->tmem_base)),
                      "r"(TMEM_COLS));
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    pair_sync();  // both CTAs' barriers are set up
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = sh->tmem_base;
     volatile int* abort = &sh->abort;
+    auto give_up = [&](int stage) {
+        *abort = 1;
+        atomicExch(error, stage);
+    };
 
     if (warp == 0) {
         if (lane == 0) {
             // TMA producer.
-            int it = 0;
-            for (int n = 0; n < n_tiles && !*abort; ++n) {
-                for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!wait_parity(smem_u32(&sh->empty[s]), ph ^ 1)) {
-                        *abort = 1;
-                        atomicExch(error, 1);
-                        break;
-                    }
-                    const uint32_t full = smem_u32(&sh->full[s]);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full),
-                                 "r"(STAGE_BYTES)
+            // Both CTAs' bytes of a slot land on the first CTA's barrier,
+            // which that CTA arms for the sum.
+            auto fetch = [&](const CUtensorMap& map, uint8_t* slot, uint64_t* bar, int bytes, int x,
+                             int y) {
+                const uint32_t own = smem_u32(bar);
+                if (rank == 0)
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(own),
+                                 "r"(kPair * bytes)
                                  : "memory");
-                    const uint32_t a_dst = smem_u32(tiles + s * STAGE_BYTES);
-                    const uint32_t b_dst = a_dst + SMEM_A;
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-                        "[%0], [%1, {%2, %3}], [%4];" ::"r"(a_dst),
-                        "l"(reinterpret_cast<uint64_t>(&qmap)), "r"(kt * BK), "r"(int(row0)), "r"(full)
-                        : "memory");
-                    asm volatile(
-                        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-                        "[%0], [%1, {%2, %3}], [%4];" ::"r"(b_dst),
-                        "l"(reinterpret_cast<uint64_t>(&amap)), "r"(kt * BK), "r"(n * BN), "r"(full)
-                        : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global"
+                    ".mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(slot)),
+                    "l"(reinterpret_cast<uint64_t>(&map)), "r"(x), "r"(y), "r"(first_cta(own))
+                    : "memory");
+            };
+            int as = 0, bs = 0;
+            uint32_t ap = 1, bp = 1;  // parity of the slots' release
+            for (int i = first_item; i < items && !*abort; i += item_step) {
+                const ScreenItem it = screen_item(w, i);
+                for (int n = it.begin; n < it.end && !*abort; ++n) {
+                    for (int kt = 0; kt < w.k_tiles && !*abort; ++kt) {
+                        if (!w.resident || n == it.begin) {
+                            if (!wait_parity(smem_u32(&sh->a_empty[as]), ap)) {
+                                give_up(1);
+                                break;
+                            }
+                            fetch(qmap, a_tiles + as * SMEM_A, &sh->a_full[as], SMEM_A, kt * BK,
+                                  (it.row_pair * kPair + rank) * BM);
+                            if (++as == w.na) {
+                                as = 0;
+                                ap ^= 1;
+                            }
+                        }
+                        for (int part = 0; part < w.parts; ++part) {
+                            if (!wait_parity(smem_u32(&sh->b_empty[bs]), bp)) {
+                                give_up(1);
+                                break;
+                            }
+                            fetch(amap, b_tiles + bs * SMEM_B, &sh->b_full[bs], SMEM_B,
+                                  part * w.k_step + kt * BK, n * BN + rank * (BN / kPair));
+                            if (++bs == w.nb) {
+                                bs = 0;
+                                bp ^= 1;
+                            }
+                        }
+                    }
+                }
+            }
+            // Every release of a slot, sent by the first CTA, has arrived
+            // before this CTA can end.
+            for (int j = 0; j < w.nb && !*abort; ++j) {
+                if (!wait_parity(smem_u32(&sh->b_empty[bs]), bp)) give_up(1);
+                if (++bs == w.nb) {
+                    bs = 0;
+                    bp ^= 1;
+                }
+            }
+            for (int j = 0; j < w.na && !*abort; ++j) {
+                if (!wait_parity(smem_u32(&sh->a_empty[as]), ap)) give_up(1);
+                if (++as == w.na) {
+                    as = 0;
+                    ap ^= 1;
                 }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            // MMA issuer.
-            int it = 0;
-            for (int n = 0; n < n_tiles && !*abort; ++n) {
-                const int b = n & 1;
-                const uint32_t use = uint32_t(n >> 1);
-                if (!wait_parity(smem_u32(&sh->tempty[b]), (use & 1) ^ 1)) {
-                    *abort = 1;
-                    atomicExch(error, 2);
-                    break;
-                }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d = tmem + uint32_t(b * BN);
-                for (int kt = 0; kt < k_tiles; ++kt, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1;
-                    if (!wait_parity(smem_u32(&sh->full[s]), ph)) {
-                        *abort = 1;
-                        atomicExch(error, 3);
+        if (lane == 0 && rank == 0) {
+            // MMA issuer, for the pair. A commit arrives on both CTAs' barrier.
+            auto commit = [&](uint64_t* bar) {
+                asm volatile(
+                    "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster"
+                    ".multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                    "h"(kBoth)
+                    : "memory");
+            };
+            int as = 0, bs = 0;
+            uint32_t ap = 0, bp = 0;
+            int t = 0;  // tiles so far: the accumulator is t & 1
+            for (int i = first_item; i < items && !*abort; i += item_step) {
+                const ScreenItem it = screen_item(w, i);
+                for (int n = it.begin; n < it.end && !*abort; ++n, ++t) {
+                    const int b = t & 1;
+                    if (!wait_parity(smem_u32(&sh->tempty[b]), ((t >> 1) & 1) ^ 1)) {
+                        give_up(2);
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint32_t a_addr = smem_u32(tiles + s * STAGE_BYTES);
-                    const uint32_t b_addr = a_addr + SMEM_A;
+                    const uint32_t d = tmem + uint32_t(b * BN);
+                    uint32_t acc = 0;
+                    for (int kt = 0; kt < w.k_tiles && !*abort; ++kt) {
+                        int slot = kt;
+                        if (!w.resident || n == it.begin) {
+                            if (!wait_parity(smem_u32(&sh->a_full[as]), ap)) {
+                                give_up(3);
+                                break;
+                            }
+                            slot = as;
+                            if (++as == w.na) {
+                                as = 0;
+                                ap ^= 1;
+                            }
+                        }
+                        const uint32_t a_addr = smem_u32(a_tiles + slot * SMEM_A);
+                        for (int part = 0; part < w.parts; ++part) {
+                            if (!wait_parity(smem_u32(&sh->b_full[bs]), bp)) {
+                                give_up(3);
+                                break;
+                            }
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            const uint32_t b_addr = smem_u32(b_tiles + bs * SMEM_B);
 #pragma unroll
-                    for (int j = 0; j < BK / 16; ++j) {
-                        const uint64_t adesc = tile_desc(a_addr + j * 32);
-                        const uint64_t bdesc = tile_desc(b_addr + j * 32);
-                        const uint32_t acc = (kt > 0 || j > 0) ? 1u : 0u;
-                        asm volatile(
-                            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-                            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
-                            "l"(adesc), "l"(bdesc), "r"(kInstr), "r"(acc)
-                            : "memory");
+                            for (int j = 0; j < BK / 16; ++j) {
+                                const uint64_t adesc = tile_desc(a_addr + j * 32);
+                                const uint64_t bdesc = tile_desc(b_addr + j * 32);
+                                asm volatile(
+                                    "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+                                    "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+                                    "l"(adesc), "l"(bdesc), "r"(kInstr), "r"(acc)
+                                    : "memory");
+                                acc = 1;
+                            }
+                            commit(&sh->b_empty[bs]);
+                            if (++bs == w.nb) {
+                                bs = 0;
+                                bp ^= 1;
+                            }
+                        }
+                        if (!w.resident || n + 1 == it.end) commit(&sh->a_empty[slot]);
                     }
-                    asm volatile(
-                        "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                            smem_u32(&sh->empty[s]))
-                        : "memory");
+                    if (*abort) break;
+                    commit(&sh->tfull[b]);
                 }
-                if (*abort) break;
-                asm volatile(
-                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                        smem_u32(&sh->tfull[b]))
-                    : "memory");
             }
         }
     } else {
@@ -241,75 +385,100 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int half = (warp - 2) / 4;
         const int r = quarter * 32 + lane;
         const int parity = lane & 1;
-        float best_s[kScreen];
-        int best_i[kScreen];
+        const int64_t whole = atoms & ~int64_t(63);  // rows below hold atoms only
+        int t = 0;
+        for (int i = first_item; i < items && !*abort; i += item_step) {
+            const ScreenItem it = screen_item(w, i);
+            float best_s[kScreen];
+            int best_i[kScreen];
 #pragma unroll
-        for (int k = 0; k < kScreen; ++k) {
-            best_s[k] = -1.f;
-            best_i[k] = -1;
-        }
-        for (int n = 0; n < n_tiles && !*abort; ++n) {
-            const int b = n & 1;
-            const uint32_t use = uint32_t(n >> 1);
-            if (!wait_parity(smem_u32(&sh->tfull[b]), use & 1)) {
-                *abort = 1;
-                atomicExch(error, 4);
-                break;
+            for (int k = 0; k < kScreen; ++k) {
+                best_s[k] = -1.f;
+                best_i[k] = -1;
             }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-            for (int cc = 0; cc < BN / 64; ++cc) {
-                // The warp of half h takes the 32-column chunks of parity h.
-                const int c = 2 * cc + half;
-                uint32_t v[32];
-                const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(b * BN + c * 32);
-                TSG_LD32(v, taddr);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float sc[16];
-                float chunk_best = -1.f;
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float x0 = __uint_as_float(v[2 * j]), x1 = __uint_as_float(v[2 * j + 1]);
-                    // Send the partner the value of its column; keep our own.
-                    const float mine = parity ? x1 : x0;
-                    const float other = __shfl_xor_sync(0xffffffffu, parity ? x0 : x1, 1);
-                    sc[j] = fmaf(mine, mine, other * other);
-                    chunk_best = fmaxf(chunk_best, sc[j]);
+            for (int n = it.begin; n < it.end && !*abort; ++n, ++t) {
+                const int b = t & 1;
+                if (!wait_parity(smem_u32(&sh->tfull[b]), (t >> 1) & 1)) {
+                    give_up(4);
+                    break;
                 }
-                if (chunk_best > best_s[kScreen - 1]) {
-                    const int pos0 = n * BN + c * 32 + parity;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-                    for (int j = 0; j < 16; ++j) {
-                        const int atom = stored_atom(pos0 + 2 * j);
-                        const float score = sc[j];
-                        if (atom < atoms && score > best_s[kScreen - 1]) {
-                            best_s[kScreen - 1] = score;
-                            best_i[kScreen - 1] = atom;
+                for (int cc = 0; cc < BN / 64; ++cc) {
+                    // The warp of half h takes the 32-column chunks of parity h.
+                    const int c = 2 * cc + half;
+                    uint32_t v[32];
+                    const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(b * BN + c * 32);
+                    TSG_LD32(v, taddr);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    float sc[16];
+                    float chunk_best = -1.f;
 #pragma unroll
-                            for (int k = kScreen - 1; k > 0; --k) {
-                                if (best_s[k] > best_s[k - 1]) {
-                                    const float ts = best_s[k];
-                                    best_s[k] = best_s[k - 1];
-                                    best_s[k - 1] = ts;
-                                    const int ti = best_i[k];
-                                    best_i[k] = best_i[k - 1];
-                                    best_i[k - 1] = ti;
-                                }
-                            }
+                    for (int j = 0; j < 16; ++j) {
+                        const float x0 = __uint_as_float(v[2 * j]), x1 = __uint_as_float(v[2 * j + 1]);
+                        // Send the partner the value of its column; keep our own.
+                        const float mine = parity ? x1 : x0;
+                        const float other = __shfl_xor_sync(0xffffffffu, parity ? x0 : x1, 1);
+                        sc[j] = fmaf(mine, mine, other * other);
+                        chunk_best = fmaxf(chunk_best, sc[j]);
+                    }
+                    const int pos0 = n * BN + c * 32 + parity;
+                    if (n * BN + c * 32 + 32 > whole) {
+                        // The last atoms' block: rows past the end do not count.
+                        chunk_best = -1.f;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (stored_atom(pos0 + 2 * j) >= atoms) sc[j] = -1.f;
+                            chunk_best = fmaxf(chunk_best, sc[j]);
+                        }
+                    }
+                    // Each round takes every lane's best remaining score at
+                    // once, so the warp pays for the lane with the most.
+                    while (__any_sync(0xffffffffu, chunk_best > best_s[kScreen - 1])) {
+                        const float score = chunk_best;
+                        const bool take = score > best_s[kScreen - 1];
+                        int at = 0;
+                        float rest = -1.f;
+#pragma unroll
+                        for (int j = 15; j >= 0; --j) {
+                            if (sc[j] == score) at = j;
+                        }
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            if (j == at) sc[j] = -1.f;
+                            rest = fmaxf(rest, sc[j]);
+                        }
+                        chunk_best = rest;
+                        const int atom = stored_atom(pos0 + 2 * at);
+                        best_s[kScreen - 1] = take ? score : best_s[kScreen - 1];
+                        best_i[kScreen - 1] = take ? atom : best_i[kScreen - 1];
+#pragma unroll
+                        for (int k = kScreen - 1; k > 0; --k) {
+                            const bool up = best_s[k] > best_s[k - 1];
+                            const float hi = up ? best_s[k] : best_s[k - 1];
+                            const float lo = up ? best_s[k - 1] : best_s[k];
+                            const int hi_i = up ? best_i[k] : best_i[k - 1];
+                            const int lo_i = up ? best_i[k - 1] : best_i[k];
+                            best_s[k - 1] = hi;
+                            best_s[k] = lo;
+                            best_i[k - 1] = hi_i;
+                            best_i[k] = lo_i;
                         }
                     }
                 }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) arrive_cluster(first_cta(smem_u32(&sh->tempty[b])));
             }
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            arrive(smem_u32(&sh->tempty[b]));
-        }
-        const int64_t row = row0 + (r & ~1);
-        if (row < rows) {
-            const int64_t voxel = row >> 1;
+            const int64_t row = int64_t(it.row_pair * kPair + rank) * BM + (r & ~1);
+            if (row < rows && !*abort) {
+                const int64_t at = (int64_t(it.piece) * (rows >> 1) + (row >> 1)) * kCand +
+                                   (half * 2 + parity) * kScreen;
 #pragma unroll
-            for (int k = 0; k < kScreen; ++k) {
-                cand_score[voxel * kCand + (half * 2 + parity) * kScreen + k] = best_s[k];
-                cand_index[voxel * kCand + (half * 2 + parity) * kScreen + k] = best_i[k];
+                for (int k = 0; k < kScreen; ++k) {
+                    cand_score[at + k] = best_s[k];
+                    cand_index[at + k] = best_i[k];
+                }
             }
         }
     }
@@ -319,63 +488,247 @@ __global__ void __launch_bounds__(kThreads, 1)
         // Let copies and products in flight land before the memory goes away.
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
     }
+    // The other CTA may still copy into this one's slots and arrive on its
+    // barriers until it is done too.
+    pair_sync();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (warp == 1)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                      "r"(TMEM_COLS));
 }
 
-// Exact FP32 rescoring of each voxel's screened candidates against the complex
-// normalized signal and atoms; keeps the best `top_k` in descending order.
-// One warp per voxel: lanes stride over the samples.
-__global__ void rescore_kernel(const float2* __restrict__ signals, const float2* __restrict__ atoms,
-                               int64_t voxels, int64_t samples, const int32_t* __restrict__ cand,
-                               int top_k, float* __restrict__ scores, int64_t* __restrict__ index) {
+// Two fp16 rows per normalized signal (see the head of this file), scaled,
+// zero-padded to `k` columns. One warp per voxel.
+__global__ void query_kernel(const float2* __restrict__ signals, int64_t voxels, int64_t samples,
+                             int64_t k, float scale, bool complex_atoms, __half* __restrict__ out) {
     const int64_t voxel = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (voxel >= voxels) return;
     const float2* s = signals + voxel * samples;
-    float best_s[kCand];
-    int best_i[kCand];
-#pragma unroll 4
-    for (int k = 0; k < kCand; ++k) {
-        const int a = cand[voxel * kCand + k];
-        float re = 0.f, im = 0.f;
-        if (a >= 0) {
-            const float2* d = atoms + int64_t(a) * samples;
-            for (int64_t p = lane; p < samples; p += 32) {
-                const float2 x = s[p], y = d[p];
-                // s * conj(d)
-                re = fmaf(x.x, y.x, fmaf(x.y, y.y, re));
-                im = fmaf(x.y, y.x, fmaf(-x.x, y.y, im));
+    __half* a = out + 2 * voxel * k;
+    __half* b = a + k;
+    for (int64_t p = lane; p < k; p += 32) {
+        float x = 0.f, y = 0.f;
+        if (p < samples) {
+            const float2 v = s[p];
+            x = v.x;
+            y = v.y;
+        } else if (complex_atoms && p < 2 * samples) {
+            const float2 v = s[p - samples];
+            x = v.y;
+            y = -v.x;
+        }
+        a[p] = __float2half_rn(x * scale);
+        b[p] = __float2half_rn(y * scale);
+    }
+}
+
+// Keeps in (s, x) the best kScreen of two lists sorted best first, ties to the
+// first: the larger of opposite ends is the set, as a bitonic sequence.
+__device__ __forceinline__ void merge_lists(float (&s)[kScreen], int (&x)[kScreen],
+                                            const float (&t)[kScreen], const int (&y)[kScreen]) {
+#pragma unroll
+    for (int k = 0; k < kScreen; ++k) {
+        const bool other = t[kScreen - 1 - k] > s[k];
+        s[k] = other ? t[kScreen - 1 - k] : s[k];
+        x[k] = other ? y[kScreen - 1 - k] : x[k];
+    }
+#pragma unroll
+    for (int half = kScreen / 2; half > 0; half >>= 1)
+#pragma unroll
+        for (int k = 0; k < kScreen; ++k) {
+            if (k & half) continue;
+            const bool swap = s[k + half] > s[k];
+            const float hi = swap ? s[k + half] : s[k], lo = swap ? s[k] : s[k + half];
+            const int hx = swap ? x[k + half] : x[k], lx = swap ? x[k] : x[k + half];
+            s[k] = hi;
+            s[k + half] = lo;
+            x[k] = hx;
+            x[k + half] = lx;
+        }
+}
+
+// The merged candidate of this lane (class lane / kScreen, rank lane %
+// kScreen) of `count` lists of the same voxel, `step` entries apart: per class
+// the best kScreen of the lists' (each sorted best first) -- what one list
+// over all the atoms would hold. A class's eight lanes look after every eighth
+// list each and hand out the best of their heads in turn.
+__device__ __forceinline__ int merged_candidate(const float* score, const int32_t* index, int64_t at,
+                                                int64_t step, int count, int lane) {
+    static_assert(kClasses * kScreen == 32 && kScreen == 8, "a lane per candidate");
+    if (count == 1) return index[at + lane];
+    const int g = lane & 7;
+    const int64_t mine0 = at + (lane & ~7);
+    float s[kScreen];
+    int x[kScreen];
+    auto read = [&](int list, float (&u)[kScreen], int (&v)[kScreen]) {
+#pragma unroll
+        for (int k = 0; k < kScreen; ++k) {
+            u[k] = list < count ? score[mine0 + list * step + k] : -2.f;
+            v[k] = list < count ? index[mine0 + list * step + k] : -1;
+        }
+    };
+    read(g, s, x);
+    for (int list = g + 8; list - g < count; list += 8) {
+        float t[kScreen];
+        int y[kScreen];
+        read(list, t, y);
+        merge_lists(s, x, t, y);
+    }
+    int mine = -1;
+#pragma unroll
+    for (int k = 0; k < kScreen; ++k) {
+        float best = s[0];
+        int from = g;
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1) {
+            const float o = __shfl_xor_sync(0xffffffffu, best, off);
+            const int f = __shfl_xor_sync(0xffffffffu, from, off);
+            if (o > best || (o == best && f < from)) {
+                best = o;
+                from = f;
+            }
+        }
+        const int atom = __shfl_sync(0xffffffffu, x[0], (lane & ~7) + from);
+        if (g == k) mine = atom;
+        const bool mine_won = g == from;
+#pragma unroll
+        for (int j = 0; j + 1 < kScreen; ++j) {
+            s[j] = mine_won ? s[j + 1] : s[j];
+            x[j] = mine_won ? x[j + 1] : x[j];
+        }
+        if (mine_won) {
+            s[kScreen - 1] = -2.f;
+            x[kScreen - 1] = -1;
+        }
+    }
+    return mine;
+}
+
+// Exact FP32 rescoring of each voxel's screened candidates against the complex
+// normalized signal and atoms; keeps the best `top_k` in descending order.
+// One warp per voxel: lanes stride over the samples. Bound by reading the
+// candidates' atoms, so a dictionary on one axis is read as its one part:
+// AXIS 0 complex atoms, 1 real, 2 on the imaginary axis (the products with
+// the other part, zero, leave the sums as they are).
+template <int AXIS>
+__global__ void rescore_kernel(const float2* __restrict__ signals, const void* __restrict__ atoms,
+                               int64_t voxels, int64_t samples, const float* __restrict__ list_score,
+                               const int32_t* __restrict__ list_index, int full_pairs, int pieces,
+                               int top_k, float* __restrict__ scores, int64_t* __restrict__ index) {
+    const int64_t voxel = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (voxel >= voxels) return;
+    const int count = 2 * voxel / (BM * kPair) < full_pairs ? 1 : pieces;
+    int mine = merged_candidate(list_score, list_index, voxel * kCand, voxels * kCand, count, lane);
+    const float2* s = signals + voxel * samples;
+    float my_score = -1.f;
+    // Four candidates at a time, whose loads overlap and share the signal's.
+    constexpr int kTogether = 4;
+#pragma unroll 1
+    for (int k = 0; k < kCand; k += kTogether) {
+        int atom[kTogether];
+        float re[kTogether], im[kTogether];
+        const void* row[kTogether];
+#pragma unroll
+        for (int j = 0; j < kTogether; ++j) {
+            atom[j] = __shfl_sync(0xffffffffu, mine, k + j);
+            re[j] = im[j] = 0.f;
+            const int64_t at = int64_t(max(atom[j], 0)) * samples;
+            row[j] = AXIS == 0 ? static_cast<const void*>(static_cast<const float2*>(atoms) + at)
+                               : static_cast<const void*>(static_cast<const float*>(atoms) + at);
+        }
+#pragma unroll 2
+        for (int64_t p = lane; p < samples; p += 32) {
+            const float2 x = s[p];
+#pragma unroll
+            for (int j = 0; j < kTogether; ++j) {
+                if constexpr (AXIS == 0) {
+                    const float2 y = static_cast<const float2*>(row[j])[p];
+                    // s * conj(d)
+                    re[j] = fmaf(x.x, y.x, fmaf(x.y, y.y, re[j]));
+                    im[j] = fmaf(x.y, y.x, fmaf(-x.x, y.y, im[j]));
+                } else {
+                    const float y = static_cast<const float*>(row[j])[p];
+                    if constexpr (AXIS == 1) {
+                        re[j] = fmaf(x.x, y, re[j]);
+                        im[j] = fmaf(x.y, y, im[j]);
+                    } else {
+                        re[j] = fmaf(x.y, y, re[j]);
+                        im[j] = fmaf(-x.x, y, im[j]);
+                    }
+                }
             }
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            re += __shfl_xor_sync(0xffffffffu, re, off);
-            im += __shfl_xor_sync(0xffffffffu, im, off);
+        for (int j = 0; j < kTogether; ++j) {
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                re[j] += __shfl_xor_sync(0xffffffffu, re[j], off);
+                im[j] += __shfl_xor_sync(0xffffffffu, im[j], off);
+            }
+            if (lane == k + j && atom[j] >= 0) my_score = sqrtf(re[j] * re[j] + im[j] * im[j]);
         }
-        best_s[k] = a >= 0 ? sqrtf(re * re + im * im) : -1.f;
-        best_i[k] = a;
     }
-    if (lane != 0) return;
-    // Descending by score, ties to the lower atom index.
+    // Descending by score, ties to the lower atom index; -1 where none is left.
     for (int k = 0; k < top_k; ++k) {
-        int pick = k;
-        for (int j = k + 1; j < kCand; ++j) {
-            const bool better = best_s[j] > best_s[pick] ||
-                                (best_s[j] == best_s[pick] && best_i[j] >= 0 &&
-                                 (best_i[pick] < 0 || best_i[j] < best_i[pick]));
-            if (better) pick = j;
+        float best = my_score;
+        int atom = mine;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const float o = __shfl_xor_sync(0xffffffffu, best, off);
+            const int a = __shfl_xor_sync(0xffffffffu, atom, off);
+            if (o > best || (o == best && a >= 0 && (atom < 0 || a < atom))) {
+                best = o;
+                atom = a;
+            }
         }
-        const float ts = best_s[k];
-        best_s[k] = best_s[pick];
-        best_s[pick] = ts;
-        const int ti = best_i[k];
-        best_i[k] = best_i[pick];
-        best_i[pick] = ti;
-        scores[voxel * top_k + k] = best_s[k];
-        index[voxel * top_k + k] = best_i[k];
+        if (lane == 0) {
+            scores[voxel * top_k + k] = best;
+            index[voxel * top_k + k] = atom;
+        }
+        if (mine == atom) {
+            my_score = -1.f;
+            mine = -1;
+        }
+    }
+}
+
+// What goes with the atoms found: the least-squares scale <d, s> / |d|^2 of
+// the signals as given, its size from the score, and the atoms' parameters.
+// One warp per voxel and place.
+__global__ void result_kernel(const float2* __restrict__ signals, const float* __restrict__ norms,
+                              int64_t found, int64_t samples, int top_k, int64_t atoms,
+                              const float2* __restrict__ dictionary, const float* __restrict__ power,
+                              const float* __restrict__ scores, const int64_t* __restrict__ index,
+                              const float* __restrict__ table, int columns,
+                              float2* __restrict__ scales, float* __restrict__ densities,
+                              float* __restrict__ parameters) {
+    const int64_t i = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= found) return;
+    const int64_t voxel = i / top_k;
+    // A signal that matches nothing (a NaN in it) has index -1, which reads as
+    // the last atom, as indexing from the end does.
+    const int64_t atom = index[i] < 0 ? atoms - 1 : index[i];
+    const float2* s = signals + voxel * samples;
+    const float2* d = dictionary + atom * samples;
+    float re = 0.f, im = 0.f;
+    for (int64_t p = lane; p < samples; p += 32) {
+        const float2 x = s[p], y = d[p];
+        re = fmaf(x.x, y.x, fmaf(x.y, y.y, re));
+        im = fmaf(x.y, y.x, fmaf(-x.x, y.y, im));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        re += __shfl_xor_sync(0xffffffffu, re, off);
+        im += __shfl_xor_sync(0xffffffffu, im, off);
+    }
+    for (int c = lane; c < columns; c += 32) parameters[i * columns + c] = table[atom * columns + c];
+    if (lane == 0) {
+        const float pw = power[atom];
+        scales[i] = make_float2(re / pw, im / pw);
+        densities[i] = norms[voxel] * scores[i] / sqrtf(pw);
     }
 }
 
@@ -422,35 +775,111 @@ extern "C" int tsg_match_screen_rows(int64_t atom_count) {
     return int((atom_count + 63) / 64 * 64);
 }
 
-extern "C" int tsg_match_screen(const void* queries, int64_t query_rows, const void* atoms,
-                                int64_t atom_count, int64_t k, float* candidate_scores,
-                                int32_t* candidate_index, int* error, void* stream) {
+namespace tsg {
+namespace {
+
+int match_sms() {
+    int dev = 0, n = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return n > 0 ? n : 1;
+}
+
+// The work split over the CTA pairs of `sms` SMs. Row pairs that fill whole
+// waves stay whole; the rest are cut so that the last waves are full: the number of
+// pieces that minimises waves x (piece + 2 tiles of filling and draining the
+// pipeline), up to 32 lists a voxel and at least 8 tiles a piece. At 16,384
+// voxels x 65,536 atoms (256 row tiles, 256 atom tiles, 152 SMs) two waves of
+// 256 tiles become 256 + 3 x 64; at 1,024 voxels one wave of 256 becomes 29.
+ScreenWork plan_screen(int64_t query_rows, int64_t atom_count, int64_t k, int parts, int sms,
+                       bool may_split) {
+    ScreenWork w{};
+    const int pairs = int((query_rows + kPair * BM - 1) / (kPair * BM));
+    const int slots = std::max(1, sms / kPair);
+    const int64_t stored = (atom_count + 63) / 64 * 64;
+    w.n_tiles = int((stored + BN - 1) / BN);
+    w.parts = parts;
+    w.k_step = int(k);
+    w.k_tiles = int((k + BK - 1) / BK);
+    w.resident = w.k_tiles <= kResident;
+    w.na = w.resident ? w.k_tiles : 4;
+    w.nb = std::min(kMaxB, (kTileBytes - w.na * SMEM_A) / SMEM_B);
+    w.full = may_split ? pairs / slots * slots : pairs;
+    w.split = pairs - w.full;
+    w.pieces = 1;
+    w.run = w.n_tiles;
+    double best = 1e300;
+    for (int p = 1; w.split > 0 && p <= 32 && (p == 1 || w.n_tiles / p >= 8); ++p) {
+        const int run = (w.n_tiles + p - 1) / p;
+        const int pieces = (w.n_tiles + run - 1) / run;  // none empty
+        const int64_t waves = (int64_t(w.split) * pieces + slots - 1) / slots;
+        const double cost = double(waves) * (run + 2);
+        if (cost < best) {
+            best = cost;
+            w.run = run;
+            w.pieces = pieces;
+        }
+    }
+    return w;
+}
+
+int check_screen(const void* queries, int64_t query_rows, const void* atoms, int64_t atom_count,
+                 int64_t k, const void* scores, const void* index, const void* error) {
     if (query_rows < 0 || atom_count < 0 || k < 1)
         return fail(TSG_ERR_ARGUMENT, "invalid matching dimensions");
     if (query_rows % 2) return fail(TSG_ERR_ARGUMENT, "queries come as two rows per voxel");
     if (k % 8) return fail(TSG_ERR_ARGUMENT, "the inner dimension must be a multiple of 8 (16 bytes)");
     if (query_rows == 0) return TSG_OK;
-    if (!queries || !atoms || !candidate_scores || !candidate_index || !error)
+    if (!queries || !atoms || !scores || !index || !error)
         return fail(TSG_ERR_ARGUMENT, "null matching buffer");
     if ((reinterpret_cast<uintptr_t>(queries) | reinterpret_cast<uintptr_t>(atoms)) & 15)
         return fail(TSG_ERR_ARGUMENT, "matrices must be 16-byte aligned");
     if (atom_count == 0) return fail(TSG_ERR_ARGUMENT, "empty dictionary");
-    if (query_rows > (int64_t(1) << 31) || atom_count > (int64_t(1) << 31) - BN)
+    if (query_rows > (int64_t(1) << 31) - BM || atom_count > (int64_t(1) << 31) - BN ||
+        k > (int64_t(1) << 29))
         return fail(TSG_ERR_CAPACITY, "matrix too large");
+    return TSG_OK;
+}
+
+int run_screen(const ScreenWork& w, const void* queries, int64_t query_rows, const void* atoms,
+               int64_t atom_count, int64_t k, float* scores, int32_t* index, int* error, int sms,
+               cudaStream_t stream) {
     CUtensorMap qmap, amap;
     const int64_t stored_rows = (atom_count + 63) / 64 * 64;
     int rc = tile_map(&qmap, queries, query_rows, k, BM);
-    if (!rc) rc = tile_map(&amap, atoms, stored_rows, k, BN);
+    if (!rc) rc = tile_map(&amap, atoms, stored_rows, k * w.parts, BN / kPair);
     if (rc) return rc;
-    const size_t smem = 1024 + STAGES * STAGE_BYTES + sizeof(ScreenShared);
+    const size_t smem = 1024 + w.na * SMEM_A + w.nb * SMEM_B + sizeof(ScreenShared);
     TSG_CUDA(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const int k_tiles = int((k + BK - 1) / BK);
-    const unsigned blocks = unsigned((query_rows + BM - 1) / BM);
-    screen_kernel<<<blocks, kThreads, smem, static_cast<cudaStream_t>(stream)>>>(
-        qmap, amap, query_rows, atom_count, stored_rows, k_tiles, candidate_scores,
-        candidate_index, error);
+    const int grid = kPair * std::min(std::max(1, sms / kPair), screen_items(w));
+    screen_kernel<<<unsigned(grid), kThreads, smem, stream>>>(
+        qmap, amap, w, query_rows, atom_count, scores, index, error);
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
+}
+
+template <int AXIS>
+void run_rescore(const void* signals, int64_t voxels, const void* atoms, int64_t samples,
+                 const float* list_score, const int32_t* list_index, int full_pairs, int pieces,
+                 int top_k, float* scores, int64_t* index, cudaStream_t stream) {
+    rescore_kernel<AXIS><<<unsigned((voxels * 32 + 255) / 256), 256, 0, stream>>>(
+        static_cast<const float2*>(signals), atoms, voxels, samples, list_score, list_index,
+        full_pairs, pieces, top_k, scores, index);
+}
+
+}  // namespace
+}  // namespace tsg
+
+extern "C" int tsg_match_screen(const void* queries, int64_t query_rows, const void* atoms,
+                                int64_t atom_count, int64_t k, float* candidate_scores,
+                                int32_t* candidate_index, int* error, void* stream) {
+    const int rc = check_screen(queries, query_rows, atoms, atom_count, k, candidate_scores,
+                                candidate_index, error);
+    if (rc || query_rows == 0) return rc;
+    const int sms = match_sms();
+    return run_screen(plan_screen(query_rows, atom_count, k, 1, sms, false), queries, query_rows, atoms,
+                      atom_count, k, candidate_scores, candidate_index, error, sms,
+                      static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tsg_match_rescore(const void* signals, int64_t voxels, const void* atoms,
@@ -462,11 +891,75 @@ extern "C" int tsg_match_rescore(const void* signals, int64_t voxels, const void
     if (voxels == 0) return TSG_OK;
     if (!signals || !atoms || !candidate_index || !scores || !index)
         return fail(TSG_ERR_ARGUMENT, "null rescoring buffer");
-    const int64_t threads = voxels * 32;
-    const unsigned blocks = unsigned((threads + 255) / 256);
-    rescore_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const float2*>(signals), static_cast<const float2*>(atoms), voxels, samples,
-        candidate_index, top_k, scores, index);
+    run_rescore<0>(signals, voxels, atoms, samples, nullptr, candidate_index, 0, 1, top_k, scores,
+                   index, static_cast<cudaStream_t>(stream));
+    TSG_CUDA(cudaGetLastError());
+    return TSG_OK;
+}
+
+extern "C" int tsg_match_queries(const void* normalized, int64_t voxels, int64_t samples, int64_t k,
+                                 float scale, int complex_atoms, void* queries, void* stream) {
+    if (voxels < 0 || samples < 1 || k < (complex_atoms ? 2 : 1) * samples)
+        return fail(TSG_ERR_ARGUMENT, "invalid query dimensions");
+    if (voxels == 0) return TSG_OK;
+    if (!normalized || !queries) return fail(TSG_ERR_ARGUMENT, "null matching buffer");
+    query_kernel<<<unsigned((voxels * 32 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const float2*>(normalized), voxels, samples, k, scale, complex_atoms != 0,
+        static_cast<__half*>(queries));
+    TSG_CUDA(cudaGetLastError());
+    return TSG_OK;
+}
+
+extern "C" int tsg_match_screen_lists(const void* queries, int64_t query_rows, const void* atoms,
+                                      int64_t atom_count, int64_t k, float* list_scores,
+                                      int32_t* list_index, int* error, void* stream) {
+    const int rc = check_screen(queries, query_rows, atoms, atom_count, k, list_scores, list_index,
+                                error);
+    if (rc || query_rows == 0) return rc;
+    const int sms = match_sms();
+    return run_screen(plan_screen(query_rows, atom_count, k, 2, sms, true), queries, query_rows, atoms,
+                      atom_count, k, list_scores, list_index, error, sms,
+                      static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tsg_match_lists(int64_t voxels, int64_t atom_count, int64_t k) {
+    if (voxels < 1 || atom_count < 1 || k < 1) return 1;
+    return plan_screen(2 * voxels, atom_count, k, 2, match_sms(), true).pieces;
+}
+
+extern "C" int tsg_match(const tsg_match_dictionary* d, const void* signals, const void* normalized,
+                         const float* norms, int64_t voxels, int top_k, void* queries,
+                         float* list_scores, int32_t* list_index, int* error, float* scores,
+                         int64_t* index, void* scales, float* densities, float* parameters,
+                         void* stream) {
+    if (!d || voxels < 0 || top_k < 1 || top_k > 8)
+        return fail(TSG_ERR_ARGUMENT, "invalid matching dimensions (top_k must be 1..8)");
+    if (d->samples < 1 || d->axis < 0 || d->axis > 2)
+        return fail(TSG_ERR_ARGUMENT, "invalid matching dictionary");
+    const int64_t need = d->axis == 0 ? 2 * d->samples : d->samples;
+    if (d->k < need) return fail(TSG_ERR_ARGUMENT, "the contraction is shorter than the signals");
+    const int rc = check_screen(queries, 2 * voxels, d->screen_atoms, d->atom_count, d->k, list_scores,
+                                list_index, error);
+    if (rc || voxels == 0) return rc;
+    if (!signals || !normalized || !norms || !scores || !index || !scales || !densities ||
+        !d->normalized_atoms || !d->dictionary || !d->power || (d->columns > 0 && (!d->table || !parameters)))
+        return fail(TSG_ERR_ARGUMENT, "null matching buffer");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int run = tsg_match_queries(normalized, voxels, d->samples, d->k, d->scale, d->axis == 0, queries, stream);
+    if (!run)
+        run = tsg_match_screen_lists(queries, 2 * voxels, d->screen_atoms, d->atom_count, d->k, list_scores,
+                                     list_index, error, stream);
+    if (run) return run;
+    const ScreenWork w = plan_screen(2 * voxels, d->atom_count, d->k, 2, match_sms(), true);
+    auto rescore = d->axis == 0 ? &run_rescore<0> : (d->axis == 1 ? &run_rescore<1> : &run_rescore<2>);
+    rescore(normalized, voxels, d->normalized_atoms, d->samples, list_scores, list_index, w.full,
+            w.pieces, top_k, scores, index, s);
+    TSG_CUDA(cudaGetLastError());
+    const int64_t found = voxels * top_k;
+    result_kernel<<<unsigned((found * 32 + 255) / 256), 256, 0, s>>>(
+        static_cast<const float2*>(signals), norms, found, d->samples, top_k, d->atom_count,
+        static_cast<const float2*>(d->dictionary), d->power, scores, index, d->table,
+        int(d->columns), static_cast<float2*>(scales), densities, parameters);
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
 }

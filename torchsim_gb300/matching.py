@@ -221,11 +221,13 @@ class DictionaryMatcher:
         # A real dictionary (or one on the imaginary axis, as the MRF signal
         # 1j*s is) scores like its real profile: |<s, e^{i c} d>| = |<s, d>|.
         if not bool(im.ne(0).any()):
-            self._screen_atoms, self._complex_atoms = re, False
+            self._screen_atoms, self._axis = re, 1
         elif not bool(re.ne(0).any()):
-            self._screen_atoms, self._complex_atoms = im, False
+            self._screen_atoms, self._axis = im, 2
         else:
-            self._screen_atoms, self._complex_atoms = torch.cat((re, im), dim=1), True
+            self._screen_atoms, self._axis = torch.cat((re, im), dim=1), 0
+        # What the rescoring reads: the one part of atoms on an axis.
+        self._exact_atoms = (self.normalized if self._axis == 0 else self._screen_atoms).contiguous()
         # Each screen atom is a pair of fp16 rows, hi and lo = (atom - hi),
         # side by side along the contraction: the query meets both, so its
         # product is <q, atom> with the atom carried to ~22 bits. What rounding
@@ -262,17 +264,15 @@ class DictionaryMatcher:
             self.parameter_values = p
         return self
 
-    def _queries(self, s: torch.Tensor) -> torch.Tensor:
-        """Two fp16 rows per voxel whose products with the screen atoms are
-        Re and Im of <s, d>."""
-        if self._complex_atoms:
-            a = torch.cat((s.real, s.imag), dim=1)
-            b = torch.cat((s.imag, -s.real), dim=1)
-        else:
-            a, b = s.real, s.imag
-        rows = torch.stack((a, b), dim=1).reshape(2 * s.shape[0], a.shape[1])
-        rows = _pad8(rows * self._screen_scale).to(torch.float16)
-        return torch.cat((rows, rows), dim=1).contiguous()
+    def _prepared(self) -> _native.MatchDictionary:
+        """The dictionary as the kernels take it; the tensors stay on ``self``."""
+        table = self.parameter_values
+        atoms, samples = self.dictionary.shape
+        return _native.MatchDictionary(
+            self._screen_atoms.data_ptr(), self._exact_atoms.data_ptr(), self.dictionary.data_ptr(),
+            self.power.data_ptr(), None if table is None else table.data_ptr(), atoms, samples,
+            self._screen_atoms.shape[1] // 2, self._screen_scale, self._axis,
+            0 if table is None else table.shape[1])
 
     @torch.no_grad()
     def match(self, signals: torch.Tensor) -> MatchResult:
@@ -284,41 +284,54 @@ class DictionaryMatcher:
             raise ValueError("signal and dictionary contrast counts differ")
         sample_shape = signals.shape[:-1]
         flat = signals.reshape(-1, signals.shape[-1]).to(self.device, torch.complex64)
+        if self.grouping is not None:
+            return self._match_groups(flat, sample_shape)
         lib = _native.library()
         stream = torch.cuda.current_stream(self.device).cuda_stream
-        A, P = self.dictionary.shape
-        screen_k = self._screen_atoms.shape[1]  # rows: the padded, permuted atoms
+        prepared = self._prepared()
+        n, k = flat.shape[0], self.top_k
         m = lib.tsg_match_candidates()
         error = torch.zeros(1, dtype=torch.int32, device=self.device)
-        scores, indices = [], []
-        for chunk in flat.split(self.query_chunk_size):
+        scores = torch.empty((n, k), dtype=torch.float32, device=self.device)
+        indices = torch.empty((n, k), dtype=torch.int64, device=self.device)
+        scales = torch.empty((n, k), dtype=torch.complex64, device=self.device)
+        densities = torch.empty((n, k), dtype=torch.float32, device=self.device)
+        params = None
+        if self.parameter_values is not None:
+            params = torch.empty((n, k, prepared.columns), dtype=torch.float32, device=self.device)
+        for begin in range(0, n, self.query_chunk_size):
+            rows = slice(begin, min(begin + self.query_chunk_size, n))
+            chunk = flat[rows].contiguous()
             V = chunk.shape[0]
-            s_hat, _ = _normalized(chunk)
-            if self.grouping is not None:
-                ix, sc = _search_groups(s_hat, self.grouping, self.top_k, self.prune)
-                scores.append(sc)
-                indices.append(ix)
-                continue
-            queries = self._queries(s_hat)
-            cand_s = torch.empty((V, m), dtype=torch.float32, device=self.device)
-            cand_i = torch.empty((V, m), dtype=torch.int32, device=self.device)
-            _native.check(lib.tsg_match_screen(
-                queries.data_ptr(), 2 * V, self._screen_atoms.data_ptr(), A, screen_k,
-                cand_s.data_ptr(), cand_i.data_ptr(), error.data_ptr(), stream))
-            sc = torch.empty((V, self.top_k), dtype=torch.float32, device=self.device)
-            ix = torch.empty((V, self.top_k), dtype=torch.int64, device=self.device)
+            s_hat, norms = _normalized(chunk)
             s_hat = s_hat.contiguous()
-            _native.check(lib.tsg_match_rescore(
-                s_hat.data_ptr(), V, self.normalized.data_ptr(), A, P, cand_i.data_ptr(),
-                self.top_k, sc.data_ptr(), ix.data_ptr(), stream))
-            scores.append(sc)
-            indices.append(ix)
+            queries = torch.empty((2 * V, prepared.k), dtype=torch.float16, device=self.device)
+            lists = lib.tsg_match_lists(V, prepared.atom_count, prepared.k)
+            list_s = torch.empty((lists, V, m), dtype=torch.float32, device=self.device)
+            list_i = torch.empty((lists, V, m), dtype=torch.int32, device=self.device)
+            _native.check(lib.tsg_match(
+                ctypes.byref(prepared), chunk.data_ptr(), s_hat.data_ptr(), norms.data_ptr(), V, k,
+                queries.data_ptr(), list_s.data_ptr(), list_i.data_ptr(), error.data_ptr(),
+                scores[rows].data_ptr(), indices[rows].data_ptr(), scales[rows].data_ptr(),
+                densities[rows].data_ptr(), None if params is None else params[rows].data_ptr(),
+                stream))
         if int(error.item()) != 0:
             raise _native.NativeError(_native.TSG_ERR_CUDA,
                                       f"matching kernel stopped waiting (stage {int(error.item())})")
-        scores = torch.cat(scores) if scores else torch.empty((0, self.top_k), device=self.device)
-        indices = (torch.cat(indices) if indices
-                   else torch.empty((0, self.top_k), dtype=torch.int64, device=self.device))
+        shape = (*sample_shape, k)
+        return MatchResult(
+            parameters=None if params is None else params.reshape(*shape, prepared.columns),
+            indices=indices.reshape(shape), scores=scores.reshape(shape),
+            scales=scales.reshape(shape), densities=densities.reshape(shape))
+
+    def _match_groups(self, flat: torch.Tensor, sample_shape) -> MatchResult:
+        """The match through the groups, ``query_chunk_size`` voxels at a time."""
+        scores, indices = [], []
+        for chunk in flat.split(self.query_chunk_size):
+            ix, sc = _search_groups(_normalized(chunk)[0], self.grouping, self.top_k, self.prune)
+            scores.append(sc)
+            indices.append(ix)
+        scores, indices = torch.cat(scores), torch.cat(indices)
         signal_norm = torch.linalg.vector_norm(flat, dim=-1).clamp_min(torch.finfo(torch.float32).eps)
         densities = signal_norm[:, None] * scores / self.power[indices].sqrt()
         atoms = self.dictionary[indices]
