@@ -218,6 +218,21 @@ int tsg_program_view(const tsg_program* program, void* device_ops, tsg_program**
  * sequential float32 clock cursor (simulators/mrf.py:46-77) on the device. */
 int tsg_sequential_sum(const float* x, int64_t n, float* out, void* stream);
 
+/* The MRF train of flip_deg (deg, `pulses` of them) and TRs (ms: tr_count of
+ * them, one or one per pulse; tr_count 0: tr_value) starting at start_s, built
+ * on the device by the host builder's float32 arithmetic: the packed flip and
+ * duration buffers (1 + 4 pulses each) and the template's op table rebound to
+ * them. first_stamp_us is the first pulse's time. All DEVICE but the scalars. */
+int tsg_mrf_stream(const tsg_program* tmpl, const float* flip_deg, const float* tr_ms,
+                   int64_t tr_count, float tr_value, int64_t pulses, float start_s,
+                   float first_stamp_us, float* flip_rad, float* duration_s, void* device_ops,
+                   void* stream);
+/* Its transpose: cotangents of the two event buffers (nullable: zero) onto the
+ * flips and per-pulse TRs (nullable: not computed). */
+int tsg_mrf_stream_vjp(const float* flip_deg, int64_t pulses, const float* flip_cotangent,
+                       const float* duration_cotangent, float* flip_gradient, float* tr_gradient,
+                       void* stream);
+
 /* ---- device-resident kernels ------------------------------------------- */
 
 /* Complex forward (one pool, instant RF): RF and receiver phases of the

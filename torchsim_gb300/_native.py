@@ -120,6 +120,9 @@ SIGNATURES: dict[str, tuple] = {
                                 ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
     "tsg_program_rebind": (_int, [_vp, _vp, _vp, _vp, _vp]),
     "tsg_program_view": (_int, [_vp, _vp, ctypes.POINTER(_vp)]),
+    "tsg_mrf_stream": (_int, [_vp, _vp, _vp, _i64, ctypes.c_float, _i64, ctypes.c_float,
+                              ctypes.c_float, _vp, _vp, _vp, _vp]),
+    "tsg_mrf_stream_vjp": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp]),
     "tsg_sequential_sum": (_int, [_vp, _i64, _vp, _vp]),
     "tsg_epg_forward": (_int, [_vp, ctypes.POINTER(Tissue), _i64, _i64, _int, _vp, _vp,
                                ctypes.POINTER(Launch), _vp]),

@@ -396,6 +396,90 @@ __global__ void rebind_kernel(const Op* __restrict__ tmpl, const OpSource* __res
     out[i] = op;
 }
 
+// The whole MRF stream of a protocol and its program in one block: what
+// torchsim_gb300/sequence.py's host builder does in float32, value by value
+// (the played flips; the cursor as a left-to-right running sum of the TRs;
+// stamps in microseconds, their differences back to seconds), then the op
+// table (rebind_kernel). Latency-bound: one launch for some twenty
+// elementwise ones, the sum by one thread from shared memory.
+constexpr int kStreamChunk = 1024;
+constexpr int kStreamThreads = 256;
+__global__ void __launch_bounds__(kStreamThreads)
+    mrf_stream_kernel(const float* __restrict__ flip_deg, const float* __restrict__ tr_ms,
+                      int64_t tr_count, float tr_value, int64_t n, float start, float first_stamp,
+                      const Op* __restrict__ tmpl, const OpSource* __restrict__ src, int64_t ops,
+                      float* flip_ev, float* dur_ev, Op* __restrict__ out) {
+    __shared__ float s_cursor[kStreamChunk + 1];  // [0]: the pulse before the chunk
+    __shared__ float s_next;
+    if (threadIdx.x == 0) {
+        s_next = start;
+        flip_ev[0] = dur_ev[0] = 0.f;
+    }
+    auto stamp = [&](int64_t k, float cursor) { return k == 0 ? first_stamp : __fmul_rn(1e6f, cursor); };
+    for (int64_t base = 0; base < n; base += kStreamChunk) {
+        const int count = int(min(int64_t(kStreamChunk), n - base));
+        __syncthreads();
+        for (int i = threadIdx.x; i < count; i += kStreamThreads) {
+            const float tr = tr_count == 0 ? tr_value : tr_ms[tr_count == 1 ? 0 : base + i];
+            s_cursor[1 + i] = __fmul_rn(tr, 1e-3f);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float at = s_next;
+#pragma unroll 8
+            for (int i = 0; i < count; ++i) {
+                const float spacing = s_cursor[1 + i];
+                s_cursor[1 + i] = at;
+                at = __fadd_rn(at, spacing);
+            }
+            s_next = at;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i < count; i += kStreamThreads) {
+            const int64_t k = base + i;
+            const float now = stamp(k, s_cursor[1 + i]);
+            const float before = k == 0 ? 0.f : stamp(k - 1, s_cursor[i]);
+            const float angle = __fmul_rn(flip_deg[k], 0.017453292519943295f);
+            const float played = __fmul_rn(6.283185307179586f, fabsf(__fmul_rn(angle, 0.15915493667125702f)));
+            float* d = dur_ev + 1 + 4 * k;
+            float* f = flip_ev + 1 + 4 * k;
+            d[0] = __fmul_rn(__fadd_rn(now, -before), 1e-6f);
+            f[0] = played;
+            d[1] = d[2] = d[3] = f[1] = f[2] = f[3] = 0.f;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_cursor[0] = s_cursor[count];
+    }
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < ops; i += kStreamThreads) {
+        Op op = tmpl[i];
+        const OpSource s = src[i];
+        if ((op.code & OP_RELAX) && s.dt_event >= 0) op.dt = dur_ev[s.dt_event];
+        if (op_rf(op.code) == RF_ROTATE && s.rf_event >= 0) op.flip = flip_ev[s.rf_event];
+        out[i] = op;
+    }
+}
+
+// The stream's cotangents back onto flips (deg) and TRs (ms): the chain of the
+// played flip 2 pi |deg2rad(f) area| in its own order of roundings, and the
+// interval before pulse k + 1 as TR k (the last TR moves nothing).
+__global__ void mrf_stream_vjp_kernel(const float* __restrict__ flip_deg, int64_t n,
+                                      const float* __restrict__ g_flip_ev,
+                                      const float* __restrict__ g_dur_ev, float* __restrict__ g_flip,
+                                      float* __restrict__ g_tr) {
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    if (g_flip != nullptr) {
+        const float f = flip_deg[k];
+        const float sign = f > 0.f ? 1.f : (f < 0.f ? -1.f : (f == 0.f ? 0.f : f));
+        float g = g_flip_ev != nullptr ? g_flip_ev[1 + 4 * k] : 0.f;
+        g = __fmul_rn(__fmul_rn(g, 6.283185307179586f), sign);
+        g_flip[k] = __fmul_rn(__fmul_rn(g, 0.15915493667125702f), 0.017453292519943295f);
+    }
+    if (g_tr != nullptr)
+        g_tr[k] = k + 1 < n && g_dur_ev != nullptr ? __fmul_rn(g_dur_ev[5 + 4 * k], 1e-3f) : 0.f;
+}
+
 // x[0], x[0]+x[1], ... summed left to right in float32, one rounding per
 // addition, as a sequential loop on the host does.
 __global__ void sequential_sum_kernel(const float* __restrict__ x, int64_t n,
@@ -439,6 +523,37 @@ extern "C" int tsg_program_rebind(const tsg_program* tmpl, const float* duration
                     static_cast<cudaStream_t>(stream)>>>(
         tmpl->d_ops, tmpl->d_src, tmpl->host.ops, tmpl->host.events, total, duration_s, flip_rad,
         static_cast<Op*>(device_ops));
+    TSG_CUDA(cudaGetLastError());
+    return TSG_OK;
+}
+
+extern "C" int tsg_mrf_stream(const tsg_program* tmpl, const float* flip_deg, const float* tr_ms,
+                              int64_t tr_count, float tr_value, int64_t pulses, float start_s,
+                              float first_stamp_us, float* flip_rad, float* duration_s,
+                              void* device_ops, void* stream) {
+    if (!tmpl) return fail(TSG_ERR_ARGUMENT, "null program");
+    if (pulses < 1 || (tr_count != 0 && tr_count != 1 && tr_count != pulses))
+        return fail(TSG_ERR_ARGUMENT, "one TR, or one for each pulse");
+    if (tmpl->host.trains != 1 || tmpl->host.events != 1 + 4 * pulses)
+        return fail(TSG_ERR_ARGUMENT, "the template is not a train of this many pulses");
+    if (!flip_deg || (tr_count > 0 && !tr_ms) || !flip_rad || !duration_s ||
+        (tmpl->host.ops > 0 && !device_ops))
+        return fail(TSG_ERR_ARGUMENT, "null stream buffer");
+    mrf_stream_kernel<<<1, kStreamThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+        flip_deg, tr_ms, tr_count, tr_value, pulses, start_s, first_stamp_us, tmpl->d_ops, tmpl->d_src,
+        tmpl->host.ops, flip_rad, duration_s, static_cast<Op*>(device_ops));
+    TSG_CUDA(cudaGetLastError());
+    return TSG_OK;
+}
+
+extern "C" int tsg_mrf_stream_vjp(const float* flip_deg, int64_t pulses, const float* flip_cotangent,
+                                  const float* duration_cotangent, float* flip_gradient,
+                                  float* tr_gradient, void* stream) {
+    if (pulses < 1) return fail(TSG_ERR_ARGUMENT, "an MRF train needs at least one pulse");
+    if (flip_gradient && !flip_deg) return fail(TSG_ERR_ARGUMENT, "null flips");
+    if (!flip_gradient && !tr_gradient) return TSG_OK;
+    mrf_stream_vjp_kernel<<<unsigned((pulses + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+        flip_deg, pulses, flip_cotangent, duration_cotangent, flip_gradient, tr_gradient);
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
 }

@@ -818,18 +818,12 @@ class JacobianFunction(torch.autograd.Function):
         if grad_jac is None:
             grad_jac = torch.zeros((rows, kk, program.outputs), dtype=torch.complex64, device=dev)
         # Back to the kernel's column order.
-        seed = torch.empty_like(grad_jac)
-        seed[:, ctx.order] = grad_jac
-        curvature: dict[str, torch.Tensor] = {}
-        names = ("t1_ms", "t2_ms", "m0", "b1", "inversion")
-        for i, name in enumerate(names):
-            if need[4 + i]:
-                curvature[name] = torch.zeros(V, dtype=torch.float32, device=dev)
-        ev_shape = (program.trains, program.events.events)
-        if need[9]:
-            curvature["flip_rad"] = torch.zeros(ev_shape, dtype=torch.float32, device=dev)
-        if need[10]:
-            curvature["duration_s"] = torch.zeros(ev_shape, dtype=torch.float32, device=dev)
+        seed = grad_jac
+        if ctx.order != list(range(kk)):
+            seed = torch.empty_like(grad_jac)
+            seed[:, ctx.order] = grad_jac
+        names = ("t1_ms", "t2_ms", "m0", "b1", "inversion", "flip_rad", "duration_s")
+        curvature = zero_gradients([n for i, n in enumerate(names) if need[4 + i]], program, V, dev)
         if ctx.mask:
             design_reverse(program, tissue, ctx.states, ctx.mask, seed, traj,
                            seed_signal=grad_sig, with_m0=ctx.with_m0, curvature=curvature,
@@ -838,10 +832,7 @@ class JacobianFunction(torch.autograd.Function):
             second_reverse(program, tissue, ctx.states, ctx.directions, seed, traj, ws,
                            seed_signal=grad_sig, with_m0=ctx.with_m0, curvature=curvature,
                            launch=ctx.launch)
-        out = [None, None, None, None]
-        out += [curvature.get(n) for n in names]
-        out += [curvature.get("flip_rad"), curvature.get("duration_s")]
-        return tuple(out)
+        return (None, None, None, None, *(curvature.get(n) for n in names))
 
 
 # ---- gradients on the complex path ------------------------------------------
@@ -982,22 +973,12 @@ class EpgComplexFunction(torch.autograd.Function):
         need = ctx.needs_input_grad
         dev = grad_out.device
         V = tissue.voxels
-        names = ("t1_ms", "t2_ms", "m0", "b1", "inversion", "b1_phase_rad", "b0_hz")
-        grads: dict[str, torch.Tensor] = {}
-        for i, name in enumerate(names):
-            if need[3 + i]:
-                grads[name] = torch.zeros(V, dtype=torch.float32, device=dev)
-        ev_shape = (program.trains, program.events.events)
-        for i, name in enumerate(("flip_rad", "duration_s", "phase_rad")):
-            if need[10 + i]:
-                grads[name] = torch.zeros(ev_shape, dtype=torch.float32, device=dev)
+        grads = zero_gradients([n for i, n in enumerate(COMPLEX_GRAD_NAMES) if need[3 + i]], program,
+                               V, dev)
         # The output is 1j * s: the cotangent of s is -1j times the output's.
         adjoint_complex(program, tissue, ctx.states, -1j * grad_out, traj, grads,
                         _offaxis_of(ctx.keep), launch=ctx.launch)
-        out = [None, None, None]
-        out += [grads.get(n) for n in names]
-        out += [grads.get(n) for n in ("flip_rad", "duration_s", "phase_rad")]
-        return tuple(out)
+        return (None, None, None, *(grads.get(n) for n in COMPLEX_GRAD_NAMES))
 
 
 class EpgFunction(torch.autograd.Function):
@@ -1074,6 +1055,18 @@ class EpgFunction(torch.autograd.Function):
         return tuple(out)
 
 
+def zero_gradients(names: Sequence[str], program: Program, voxels: int,
+                   device: torch.device) -> dict[str, torch.Tensor]:
+    """A zeroed gradient of each of ``names``, per voxel or per (train, event),
+    all filled by one launch."""
+    events = (program.trains, program.events.events)
+    grads = {n: torch.empty(events if n in ("flip_rad", "duration_s", "phase_rad") else (voxels,),
+                            dtype=torch.float32, device=device) for n in names}
+    if grads:
+        torch._foreach_zero_(list(grads.values()))
+    return grads
+
+
 VJP_NAMES = ("t1_ms", "t2_ms", "m0", "b1", "inversion", "flip_rad", "duration_s")
 
 
@@ -1093,23 +1086,13 @@ class EpgVjpFunction(torch.autograd.Function):
     @staticmethod
     def forward(ctx, program, states, launch, c, ckpt, tissue, want, grad_out, t1, t2, m0, b1,
                 inv, flip_events, duration_events):
-        dev = grad_out.device
-        V = tissue.voxels
-        grads: dict[str, torch.Tensor] = {}
-        ev_shape = (program.trains, program.events.events)
-        for name, w in zip(VJP_NAMES, want, strict=True):
-            if w:
-                shape = ev_shape if name in ("flip_rad", "duration_s") else (V,)
-                grads[name] = torch.zeros(shape, dtype=torch.float32, device=dev)
+        grads = zero_gradients([n for n, w in zip(VJP_NAMES, want, strict=True) if w], program,
+                               tissue.voxels, grad_out.device)
         adjoint(program, tissue, states, grad_out.detach(), ckpt, c, grads, launch=launch)
         ctx.program, ctx.states, ctx.launch, ctx.tissue = program, states, launch, tissue
         ctx.save_for_backward(grad_out)
-        out = []
-        for name in VJP_NAMES:
-            g = grads.get(name)
-            shape = ev_shape if name in ("flip_rad", "duration_s") else (V,)
-            out.append(g if g is not None else torch.zeros(shape, dtype=torch.float32, device=dev))
-        return tuple(out)
+        ctx.set_materialize_grads(False)
+        return tuple(grads.get(name) for name in VJP_NAMES)
 
     @staticmethod
     def backward(ctx, *vs):

@@ -437,6 +437,152 @@ def sequential_sum(x: torch.Tensor) -> torch.Tensor:
 _templates: dict[tuple, Program] = {}
 
 
+def _mrf_template(n: int, ti: float, TI_ms: float, device: torch.device) -> Program:
+    """The compiled train of ``n`` pulses after ``ti`` seconds that device
+    streams rebind."""
+    key = (n, ti, device.index)
+    template = _templates.get(key)
+    if template is None:
+        template = program_for(mrf_events(np.full(n, 10.0, np.float32),
+                                          np.full(n, 10.0, np.float32), TI_ms=TI_ms), device)
+        _templates[key] = template
+    return template
+
+
+def _stream_in_one_kernel(flip_deg: Any, TR_ms: Any, device: torch.device):
+    """``(flips, TRs or None, TR value)`` where one kernel builds the stream:
+    float32 flips on ``device``, the TRs a number or float32 there too, one or
+    one per pulse; None for any other protocol."""
+    flip = flip_deg.detach()
+    if (flip.ndim != 1 or flip.numel() < 2 or flip.dtype != torch.float32
+            or flip.device != device):
+        return None
+    if isinstance(TR_ms, torch.Tensor):
+        tr = TR_ms.detach()
+        if (tr.dtype != torch.float32 or tr.device != device or tr.numel() not in (1, flip.numel())
+                or tr.ndim > 1):
+            return None
+        return flip.contiguous(), tr.contiguous(), 0.0
+    if isinstance(TR_ms, (int, float)):
+        return flip.contiguous(), None, float(TR_ms)
+    return None
+
+
+def _mrf_stream_kernel(template: Program, flip: torch.Tensor, tr: torch.Tensor | None,
+                       tr_value: float, ti: float):
+    """Flip and duration buffers ``(1, events)`` and the rebound op table of
+    :func:`mrf_stream_on_device`, by one kernel."""
+    n = flip.numel()
+    both = torch.empty((2, 1, 1 + 4 * n), dtype=torch.float32, device=flip.device)
+    ops = torch.empty((max(template.ops, 1), 4), dtype=torch.float32, device=flip.device)
+    _native.check(_native.library().tsg_mrf_stream(
+        template.handle, flip.data_ptr(), None if tr is None else tr.data_ptr(),
+        0 if tr is None else tr.numel(), tr_value, n, float(np.float32(ti)),
+        float(np.float32(1e6 * ti)), both[0].data_ptr(), both[1].data_ptr(), ops.data_ptr(),
+        torch.cuda.current_stream(flip.device).cuda_stream))
+    return both[0], both[1], ops
+
+
+class MrfStream(torch.autograd.Function):
+    """The device-built MRF stream as a function of the flips (deg) and TRs
+    (ms): the packed flip and duration buffers, and (not differentiable) the
+    program's op table. Its transpose is one kernel too; under
+    ``create_graph`` it is the same chain in differentiable operations."""
+
+    @staticmethod
+    def forward(ctx, flip, tr, tr_value, ti, template):
+        got = _mrf_stream_kernel(template, flip.detach().contiguous(),
+                                 None if tr is None else tr.detach().contiguous(), tr_value, ti)
+        ctx.mark_non_differentiable(got[2])
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(flip)
+        ctx.tr_shape = None if tr is None else tr.shape
+        return got
+
+    @staticmethod
+    def backward(ctx, g_flip_ev, g_dur_ev, _g_ops):
+        (flip,) = ctx.saved_tensors
+        grads = _stream_transpose(flip, g_flip_ev if ctx.needs_input_grad[0] else None,
+                                  g_dur_ev if ctx.needs_input_grad[1] else None)
+        return grads[0], _summed_to(grads[1], ctx.tr_shape), None, None, None
+
+
+class MrfEvents(torch.autograd.Function):
+    """The event buffers of a host-built MRF train (one playing), which carry
+    the values of the flips (deg) and TRs (ms) already, as a function of
+    these: the buffers as they are, with :class:`MrfStream`'s transpose."""
+
+    @staticmethod
+    def forward(ctx, flip, tr, flip_ev, dur_ev):
+        ctx.set_materialize_grads(False)
+        ctx.save_for_backward(flip)
+        ctx.tr = None if tr is None else (tr.shape, tr.device, tr.dtype)
+        return flip_ev.clone(), dur_ev.clone()
+
+    @staticmethod
+    def backward(ctx, g_flip_ev, g_dur_ev):
+        (flip,) = ctx.saved_tensors
+        if not ctx.needs_input_grad[0]:
+            g_flip_ev = None
+        if not ctx.needs_input_grad[1]:
+            g_dur_ev = None
+        some = g_flip_ev if g_flip_ev is not None else g_dur_ev
+        if some is None:
+            return (None,) * 4
+        g_flip, g_tr = _stream_transpose(flip.detach().to(some.device), g_flip_ev, g_dur_ev)
+        if g_flip is not None:
+            g_flip = g_flip.to(flip.device, flip.dtype)
+        if g_tr is not None:
+            g_tr = _summed_to(g_tr, ctx.tr[0]).to(ctx.tr[1], ctx.tr[2])
+        return g_flip, g_tr, None, None
+
+
+def _summed_to(g: torch.Tensor | None, shape: torch.Size | None) -> torch.Tensor | None:
+    """Per-pulse gradients for the TRs as they were given: one, or one each."""
+    if g is None:
+        return None
+    return g.sum().reshape(shape) if shape.numel() == 1 else g.reshape(shape)
+
+
+def _stream_transpose(flip: torch.Tensor, g_flip_ev: torch.Tensor | None,
+                      g_dur_ev: torch.Tensor | None):
+    """Cotangents of the event buffers (None: not wanted) back onto the flips
+    (deg, on the buffers' device) and the per-pulse TRs (ms)."""
+    n = flip.numel()
+    if torch.is_grad_enabled():
+        g_flip = g_tr = None
+        if g_flip_ev is not None:
+            played = g_flip_ev[0, 1::4] * (2.0 * torch.pi) * flip.detach().sgn()
+            g_flip = torch.deg2rad(played * _HARD_PULSE_AREA)
+        if g_dur_ev is not None:
+            g_tr = torch.cat((g_dur_ev[0, 5::4] * 1e-3, g_dur_ev.new_zeros(1)))
+        return g_flip, g_tr
+    if g_flip_ev is None and g_dur_ev is None:
+        return None, None
+    ev = [None if g is None else g.to(torch.float32).contiguous() for g in (g_flip_ev, g_dur_ev)]
+    out = [None if g is None else torch.empty(n, dtype=torch.float32, device=flip.device) for g in ev]
+    at = flip.detach().contiguous()
+    _native.check(_native.library().tsg_mrf_stream_vjp(
+        at.data_ptr(), n, *[None if t is None else t.data_ptr() for t in (*ev, *out)],
+        torch.cuda.current_stream(flip.device).cuda_stream))
+    return out
+
+
+def mrf_stream_with_gradients(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
+                              device: torch.device):
+    """:func:`mrf_stream_on_device` with the buffers carrying gradients to the
+    flips and TRs (:class:`MrfStream`), or None where that function's kernel
+    does not take the protocol."""
+    plain = _stream_in_one_kernel(flip_deg, TR_ms, device)
+    if plain is None:
+        return None
+    ti = float(TI_ms) * 1e-3
+    template = _mrf_template(flip_deg.numel(), ti, float(TI_ms), device)
+    flip, duration, ops = MrfStream.apply(
+        flip_deg, TR_ms if isinstance(TR_ms, torch.Tensor) else None, plain[2], ti, template)
+    return ProgramView(template, ops), flip, duration
+
+
 def mrf_stream_on_device(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
                          device: torch.device) -> tuple[ProgramView, torch.Tensor, torch.Tensor]:
     """The MRF train of :func:`mrf_events` (one playing, TI a number, zero
@@ -446,6 +592,11 @@ def mrf_stream_on_device(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
     the program by rebinding a template compiled once per (pulses, TI) with
     :func:`rebind`. Returns ``(program, flip (1, events), duration (1,
     events))``, the last two the packed event buffers on the device."""
+    one_kernel = _stream_in_one_kernel(flip_deg, TR_ms, device)
+    if one_kernel is not None:
+        template = _mrf_template(one_kernel[0].numel(), float(TI_ms) * 1e-3, float(TI_ms), device)
+        flip, duration, ops = _mrf_stream_kernel(template, *one_kernel, float(TI_ms) * 1e-3)
+        return ProgramView(template, ops), flip, duration
     angles = torch.deg2rad(torch.atleast_1d(flip_deg.detach()).to(device))
     if angles.ndim != 1:
         raise ValueError("flip must be one angle per repetition")
@@ -465,13 +616,7 @@ def mrf_stream_on_device(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
                          f"against {tuple(angles.shape)}")
     s32 = (tr * 1e-3).to(torch.float32)
     ti = float(TI_ms) * 1e-3
-    key = (n, ti, device.index)
-    template = _templates.get(key)
-    if template is None:
-        template = program_for(mrf_events(np.full(n, 10.0, np.float32),
-                                          np.full(n, 10.0, np.float32), TI_ms=float(TI_ms)),
-                               device)
-        _templates[key] = template
+    template = _mrf_template(n, ti, float(TI_ms), device)
     start = torch.full((1,), float(np.float32(ti)), dtype=torch.float32, device=device)
     cursor = sequential_sum(torch.cat((start, s32)))
     starts = cursor[:n] * np.float32(1e6)

@@ -26,8 +26,9 @@ import torch
 from torch.autograd import forward_ad
 
 from . import engine
-from .sequence import (POST_SHIFT, PRE_SHIFT, SHIFT_AFTER, PackedEvents, fse_events, mrf_events,
-                       mrf_gradient_map, mrf_stream_on_device, played_flip_torch, program_for)
+from .sequence import (POST_SHIFT, PRE_SHIFT, SHIFT_AFTER, MrfEvents, PackedEvents, fse_events,
+                       mrf_events, mrf_gradient_map, mrf_stream_on_device, mrf_stream_with_gradients,
+                       played_flip_torch, program_for)
 
 
 def _tracked(value: Any) -> bool:
@@ -41,6 +42,20 @@ def _tracked(value: Any) -> bool:
     if torch._C._functorch.is_functorch_wrapped_tensor(value):
         return True
     return forward_ad.unpack_dual(value).tangent is not None
+
+
+def _reverse_only(value: torch.Tensor) -> bool:
+    """A tracked tensor that carries no forward-mode tangent, outside any
+    function transform."""
+    return (not torch._C._are_functorch_transforms_active()
+            and not torch._C._functorch.is_functorch_wrapped_tensor(value)
+            and forward_ad.unpack_dual(value).tangent is None)
+
+
+def _plain_float(value: torch.Tensor, n: int) -> bool:
+    """A float32 vector of ``n`` (or one value) under reverse mode alone."""
+    return (_reverse_only(value) and value.dtype == torch.float32 and value.ndim <= 1
+            and value.numel() in (1, n))
 
 
 def _primal(value: Any) -> Any:
@@ -92,12 +107,16 @@ def _nonzero(value: Any) -> bool:
     return bool(np.any(np.asarray(value) != 0))
 
 
+def _turns(held: dict[str, Any]) -> bool:
+    """True when a voxel carries off-resonance or a transmit phase."""
+    return _nonzero(held.get("B0")) or _nonzero(held.get("B1phase"))
+
+
 def _leaves_real_subspace(events: PackedEvents, held: dict[str, Any]) -> bool:
     """True when the stream's pulses and samples do not share one phase, or a
     voxel carries off-resonance or a transmit phase: the complex kernel runs
     (the reference's real_axis verdict, sequence/_accelerators.py:1953-2128)."""
-    return (events.real_axis() != 1 or _nonzero(held.get("B0"))
-            or _nonzero(held.get("B1phase")))
+    return events.real_axis() != 1 or _turns(held)
 
 
 class _EpgSimulator:
@@ -148,6 +167,13 @@ class _EpgSimulator:
         built on the host."""
         return None
 
+    def _device_stream_with_gradients(self, protocol: dict[str, Any], repetitions: int,
+                                      device: torch.device):
+        """The same with the event buffers carrying gradients to the
+        protocol's tensors, or None where :meth:`_event_gradients` attaches
+        them."""
+        return None
+
     def _kernel_maps(self, held: dict[str, Any]) -> dict[str, Any]:
         return {
             "T1": held.get("T1"),
@@ -184,7 +210,9 @@ class _EpgSimulator:
                   else self.events(repetitions=repetitions, **protocol))
         # A derivative along B0 or B1phase leaves the real subspace too, as
         # the reference's verdict counts the tangents (_accelerators.py:3953-3966).
-        complex_path = (_leaves_real_subspace(events, held)
+        # (A stream built on the device has one phase, zero.)
+        complex_path = ((_turns(held) if on_device is not None
+                         else _leaves_real_subspace(events, held))
                         or bool(names and {"B0", "B1phase"} & set(names)))
         if complex_path and on_device is not None:
             on_device = None
@@ -289,13 +317,21 @@ class _EpgSimulator:
         plain = {k: _primal(v) for k, v in protocol.items()}
         # The event stream and the verdict are values, built outside any
         # function transform (torch.func.jvp wraps every tensor made inside).
+        # Reverse mode alone reaches flips and TRs through the stream's own
+        # transpose; forward mode and function transforms attach them below.
+        attached = None
+        moved = [v for v in protocol.values() if _tracked(v)]
+        if moved and all(_reverse_only(v) for v in moved):
+            attached = self._device_stream_with_gradients(protocol, repetitions, dev)
         with torch._C._DisableFuncTorch():
-            on_device = self._device_stream(plain, repetitions, dev)
+            on_device = (attached if attached is not None
+                         else self._device_stream(plain, repetitions, dev))
             events = (on_device[0].events if on_device is not None
                       else self.events(repetitions=repetitions, **plain))
-            complex_path = _leaves_real_subspace(events, held)
+            complex_path = (_turns(held) if on_device is not None
+                            else _leaves_real_subspace(events, held))
             if complex_path and on_device is not None:
-                on_device = None
+                attached = on_device = None
                 events = self.events(repetitions=repetitions, **plain)
         if complex_path and names:
             raise NotImplementedError(
@@ -333,15 +369,16 @@ class _EpgSimulator:
             with torch._C._DisableFuncTorch():
                 if on_device is not None and not complex_path:
                     program, flip_ev, dur_ev = on_device
-                    phase_ev = torch.zeros_like(flip_ev)
+                    phase_ev = None
                 else:
                     program = program_for(events, dev, phased=complex_path)
                     flip_ev = torch.from_numpy(events.flip).to(dev)
                     dur_ev = torch.from_numpy(events.duration).to(dev)
                     phase_ev = torch.from_numpy(np.array(
                         np.broadcast_to(events.phase, events.duration.shape), np.float32)).to(dev)
-            flip_ev, dur_ev, phase_ev = self._event_gradients(protocol, events, flip_ev, dur_ev,
-                                                              repetitions, phase_ev)
+            if attached is None:
+                flip_ev, dur_ev, phase_ev = self._event_gradients(protocol, events, flip_ev,
+                                                                  dur_ev, repetitions, phase_ev)
             tissue = (flat(maps["T1"], True, False), flat(maps["T2"], True, False),
                       flat(maps["M0"]), flat(maps["B1"]), flat(maps["inv"]))
             jac = None
@@ -433,6 +470,15 @@ class MRFSimulator(_EpgSimulator):
             return None
         return mrf_stream_on_device(flip, tr, float(ti), device)
 
+    def _device_stream_with_gradients(self, protocol, repetitions, device):
+        flip, ti, phases = (protocol.get("flip"), protocol.get("TI", 0.0),
+                            protocol.get("phases", 0.0))
+        if (not isinstance(flip, torch.Tensor) or repetitions != 1
+                or set(protocol) - {"flip", "TR", "TI", "phases"} or _tensorish(ti)
+                or _tensorish(phases) or float(phases) != 0.0):
+            return None
+        return mrf_stream_with_gradients(flip, protocol.get("TR"), float(ti), device)
+
     def _event_gradients(self, protocol, events, flip_ev, dur_ev, repetitions, phase_ev=None):
         flip = protocol.get("flip")
         tr = protocol.get("TR")
@@ -440,6 +486,16 @@ class MRFSimulator(_EpgSimulator):
         n = int(torch.atleast_1d(torch.as_tensor(
             _primal(flip) if isinstance(flip, torch.Tensor) else np.asarray(flip))).numel())
         dev = flip_ev.device
+        if _tracked(protocol.get("phases")):
+            raise NotImplementedError("MRFSimulator: gradients w.r.t. phases are not built")
+        moved = [v for v in (flip, tr) if _tracked(v)]
+        if (moved and repetitions == 1 and not _tracked(ti) and flip_ev.shape == (1, 1 + 4 * n)
+                and all(_plain_float(v, n) for v in moved)):
+            # Reverse mode alone: one transpose instead of a chain of
+            # elementwise operations. (The flips are read for their sign.)
+            at = flip if _tracked(flip) else flip_ev.new_zeros(n)
+            flip_ev, dur_ev = MrfEvents.apply(at, tr if _tracked(tr) else None, flip_ev, dur_ev)
+            return flip_ev, dur_ev, phase_ev
         with torch._C._DisableFuncTorch():
             where = _gradient_map_on(n, repetitions, dev)
         if _tracked(flip):
@@ -455,8 +511,6 @@ class MRFSimulator(_EpgSimulator):
             t = ti.to(dev, torch.float32).reshape(()) * 1e-3
             idx = where["ti"]
             dur_ev = dur_ev.index_add(1, idx, (t - t.detach()).expand(idx.numel())[None])
-        if _tracked(protocol.get("phases")):
-            raise NotImplementedError("MRFSimulator: gradients w.r.t. phases are not built")
         return flip_ev, dur_ev, phase_ev
 
 
