@@ -494,6 +494,17 @@ int tsg_epg_batched_forward(const void* ops, const tsg_batch_sequence* sequences
                             const tsg_tissue* tissue, void* out, int orders_per_lane,
                             int warps_per_block, int blocks, void* stream);
 
+/* Whether a compiled single-train program (HOST array of 16-byte ops) is a CPMG
+ * train the echo kernel runs: the excitation, then per echo one refocusing op
+ * and one recording op, one interval throughout, at most 64 echoes. */
+int tsg_echo_train(const void* host_ops, int64_t op_count);
+/* The CPMG trains of a batch, one voxel per lane: buffers as
+ * tsg_epg_batched_forward takes them, units of up to 64 voxels of sequences
+ * for which tsg_echo_train holds (lanes_per_voxel is not read). */
+int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* sequences,
+                         const tsg_batch_unit* units, int64_t unit_count, const tsg_tissue* tissue,
+                         void* out, void* stream);
+
 /* ---- Gauss-Newton mapping ---------------------------------------------- */
 
 /* One fused evaluation of Gauss-Newton normal equations (one train only):

@@ -6,10 +6,12 @@ different echo-train lengths and voxel counts is as many launches, each sized
 to its own problem, with a tail of idle SMs after every small one.
 :class:`SequenceBatch` packs all of them into one table: the sequences'
 compiled programs back to back, their tissue back to back, and a list of
-(sequence, voxel tile) units sorted largest first. A single launch of the
-persistent kernel (``tsg_epg_batched_forward``) works through the list; the
-launch and the counter reset are captured once in a CUDA graph and replayed.
-The launch shape (orders per lane, warps per CTA, CTAs per SM) is picked by
+(sequence, voxel tile) units sorted largest first. CPMG trains (the excitation,
+then per echo one refocusing pulse and one sample) run one voxel per lane with
+only the orders that matter at each echo (``tsg_epg_echo_forward``); a single
+launch of the persistent kernel (``tsg_epg_batched_forward``) works through the
+other sequences' units. The launches and the counter reset are captured once in
+a CUDA graph and replayed. The persistent launch's shape (orders per lane, warps per CTA, CTAs per SM) is picked by
 :mod:`torchsim_gb300.autotune`.
 """
 
@@ -50,6 +52,10 @@ def compile_ops(events: PackedEvents) -> np.ndarray:
                                        code.ctypes.data, n_ops.value))
     ops["dt"], ops["flip"], ops["record"], ops["code"] = dt, fl, rec, code
     return ops
+
+
+# Voxels per unit of the echo kernel: two warps, one voxel per lane.
+ECHO_UNIT = 64
 
 
 @dataclass
@@ -105,6 +111,11 @@ class SequenceBatch:
         total = int((self.voxels * self.outputs).sum())
         self.out = torch.empty(total, dtype=torch.complex64, device=device)
         self.counter = torch.zeros(1, dtype=torch.int32, device=device)
+        # CPMG trains run one voxel per lane (tsg_epg_echo_forward), the other
+        # sequences the persistent kernel.
+        lib = _native.library()
+        self.echo = np.array([bool(lib.tsg_echo_train(p.ctypes.data, len(p))) for p in programs], bool)
+        self._echo_tables: tuple | None = None
         self.shape: tuple[int, int, int] | None = None
         self.graph: torch.cuda.CUDAGraph | None = None
         self._tables: dict[tuple, tuple] = {}
@@ -114,13 +125,7 @@ class SequenceBatch:
         """voxel x pulse x state updates of one pass (pulses = recorded echoes)."""
         return int((self.voxels * self.outputs * self.states).sum())
 
-    def _plan(self, orders: int, warps: int) -> tuple:
-        key = (orders, warps)
-        if key in self._tables:
-            return self._tables[key]
-        lanes = -(-self.states // orders)
-        if (lanes > 32).any():
-            raise ValueError(f"orders_per_lane {orders} cannot hold {int(self.states.max())} states")
+    def _sequences(self, lanes) -> np.ndarray:
         seq = np.zeros(len(self.entries), np.dtype([
             ("op_offset", "<i4"), ("op_count", "<i4"), ("states", "<i4"), ("lanes", "<i4"),
             ("outputs", "<i4"), ("voxel_count", "<i4"), ("voxel_offset", "<i8"),
@@ -128,40 +133,70 @@ class SequenceBatch:
         seq["op_offset"], seq["op_count"], seq["states"] = self.op_offset, self.op_count, self.states
         seq["lanes"], seq["outputs"], seq["voxel_count"] = lanes, self.outputs, self.voxels
         seq["voxel_offset"], seq["output_offset"] = self.voxel_offset, self.output_offset
-        per_unit = warps * (32 // lanes)
-        counts = -(-self.voxels // per_unit)
+        return seq
+
+    def _units(self, which: np.ndarray, per_unit: np.ndarray, cost: np.ndarray):
+        """(sequence, first voxel, voxel count) units of the sequences
+        ``which``, ``per_unit`` voxels each, the costliest sequences first; on
+        the device, with their number."""
+        counts = np.where(which, -(-self.voxels // per_unit), 0)
         seq_of = np.repeat(np.arange(len(self.entries)), counts)
         first = np.cumsum(np.concatenate([[0], counts]))[:-1]
         begin = (np.arange(int(counts.sum())) - np.repeat(first, counts)) * per_unit[seq_of]
         count = np.minimum(per_unit[seq_of], self.voxels[seq_of] - begin)
+        order = np.argsort(-cost[seq_of], kind="stable")
+        units = np.stack([seq_of, begin, count, np.zeros_like(count)], axis=1).astype(np.int32)[order]
+        return (torch.from_numpy(np.ascontiguousarray(units).view(np.uint8)).to(self.device),
+                int(units.shape[0]))
+
+    def _plan(self, orders: int, warps: int) -> tuple:
+        key = (orders, warps)
+        if key in self._tables:
+            return self._tables[key]
+        lanes = np.where(self.echo, 1, -(-self.states // orders))
+        if (lanes > 32).any():
+            raise ValueError(f"orders_per_lane {orders} cannot hold {int(self.states.max())} states")
+        d_seq = torch.from_numpy(self._sequences(lanes).view(np.uint8)).to(self.device)
         # Every unit holds a CTA for (ops x padded orders) steps: largest first.
-        cost = self.op_count[seq_of] * lanes[seq_of] * orders
-        order = np.argsort(-cost, kind="stable")
-        unit_arr = np.stack([seq_of, begin, count, np.zeros_like(count)], axis=1).astype(np.int32)
-        unit_arr = unit_arr[order]
-        units = unit_arr
-        d_seq = torch.from_numpy(seq.view(np.uint8)).to(self.device)
-        d_units = torch.from_numpy(np.ascontiguousarray(unit_arr).view(np.uint8)).to(self.device)
-        self._tables[key] = (d_seq, d_units, int(units.shape[0]))
+        units = self._units(~self.echo, warps * (32 // lanes), self.op_count * lanes * orders)
+        self._tables[key] = (d_seq, *units)
         return self._tables[key]
 
+    def _echo_plan(self) -> tuple:
+        if self._echo_tables is None:
+            d_seq = torch.from_numpy(self._sequences(1).view(np.uint8)).to(self.device)
+            reached = np.minimum(self.states, self.outputs)
+            units = self._units(self.echo, np.full(len(self.entries), ECHO_UNIT, np.int64),
+                                self.outputs * (reached + 8))
+            self._echo_tables = (d_seq, *units)
+        return self._echo_tables
+
     def launch(self, shape: tuple[int, int, int]) -> None:
-        """One persistent launch with (orders per lane, warps per CTA, CTAs per SM)."""
+        """The CPMG trains in one launch, the other sequences in one persistent
+        launch with (orders per lane, warps per CTA, CTAs per SM)."""
         orders, warps, per_sm = shape
-        d_seq, d_units, n_units = self._plan(orders, warps)
+        lib = _native.library()
+        stream = torch.cuda.current_stream().cuda_stream
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         tissue = _native.Tissue(self.t1.data_ptr(), self.t2.data_ptr(),
                                 None if self.m0 is None else self.m0.data_ptr(),
                                 None if self.b1 is None else self.b1.data_ptr(), None)
-        _native.check(_native.library().tsg_epg_batched_forward(
-            self.d_ops.data_ptr(), d_seq.data_ptr(), d_units.data_ptr(), n_units,
-            self.counter.data_ptr(), ctypes.byref(tissue), self.out.data_ptr(), orders, warps,
-            sms * per_sm, torch.cuda.current_stream().cuda_stream))
+        if self.echo.any():
+            d_seq, d_units, n_units = self._echo_plan()
+            _native.check(lib.tsg_epg_echo_forward(
+                self.d_ops.data_ptr(), d_seq.data_ptr(), d_units.data_ptr(), n_units,
+                ctypes.byref(tissue), self.out.data_ptr(), stream))
+        if not self.echo.all():
+            d_seq, d_units, n_units = self._plan(orders, warps)
+            _native.check(lib.tsg_epg_batched_forward(
+                self.d_ops.data_ptr(), d_seq.data_ptr(), d_units.data_ptr(), n_units,
+                self.counter.data_ptr(), ctypes.byref(tissue), self.out.data_ptr(), orders, warps,
+                sms * per_sm, stream))
 
     def candidates(self) -> list[tuple[int, int, int]]:
         cands = []
         for orders in (2, 4, 8, 16):
-            if (-(-self.states // orders) > 32).any():
+            if (-(-self.states[~self.echo] // orders) > 32).any():
                 continue
             for warps in (2, 4, 8):
                 for per_sm in (2, 4, 5, 6, 8, 10, 12, 16):
@@ -172,8 +207,10 @@ class SequenceBatch:
     def tune(self, use_cache: bool = True) -> tuple[tuple[int, int, int], dict]:
         sig = f"n={len(self.entries)},u={self.updates() // 10**6}M,smax={int(self.states.max())}"
         key = autotune.workload_key("batched", workload=sig)
-        best, timings = autotune.tune(key, self.candidates(), self.launch, use_cache=use_cache,
-                                      warmup=1, repeats=2)
+        # The shape is the persistent launch's: without one any will do.
+        candidates = self.candidates()[:1] if self.echo.all() else self.candidates()
+        best, timings = autotune.tune(key, candidates, self.launch, use_cache=use_cache, warmup=1,
+                                      repeats=2)
         self.shape = tuple(best)
         return self.shape, timings
 
