@@ -31,12 +31,16 @@
 //   (per plane pair: transverse with r2, longitudinal with r1 and the
 //   recovery e0 at order 0), and r = 1000/T, r' = -1000 T'/T^2 chain to T.
 //
-// The forward stores every op's entry state of x and of each t_k (the
-// trajectory, one tile per warp: per op, state and plane the warp's 32 lanes'
-// order pairs are 32 * RP consecutive float2, so every store and every load
-// is a whole, aligned line) and every recorded F+[0]; the reverse
-// streams them back through a cp.async ring, so nothing is re-run but each
-// op's relaxation and pre-shift. Per-event partials are summed over the warp
+// The forward stores every EVEN op's entry state of x and of each t_k (the
+// trajectory, one tile per warp: per stored op, state and plane the warp's 32
+// lanes' order pairs are 32 * RP consecutive float2, so every store and every
+// load is a whole, aligned line) and every recorded F+[0]; the reverse
+// streams them back through a cp.async ring and runs the even op forward once
+// for the entry state of the odd op after it. Measured at 16,384 voxels x 601
+// ops x 20 orders, T1, T2 and B1: with every op stored the forward spent its
+// time on 10.2 GB of stores (2.21 ms; 1.59 ms with half of them, and the
+// transcendentals shared by a voxel's lanes), while the reverse, which is
+// bound by instruction issue, pays 0.26 ms for the re-run (2.12 to 2.37 ms). Per-event partials are summed over the warp
 // with a fixed butterfly of shuffles after each op; tissue gradients are
 // summed over a voxel's lanes with shuffles. No atomics: results are
 // deterministic.
@@ -72,7 +76,7 @@ struct SecondArgs {
     float* sig_b;
     float* jac_a;
     float* jac_b;
-    // Trajectory: [train][warp][op][state][plane][lane][RP] float2 (state
+    // Trajectory: [train][warp][op / 2][state][plane][lane][RP] float2 (state
     // 0 = x, k + 1 = t_k; warp = atom / (32 / lanes_per_voxel)), and the
     // recorded F+[0] of each state, [train][output][state][atom].
     float2* traj;
@@ -99,9 +103,14 @@ inline int64_t second_warps(int64_t atoms, int lanes_per_voxel) {
 
 inline int64_t second_trajectory_floats(int64_t trains, int64_t atoms, int64_t ops,
                                         int lanes_per_voxel, int orders_per_lane, int k) {
-    return trains * second_warps(atoms, lanes_per_voxel) * ops * (k + 1) * 3 * 32 *
+    return trains * second_warps(atoms, lanes_per_voxel) * ((ops + 1) / 2) * (k + 1) * 3 * 32 *
            int64_t(orders_per_lane);
 }
+
+// Ops whose transcendentals a voxel's lanes evaluate at once in the reverse:
+// one each, an even number so that a pair of ops is never split (a lone lane
+// takes two).
+__host__ __device__ constexpr int second_group(int lanes) { return lanes < 2 ? 2 : lanes & ~1; }
 
 inline int64_t second_record_floats(int64_t trains, int64_t atoms, int64_t outputs, int k) {
     return trains * outputs * (k + 1) * atoms;
@@ -229,6 +238,57 @@ __device__ __forceinline__ void spoil_all(float2 (&P)[K + 1][RP], float2 (&M)[K 
         for (int kk = 0; kk < RP; ++kk) P[s][kk] = M[s][kk] = dup(0.f);
 }
 
+// The pulse on x and the tangents, (sin, cos) of its angle.
+template <int RP, int K, int HOT>
+__device__ __forceinline__ void rotate_all(float2 (&P)[K + 1][RP], float2 (&M)[K + 1][RP],
+                                           float2 (&Z)[K + 1][RP], float si, float co,
+                                           const float (&dal)[K]) {
+    const float2 ch = dup(0.5f * (1.f + co)), sh = dup(0.5f * (1.f - co));
+    const float2 hs = dup(0.5f * si), nhs = dup(-0.5f * si), hc = dup(0.5f * co);
+    const float2 si2 = dup(si), nsi2 = dup(-si), co2 = dup(co);
+    const float2 neg1 = dup(-1.f);
+#pragma unroll
+    for (int kk = 0; kk < RP; ++kk) {
+        const float2 p = P[0][kk], m = M[0][kk], z = Z[0][kk];
+        const float2 w = fma2(neg1, m, p);
+        // R'x: (-hs w - co z, hs w + co z, hc w - si z).
+        const float2 dM = fma2(hs, w, mul2(co2, z));
+        const float2 dZ = fma2(hc, w, mul2(nsi2, z));
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const float2 tp = P[k + 1][kk], tm = M[k + 1][kk], tz = Z[k + 1][kk];
+            if (!HOT || hot_dir(HOT, k) == 3) {
+                const float2 al = dup(dal[k]);
+                const float2 aM = mul2(al, dM);
+                P[k + 1][kk] = fma2(ch, tp, fma2(sh, tm, fma2(nsi2, tz, mul2(neg1, aM))));
+                M[k + 1][kk] = fma2(sh, tp, fma2(ch, tm, fma2(si2, tz, aM)));
+                Z[k + 1][kk] = fma2(hs, tp, fma2(nhs, tm, fma2(co2, tz, mul2(al, dZ))));
+            } else {
+                P[k + 1][kk] = fma2(ch, tp, fma2(sh, tm, mul2(nsi2, tz)));
+                M[k + 1][kk] = fma2(sh, tp, fma2(ch, tm, mul2(si2, tz)));
+                Z[k + 1][kk] = fma2(hs, tp, fma2(nhs, tm, mul2(co2, tz)));
+            }
+        }
+        P[0][kk] = fma2(ch, p, fma2(sh, m, mul2(nsi2, z)));
+        M[0][kk] = fma2(sh, p, fma2(ch, m, mul2(si2, z)));
+        Z[0][kk] = fma2(hs, w, mul2(co2, z));
+    }
+}
+
+// The inversion of x and the tangents.
+template <int RP, int K, int HOT>
+__device__ __forceinline__ void invert_all(float2 (&Z)[K + 1][RP], const Voxel<K>& v) {
+    const float2 f = dup(-v.eff);
+#pragma unroll
+    for (int kk = 0; kk < RP; ++kk) {
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            Z[k + 1][kk] = HOT ? mul2(f, Z[k + 1][kk])
+                               : fma2(f, Z[k + 1][kk], mul2(dup(-v.deff[k]), Z[0][kk]));
+        Z[0][kk] = mul2(Z[0][kk], f);
+    }
+}
+
 // One op's per-direction scalars: eps1_k, eps2_k (relaxation) and a'_k
 // (rotation); ddt_k and dflip_k from the op's directions.
 template <int K, int HOT>
@@ -298,7 +358,8 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
     const int64_t warp_global = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
     const int64_t op_stride = int64_t(NS) * 3 * 32 * RP;
     float2* lane_traj = (a.traj && warp_global < n_warps)
-                            ? a.traj + (train * n_warps + warp_global) * a.n_ops * op_stride +
+                            ? a.traj + (train * n_warps + warp_global) * ((a.n_ops + 1) >> 1) *
+                                           op_stride +
                                   lane * RP
                             : nullptr;
     const bool lane0 = active && q == 0;
@@ -342,6 +403,7 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
         }
     }
 
+    float4 my = make_float4(0.f, 1.f, 1.f, 1.f);  // (sin, cos, E1, E2) of this lane's op
     for (int base = 0; base < a.n_ops; base += kOpChunk) {
         const int count = min(kOpChunk, a.n_ops - base);
         __syncthreads();
@@ -355,8 +417,21 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
         for (int i = 0; i < count; ++i) {
             const Op op = s_ops[i];
             const uint32_t code = op.code;
-            if (lane_traj) {
-                float2* dst = lane_traj + int64_t(base + i) * op_stride;
+            // Lane q of a voxel evaluates the transcendentals of one of the
+            // next L ops; the lanes exchange them by shuffle.
+            const int g = i % L;
+            if (g == 0 && i + q < count) {
+                const Op next = s_ops[i + q];
+                my = make_float4(0.f, 1.f, expf(-v.r1 * next.dt), expf(-v.r2 * next.dt));
+                if (op_rf(next.code) == RF_ROTATE) sincosf(next.flip * v.b1, &my.x, &my.y);
+            }
+            float4 tr;
+            tr.x = __shfl_sync(0xffffffffu, my.x, lane - q + g);
+            tr.y = __shfl_sync(0xffffffffu, my.y, lane - q + g);
+            tr.z = __shfl_sync(0xffffffffu, my.z, lane - q + g);
+            tr.w = __shfl_sync(0xffffffffu, my.w, lane - q + g);
+            if (lane_traj && !((base + i) & 1)) {
+                float2* dst = lane_traj + int64_t((base + i) >> 1) * op_stride;
 #pragma unroll
                 for (int s = 0; s < NS; ++s)
 #pragma unroll
@@ -370,53 +445,13 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
             op_directions<K, HOT>(a, HOT ? nullptr : &s_dir[0][0], kOpChunk, i, op, v, ddt, eps1,
                                   eps2, dal, dfl);
             if (code & OP_RELAX)
-                relax_all<RP, K, HOT>(P, M, Z, expf(-v.r1 * op.dt), expf(-v.r2 * op.dt), eps1,
-                                      eps2, q);
+                relax_all<RP, K, HOT>(P, M, Z, tr.z, tr.w, eps1, eps2, q);
             for (int s = 0; s < op_shift1(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
             const int rf = op_rf(code);
             if (rf == RF_ROTATE) {
-                float si, co;
-                sincosf(op.flip * v.b1, &si, &co);
-                const float2 ch = dup(0.5f * (1.f + co)), sh = dup(0.5f * (1.f - co));
-                const float2 hs = dup(0.5f * si), nhs = dup(-0.5f * si), hc = dup(0.5f * co);
-                const float2 si2 = dup(si), nsi2 = dup(-si), co2 = dup(co);
-                const float2 neg1 = dup(-1.f);
-#pragma unroll
-                for (int kk = 0; kk < RP; ++kk) {
-                    const float2 p = P[0][kk], m = M[0][kk], z = Z[0][kk];
-                    const float2 w = fma2(neg1, m, p);
-                    // R'x: (-hs w - co z, hs w + co z, hc w - si z).
-                    const float2 dM = fma2(hs, w, mul2(co2, z));
-                    const float2 dZ = fma2(hc, w, mul2(nsi2, z));
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const float2 tp = P[k + 1][kk], tm = M[k + 1][kk], tz = Z[k + 1][kk];
-                        if (!HOT || hot_dir(HOT, k) == 3) {
-                            const float2 al = dup(dal[k]);
-                            const float2 aM = mul2(al, dM);
-                            P[k + 1][kk] = fma2(ch, tp, fma2(sh, tm, fma2(nsi2, tz, mul2(neg1, aM))));
-                            M[k + 1][kk] = fma2(sh, tp, fma2(ch, tm, fma2(si2, tz, aM)));
-                            Z[k + 1][kk] = fma2(hs, tp, fma2(nhs, tm, fma2(co2, tz, mul2(al, dZ))));
-                        } else {
-                            P[k + 1][kk] = fma2(ch, tp, fma2(sh, tm, mul2(nsi2, tz)));
-                            M[k + 1][kk] = fma2(sh, tp, fma2(ch, tm, mul2(si2, tz)));
-                            Z[k + 1][kk] = fma2(hs, tp, fma2(nhs, tm, mul2(co2, tz)));
-                        }
-                    }
-                    P[0][kk] = fma2(ch, p, fma2(sh, m, mul2(nsi2, z)));
-                    M[0][kk] = fma2(sh, p, fma2(ch, m, mul2(si2, z)));
-                    Z[0][kk] = fma2(hs, w, mul2(co2, z));
-                }
+                rotate_all<RP, K, HOT>(P, M, Z, tr.x, tr.y, dal);
             } else if (rf == RF_INVERT) {
-                const float2 f = dup(-v.eff);
-#pragma unroll
-                for (int kk = 0; kk < RP; ++kk) {
-#pragma unroll
-                    for (int k = 0; k < K; ++k)
-                        Z[k + 1][kk] = HOT ? mul2(f, Z[k + 1][kk])
-                                           : fma2(f, Z[k + 1][kk], mul2(dup(-v.deff[k]), Z[0][kk]));
-                    Z[0][kk] = mul2(Z[0][kk], f);
-                }
+                invert_all<RP, K, HOT>(Z, v);
             }
             for (int s = 0; s < op_shift2(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
             if (code & OP_SPOIL1) spoil_all<RP, K>(P, M);
@@ -473,10 +508,11 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
 
 // ---- reverse ---------------------------------------------------------------
 
-// Dynamic shared memory: transcendentals [D][T] float4, entry states
-// [D][NS][3][RP][T] float2, (seed, recorded F+[0]) [D][NS][T] float2, the
-// M0 derivative's seed [D][T] float, ops [n_ops], per-direction op
-// directions [K][n_ops] float2 (only with event directions).
+// Dynamic shared memory, a ring slot per pair of ops: entry states of the even
+// op [D][NS][3][RP][T] float2, transcendentals [G][VPB] float4, of both ops
+// (seed, recorded F+[0]) [D][2][NS][VPB] float2 and the M0 derivative's seed
+// [D][2][VPB4] float, ops [n_ops], per-direction op directions [K][n_ops]
+// float2 (only with event directions).
 template <int RP, int L, int K, int HOT>
 __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const SecondArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -510,10 +546,11 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     constexpr int VPB = W * VPW;
     constexpr int VPB4 = (VPB + 3) & ~3;
     float2* s_ring = reinterpret_cast<float2*>(s_raw);                    // [D][NS*3][T][RP]
-    float4* s_tring = reinterpret_cast<float4*>(s_ring + D * NS * 3 * RP * T);  // [L][VPB]
-    float2* s_sring = reinterpret_cast<float2*>(s_tring + L * VPB);       // [D][NS][VPB]
-    float* s_mring = reinterpret_cast<float*>(s_sring + D * NS * VPB);    // [D][VPB4]
-    Op* s_ops = reinterpret_cast<Op*>(s_mring + D * VPB4);                 // [n_ops]
+    constexpr int G = second_group(L);
+    float4* s_tring = reinterpret_cast<float4*>(s_ring + D * NS * 3 * RP * T);  // [G][VPB]
+    float2* s_sring = reinterpret_cast<float2*>(s_tring + G * VPB);       // [D][2][NS][VPB]
+    float* s_mring = reinterpret_cast<float*>(s_sring + D * 2 * NS * VPB);  // [D][2][VPB4]
+    Op* s_ops = reinterpret_cast<Op*>(s_mring + D * 2 * VPB4);             // [n_ops]
     float2* s_dir = reinterpret_cast<float2*>(s_ops + n_ops);              // [K][n_ops]
 
     const Voxel<K> v = load_voxel<K, HOT>(a, ac);
@@ -558,18 +595,19 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     const int64_t n_warps = (n + VPW - 1) / VPW;
     const int64_t op_stride = int64_t(NS) * 3 * 32 * RP;
     const float2* lane_traj =
-        a.traj + (train * n_warps + (warp_global < n_warps ? warp_global : 0)) * n_ops * op_stride +
+        a.traj + (train * n_warps + (warp_global < n_warps ? warp_global : 0)) *
+                     ((n_ops + 1) >> 1) * op_stride +
         lane * RP;
     const unsigned ring_base =
         static_cast<unsigned>(__cvta_generic_to_shared(s_ring + threadIdx.x * RP));
     const unsigned sring_base = static_cast<unsigned>(__cvta_generic_to_shared(s_sring + vslot));
     const unsigned mring_base = static_cast<unsigned>(__cvta_generic_to_shared(s_mring + vslot));
 
-    // Op o into ring slot rs: entry-state pairs of every state (zero past the
-    // last pair), the seeds and recorded F+[0] (zero unless this lane
-    // records), and the transcendentals.
-    auto fetch = [&](int o, int rs) {
-        const float2* src_op = lane_traj + o * op_stride;
+    // Pair i (ops 2 i, 2 i + 1) into ring slot rs: the even op's entry states,
+    // and of both ops the seeds and recorded F+[0] (zero unless this lane
+    // records).
+    auto fetch = [&](int i, int rs) {
+        const float2* src_op = lane_traj + i * op_stride;
         const unsigned dst_op = ring_base + unsigned(rs * NS * 3 * RP * T) * 8u;
 #pragma unroll
         for (int sp = 0; sp < NS * 3; ++sp) {
@@ -586,41 +624,47 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                                  : "memory");
             }
         }
-        const Op op = s_ops[o];
         // Seeds and recorded F+[0]: lane 0 of each voxel slot copies them
         // (zeros unless the voxel is live and the op records).
         if (q == 0 && slot < VPW) {
-            const bool rec = lane0 && (op.code & OP_RECORD);
-            const int64_t r = rec ? op.record : 0;
-            const unsigned sdst = sring_base + unsigned(rs * NS * VPB) * 8u;
-            const bool have0 = rec && seed0_row != nullptr;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sdst),
-                         "l"(have0 ? seed0_row + r * seed_stride : a.seed), "r"(have0 ? 4 : 0)
-                         : "memory");
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                                 sdst + unsigned((k + 1) * VPB) * 8u),
-                             "l"(seed_row + (k * a.outputs + r) * seed_stride), "r"(rec ? 4 : 0)
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {
+                const int o = 2 * i + h;
+                if (o >= n_ops) break;
+                const Op op = s_ops[o];
+                const bool rec = lane0 && (op.code & OP_RECORD);
+                const int64_t r = rec ? op.record : 0;
+                const unsigned sdst = sring_base + unsigned((rs * 2 + h) * NS * VPB) * 8u;
+                const bool have0 = rec && seed0_row != nullptr;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sdst),
+                             "l"(have0 ? seed0_row + r * seed_stride : a.seed), "r"(have0 ? 4 : 0)
                              : "memory");
-#pragma unroll
-            for (int s = 0; s < NS; ++s)
+    #pragma unroll
+                for (int k = 0; k < K; ++k)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                                     sdst + unsigned((k + 1) * VPB) * 8u),
+                                 "l"(seed_row + (k * a.outputs + r) * seed_stride), "r"(rec ? 4 : 0)
+                                 : "memory");
+    #pragma unroll
+                for (int s = 0; s < NS; ++s)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
+                                     sdst + unsigned(s * VPB) * 8u + 4u),
+                                 "l"(rec_col + (r * NS + s) * n), "r"(rec ? 4 : 0)
+                                 : "memory");
+                const bool have_m = rec && a.with_m0;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                                 sdst + unsigned(s * VPB) * 8u + 4u),
-                             "l"(rec_col + (r * NS + s) * n), "r"(rec ? 4 : 0)
+                                 mring_base + unsigned((rs * 2 + h) * VPB4) * 4u),
+                             "l"(have_m ? seed_row + (K * a.outputs + r) * seed_stride : a.seed),
+                             "r"(have_m ? 4 : 0)
                              : "memory");
-            const bool have_m = rec && a.with_m0;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                             mring_base + unsigned(rs * VPB4) * 4u),
-                         "l"(have_m ? seed_row + (K * a.outputs + r) * seed_stride : a.seed),
-                         "r"(have_m ? 4 : 0)
-                         : "memory");
+            }
         }
     };
 
+    const int n_pairs = (n_ops + 1) >> 1;
 #pragma unroll
     for (int j = 1; j < D; ++j) {
-        if (n_ops - j >= 0) fetch(n_ops - j, j - 1);
+        if (n_pairs - j >= 0) fetch(n_pairs - j, j - 1);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     }
     float2* event_out =
@@ -630,36 +674,46 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     const float2 neg1 = dup(-1.f);
 
     for (int o = n_ops - 1; o >= 0; --o) {
-        if ((n_ops - 1 - o) % L == 0) {
-            // Every L ops, the transcendentals of the next L: lane q of a
-            // voxel evaluates op o - q, so one pass of the warp covers them
-            // (slot (op % L) of each voxel; the slots' last readers are done).
-            __syncwarp();
-            const int oq = o - q;
-            if (slot < VPW && oq >= 0) {
-                const Op opq = s_ops[oq];
-                float si = 0.f, co = 1.f;
-                if (op_rf(opq.code) == RF_ROTATE) sincosf(opq.flip * v.b1, &si, &co);
-                s_tring[(oq % L) * VPB + vslot] =
-                    make_float4(si, co, expf(-v.r1 * opq.dt), expf(-v.r2 * opq.dt));
+        const bool odd = o & 1;
+        const bool new_pair = odd || o == n_ops - 1;
+        if (new_pair) {
+            if (o % G == G - 1 || o == n_ops - 1) {
+                // The transcendentals of the group of G ops that ends here:
+                // lane q of a voxel evaluates the group's op q (a lone lane
+                // both), so one pass of the warp covers them. (Their last
+                // readers are done.)
+                __syncwarp();
+#pragma unroll
+                for (int e = 0; e < (L < 2 ? 2 : 1); ++e) {
+                    const int oq = o - o % G + q + e;
+                    if (slot < VPW && q < G && oq <= o) {
+                        const Op opq = s_ops[oq];
+                        float si = 0.f, co = 1.f;
+                        if (op_rf(opq.code) == RF_ROTATE) sincosf(opq.flip * v.b1, &si, &co);
+                        s_tring[(oq % G) * VPB + vslot] =
+                            make_float4(si, co, expf(-v.r1 * opq.dt), expf(-v.r2 * opq.dt));
+                    }
+                }
             }
+            // Orders the lanes' reads of the slot this fetch refills (used by
+            // the last pair) and the transcendentals written above.
+            __syncwarp();
+            if ((o >> 1) - (D - 1) >= 0) fetch((o >> 1) - (D - 1), fill_slot);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
+            __syncwarp();  // the seeds another lane copied
         }
-        // Orders the lanes' reads of the slot this fetch refills (used last
-        // iteration) and the transcendentals written above.
-        __syncwarp();
-        if (o - (D - 1) >= 0) fetch(o - (D - 1), fill_slot);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
         const Op op = s_ops[o];
         const uint32_t code = op.code;
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
         const int cur = use_slot;
-        use_slot = use_slot + 1 == D ? 0 : use_slot + 1;
-        const float4 tr = s_tring[(o % L) * VPB + vslot];
+        if (!odd) use_slot = use_slot + 1 == D ? 0 : use_slot + 1;
+        const float4 tr = s_tring[(o % G) * VPB + vslot];
         const float2* ring = s_ring + cur * (NS * 3 * RP * T) + threadIdx.x * RP;
-        const float2* sr = s_sring + cur * (NS * VPB) + vslot;
+        const float2* sr = s_sring + (cur * 2 + (o & 1)) * (NS * VPB) + vslot;
 
-        // The pre-RF states: entry states relaxed and pre-shifted.
+        // The pre-RF states: entry states (an odd op's by running the even op
+        // before it), relaxed and pre-shifted.
         float2 P[NS][RP], M[NS][RP], Z[NS][RP];
 #pragma unroll
         for (int s = 0; s < NS; ++s)
@@ -670,6 +724,21 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                 Z[s][kk] = ring[(s * 3 + 2) * T * RP + kk];
             }
         float ddt[K], eps1[K], eps2[K], dal[K], dfl[K];
+        if (odd) {
+            const Op even = s_ops[o - 1];
+            const float4 te = s_tring[((o - 1) % G) * VPB + vslot];
+            op_directions<K, HOT>(a, dirs, n_ops, o - 1, even, v, ddt, eps1, eps2, dal, dfl);
+            if (even.code & OP_RELAX) relax_all<RP, K, HOT>(P, M, Z, te.z, te.w, eps1, eps2, q);
+            for (int s = 0; s < op_shift1(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (op_rf(even.code) == RF_ROTATE)
+                rotate_all<RP, K, HOT>(P, M, Z, te.x, te.y, dal);
+            else if (op_rf(even.code) == RF_INVERT)
+                invert_all<RP, K, HOT>(Z, v);
+            for (int s = 0; s < op_shift2(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (even.code & OP_SPOIL1) spoil_all<RP, K>(P, M);
+            for (int s = 0; s < op_shift3(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (even.code & OP_SPOIL2) spoil_all<RP, K>(P, M);
+        }
         op_directions<K, HOT>(a, dirs, n_ops, o, op, v, ddt, eps1, eps2, dal, dfl);
         const bool relax = (code & OP_RELAX) != 0;
         if (relax) relax_all<RP, K, HOT>(P, M, Z, tr.z, tr.w, eps1, eps2, q);
@@ -682,7 +751,7 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
             const float g0 = seed_sign * sr[0].x;
             const float x0 = sr[0].y;
             // The M0 derivative is F+[0] itself: its seed acts unscaled.
-            const float g_m0col = s_mring[cur * VPB4 + vslot];
+            const float g_m0col = s_mring[(cur * 2 + (o & 1)) * VPB4 + vslot];
             float add0 = fmaf(g0, v.m0, seed_sign * g_m0col);
             c_m0 = fmaf(g0, x0, c_m0);
 #pragma unroll
