@@ -356,6 +356,13 @@ int launch_complex_sweep(const tsg_program* program, const ComplexArgs& base, in
     if (warps < 1 || warps > 8) return fail(TSG_ERR_ARGUMENT, "warps_per_block must be 1..8");
     const ComplexEntry* best = choose_complex(tangents, state_count, launch_shape);
     if (!best) return fail(TSG_ERR_UNSUPPORTED, "no complex kernel for this state count / launch shape");
+    // A CPMG train has its own kernel, unless a shape of this one is asked for.
+    if (!launch_shape || (launch_shape->lanes_per_voxel <= 0 && launch_shape->orders_per_lane <= 0 &&
+                          launch_shape->warps_per_block <= 0)) {
+        bool taken = false;
+        const int rc = launch_cpmg(program, base, tangents, stream, &taken);
+        if (rc || taken) return rc;
+    }
     const int vpb = warps * (32 / best->lanes_per_voxel);
     const int64_t blocks = (atom_count + vpb - 1) / vpb;
     if (blocks > 0x7fffffffLL) return fail(TSG_ERR_CAPACITY, "launch too large");

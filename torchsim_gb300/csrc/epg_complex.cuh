@@ -194,4 +194,9 @@ __device__ __forceinline__ OpTrig op_trig(const Op& op, float2 ph, float r1, flo
 
 }  // namespace complex_detail
 
+// epg_cpmg.cu: the sweep of a train that find_cpmg accepts, where the maps
+// leave it in its two subspaces and a shape holds its orders (`taken`).
+int launch_cpmg(const tsg_program* program, const complex_detail::ComplexArgs& args, int tangents,
+                cudaStream_t stream, bool* taken);
+
 }  // namespace tsg

@@ -203,6 +203,7 @@ int compile_program(const float* duration, const int32_t* kind, const float* fli
             std::copy(per_phase[t].begin(), per_phase[t].end(), out->phase.begin() + t * longest);
     }
     out->train_first = find_train(*out);
+    out->cpmg = find_cpmg(*out);
     return TSG_OK;
 }
 

@@ -73,6 +73,9 @@ struct HostProgram {
     // A plain recorded train (find_train): the first op of the train, 0 or 1
     // (after a leading inversion); -1 for any other program.
     int train_first = -1;
+    // A CPMG train of one refocusing phase, 90 degrees from the excitation's
+    // (find_cpmg).
+    bool cpmg = false;
     std::vector<Op> op;              // [train][ops]
     std::vector<OpSource> src;       // [train][ops]
     // With event phases (the complex path): per op the phase of its pulse
@@ -118,6 +121,7 @@ int compile_program(const float* duration, const int32_t* kind, const float* fli
 
 // Where the plain recorded train of a compiled program begins (0 or 1), or -1.
 int find_train(const HostProgram& program);
+bool find_cpmg(const HostProgram& program);
 
 // Arguments of one sweep launch (forward, fused tangents, general tangent).
 struct SweepArgs {
