@@ -494,6 +494,19 @@ int tsg_epg_batched_forward(const void* ops, const tsg_batch_sequence* sequences
                             const tsg_tissue* tissue, void* out, int orders_per_lane,
                             int warps_per_block, int blocks, void* stream);
 
+/* A fast spin echo's steady state (simulators/fse.py:110-133) over `rows`
+ * recorded trains of `echoes` complex64 samples (1j * s, as the sweeps return
+ * them) and their `columns_in` Jacobian columns: one kernel. Output column c is
+ * input column sources[c] (-1: the M0 column) by the chain rule; `t1_column` is
+ * the output column that takes the recovery's own T1 term, or -1. T1 (ms) and
+ * M0 hold one value or one per row (M0 null: m0_value); left_ms = TR - ESP *
+ * echoes. The outputs are s, not 1j * s. At most 16 columns. */
+int tsg_fse_recovery(const void* signal, const void* jacobian, int64_t rows, int64_t echoes,
+                     int32_t columns_in, int32_t columns, const int32_t* sources,
+                     int32_t t1_column, const float* t1_ms, int64_t t1_count, const float* m0,
+                     int64_t m0_count, float m0_value, float left_ms, void* out,
+                     void* jacobian_out, void* stream);
+
 /* Whether a compiled single-train program (HOST array of 16-byte ops) is a CPMG
  * train the echo kernel runs: the excitation, then per echo one refocusing op
  * and one recording op, one interval throughout, at most 64 echoes. */

@@ -121,6 +121,8 @@ SIGNATURES: dict[str, tuple] = {
     "tsg_program_rebind": (_int, [_vp, _vp, _vp, _vp, _vp]),
     "tsg_program_view": (_int, [_vp, _vp, ctypes.POINTER(_vp)]),
     "tsg_echo_train": (_int, [_vp, _i64]),
+    "tsg_fse_recovery": (_int, [_vp, _vp, _i64, _i64, _int, _int, _vp, _int, _vp, _i64, _vp, _i64,
+                                ctypes.c_float, ctypes.c_float, _vp, _vp, _vp]),
     "tsg_epg_echo_forward": (_int, [_vp, _vp, _vp, _i64, ctypes.POINTER(Tissue), _vp, _vp]),
     "tsg_mrf_stream": (_int, [_vp, _vp, _vp, _i64, ctypes.c_float, _i64, ctypes.c_float,
                               ctypes.c_float, _vp, _vp, _vp, _vp]),

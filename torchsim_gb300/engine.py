@@ -152,6 +152,26 @@ def forward_complex(program: Program, tissue: TissueMaps, states: int, offaxis=N
     return out
 
 
+def fse_recovery(signal: torch.Tensor, jacobian: torch.Tensor | None, sources: Sequence[int],
+                 t1_column: int, t1: torch.Tensor, m0: torch.Tensor | float, left_ms: float):
+    """A fast spin echo's steady state over recorded trains ``(rows, P)`` and
+    their columns ``(rows, k, P)`` in one kernel (``tsg_fse_recovery``):
+    output column ``c`` is input column ``sources[c]``, or M0's for -1."""
+    rows, echoes = signal.shape
+    out = torch.empty_like(signal)
+    jac = None if jacobian is None else torch.empty((rows, len(sources), echoes),
+                                                    dtype=signal.dtype, device=signal.device)
+    tensor = isinstance(m0, torch.Tensor)
+    _native.check(_native.library().tsg_fse_recovery(
+        signal.data_ptr(), None if jacobian is None else jacobian.data_ptr(), rows, echoes,
+        0 if jacobian is None else jacobian.shape[1], len(sources),
+        (ctypes.c_int32 * len(sources))(*sources), t1_column, t1.data_ptr(), t1.numel(),
+        m0.data_ptr() if tensor else None, m0.numel() if tensor else 0,
+        1.0 if tensor else m0, left_ms, out.data_ptr(), None if jac is None else jac.data_ptr(),
+        _stream()))
+    return out, jac
+
+
 # Columns of the complex path carried by the general tangent kernel (one
 # launch each), beside the fused T1/T2/B1/M0 sweep: the property's slot in
 # the direction structs.

@@ -188,6 +188,10 @@ class _EpgSimulator:
     def _post(self, signal, jacobian, names, held, protocol, device):
         return signal, jacobian
 
+    def _post_untracked(self, signal, jacobian, names, held, protocol, device):
+        """:meth:`_post` of a call that nothing is differentiated through."""
+        return self._post(signal, jacobian, names, held, protocol, device)
+
     # -- machinery ---------------------------------------------------------
     def _split(self, values: dict[str, Any]):
         merged = {**self.protocol, **values}
@@ -249,7 +253,7 @@ class _EpgSimulator:
                 else:
                     signal, jac = engine.forward_complex(program, tissue, states, off), None
                 del keep
-                signal, jac = self._post(signal, jac, names, held, protocol, dev)
+                signal, jac = self._post_untracked(signal, jac, names, held, protocol, dev)
                 signal = signal.reshape(*batch, signal.shape[-1]) if batch else signal.reshape(-1)
                 if jac is not None:
                     jac = (jac.reshape(*batch, *jac.shape[-2:]) if batch
@@ -273,7 +277,7 @@ class _EpgSimulator:
                 signal, jac = engine.forward_tangents(program, tissue, states, kernel_names)
             else:
                 signal, jac = engine.forward(program, tissue, states), None
-            signal, jac = self._post(signal, jac, names, held, protocol, dev)
+            signal, jac = self._post_untracked(signal, jac, names, held, protocol, dev)
         signal = signal.reshape(*batch, signal.shape[-1]) if batch else signal.reshape(-1)
         if jac is not None:
             jac = jac.reshape(*batch, *jac.shape[-2:]) if batch else jac.reshape(jac.shape[-2:])
@@ -600,6 +604,31 @@ class FSESimulator(_EpgSimulator):
                 col = col + dfdrec * drec_dt1
             cols.append(col)
         return out, torch.stack(cols, dim=-2)
+
+    def _post_untracked(self, signal, jacobian, names, held, protocol, device):
+        # One kernel for the plain forms (csrc/fse_recovery.cu), against some
+        # forty launches of _post: one TR, a value of T1 and M0 for each
+        # voxel or for all.
+        tr, names = protocol.get("TR", 1e6), names or ()
+        t1 = torch.as_tensor(held["T1"], dtype=torch.float32, device=device).reshape(-1)
+        m0 = held.get("M0", 1.0)
+        if isinstance(m0, torch.Tensor):
+            m0 = m0.to(device=device, dtype=torch.float32).reshape(-1)
+        rows = signal.shape[0]
+        if (type(self)._post is not FSESimulator._post or not isinstance(tr, (int, float))
+                or t1.numel() not in (1, rows) or len(names) > 16 or len(set(names)) < len(names)
+                or not (isinstance(m0, (int, float))
+                        or isinstance(m0, torch.Tensor) and m0.numel() in (1, rows))
+                or not signal.is_contiguous()
+                or jacobian is not None and not jacobian.is_contiguous()):
+            return self._post(signal, jacobian, names, held, protocol, device)
+        kernel = self._kernel_names(names) if names else []
+        left_ms = float(np.float32(tr) - np.float32(float(protocol["ESP"]) * signal.shape[-1]))
+        t1_column = names.index("T1") if "T1" in names else -1
+        return engine.fse_recovery(signal, jacobian,
+                                   [-1 if n == "M0" else kernel.index(n) for n in names], t1_column,
+                                   t1.contiguous(), m0.contiguous() if isinstance(m0, torch.Tensor)
+                                   else float(m0), left_ms)
 
 
 def mrf_sim(flip, TR, T1, T2, diff: str | tuple[str, ...] | None = None, B1=1.0,
