@@ -511,7 +511,7 @@ int tsg_fse_recovery(const void* signal, const void* jacobian, int64_t rows, int
  * train the echo kernel runs: the excitation, then per echo one refocusing op
  * and one recording op, one interval throughout, at most 64 echoes. */
 int tsg_echo_train(const void* host_ops, int64_t op_count);
-/* The CPMG trains of a batch, one voxel per lane: buffers as
+/* The CPMG trains of a batch, two voxels per lane: buffers as
  * tsg_epg_batched_forward takes them, units of up to 64 voxels of sequences
  * for which tsg_echo_train holds (lanes_per_voxel is not read). */
 int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* sequences,

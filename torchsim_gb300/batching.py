@@ -7,7 +7,7 @@ to its own problem, with a tail of idle SMs after every small one.
 :class:`SequenceBatch` packs all of them into one table: the sequences'
 compiled programs back to back, their tissue back to back, and a list of
 (sequence, voxel tile) units sorted largest first. CPMG trains (the excitation,
-then per echo one refocusing pulse and one sample) run one voxel per lane with
+then per echo one refocusing pulse and one sample) run two voxels per lane with
 only the orders that matter at each echo (``tsg_epg_echo_forward``); a single
 launch of the persistent kernel (``tsg_epg_batched_forward``) works through the
 other sequences' units. The launches and the counter reset are captured once in
@@ -54,7 +54,7 @@ def compile_ops(events: PackedEvents) -> np.ndarray:
     return ops
 
 
-# Voxels per unit of the echo kernel: two warps, one voxel per lane.
+# Voxels per unit of the echo kernel: one warp, two voxels per lane.
 ECHO_UNIT = 64
 
 
@@ -111,7 +111,7 @@ class SequenceBatch:
         total = int((self.voxels * self.outputs).sum())
         self.out = torch.empty(total, dtype=torch.complex64, device=device)
         self.counter = torch.zeros(1, dtype=torch.int32, device=device)
-        # CPMG trains run one voxel per lane (tsg_epg_echo_forward), the other
+        # CPMG trains run two voxels per lane (tsg_epg_echo_forward), the other
         # sequences the persistent kernel.
         lib = _native.library()
         self.echo = np.array([bool(lib.tsg_echo_train(p.ctypes.data, len(p))) for p in programs], bool)
