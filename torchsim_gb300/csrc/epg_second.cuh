@@ -46,10 +46,13 @@
 // deterministic.
 #pragma once
 #include "epg_adjoint.cuh"
+#include <type_traits>
 
 namespace tsg {
 
 constexpr int kSecondMaxK = 3;
+// An op of a fingerprinting train: relaxation, pulse, sample, shift.
+constexpr uint32_t kPlainOp = kFastBits | OP_RECORD;
 constexpr int kSecondRing = 2;
 constexpr int kSecondWarps = 2;
 
@@ -174,6 +177,8 @@ __device__ __forceinline__ Voxel<K> load_voxel(const SecondArgs& a, int64_t ac) 
     }
     return v;
 }
+
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
 // Relaxation of x and the tangents over one op: t_k <- E (t_k + eps_k (x -
 // e0)), x <- E x + (1 - E1) e0, e0 the recovery target (Z at order 0, held
@@ -403,9 +408,89 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
         }
     }
 
+    // One op; of a plain one (kPlainOp, most ops of a fingerprinting train) the
+    // steps are known when this is compiled.
+    int op_base = 0;
+    auto step = [&](auto plain, int i, const Op& op, const float4& tr) {
+        const uint32_t code = decltype(plain)::value ? kPlainOp : op.code;
+        if (lane_traj && !((op_base + i) & 1)) {
+            float2* dst = lane_traj + int64_t((op_base + i) >> 1) * op_stride;
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+#pragma unroll
+                for (int kk = 0; kk < RP; ++kk) {
+                    dst[(s * 3 + 0) * 32 * RP + kk] = P[s][kk];
+                    dst[(s * 3 + 1) * 32 * RP + kk] = M[s][kk];
+                    dst[(s * 3 + 2) * 32 * RP + kk] = Z[s][kk];
+                }
+        }
+        float ddt[K], eps1[K], eps2[K], dal[K], dfl[K];
+        op_directions<K, HOT>(a, HOT ? nullptr : &s_dir[0][0], kOpChunk, i, op, v, ddt, eps1,
+                              eps2, dal, dfl);
+        if (code & OP_RELAX)
+            relax_all<RP, K, HOT>(P, M, Z, tr.z, tr.w, eps1, eps2, q);
+        for (int s = 0; s < op_shift1(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+        const int rf = op_rf(code);
+        if (rf == RF_ROTATE) {
+            rotate_all<RP, K, HOT>(P, M, Z, tr.x, tr.y, dal);
+        } else if (rf == RF_INVERT) {
+            invert_all<RP, K, HOT>(Z, v);
+        }
+        for (int s = 0; s < op_shift2(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+        if (code & OP_SPOIL1) spoil_all<RP, K>(P, M);
+        if (DIST && (code & OP_RECORD)) {
+            const int64_t rec = op.record;
+            const int first = lane - q;
+            const float p0 = __shfl_sync(0xffffffffu, P[0][0].x, first);
+            float val = v.m0 * p0;  // q = 0: the signal
+            float raw = p0;         // q = K + 2: state 0's recorded F+[0]
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const float d = __shfl_sync(0xffffffffu, P[k + 1][0].x, first);
+                if (q == k + 1) val = HOT ? v.m0 * d : fmaf(v.m0, d, v.dm0[k] * p0);
+                if (q == K + 3 + k) raw = d;
+            }
+            if (q == K + 1) val = p0;  // the M0 column
+            if (a.layout == TSG_LAYOUT_PLANES) {
+                if (row_b != nullptr) {
+                    if (row_a != nullptr) row_a[rec] = 0.f;
+                    row_b[rec] = val;
+                }
+            } else if (row_a != nullptr) {
+                reinterpret_cast<float2*>(row_a)[rec] = a.layout == TSG_LAYOUT_COMPLEX
+                                                            ? make_float2(0.f, val)
+                                                            : make_float2(-val, 0.f);
+            }
+            if (rec_row != nullptr) rec_row[rec * NS * a.atoms] = raw;
+        } else if ((code & OP_RECORD) && lane0) {
+            const int64_t rec = op.record;
+            const float p0 = P[0][0].x;
+            if (a.sig_a != nullptr || a.sig_b != nullptr)
+                store_sample(a.layout, a.sig_a, a.sig_b, row * a.outputs + rec, v.m0 * p0);
+            if (a.jac_a != nullptr || a.jac_b != nullptr) {
+                const int jc = K + a.with_m0;
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + k) * a.outputs + rec,
+                                 HOT ? v.m0 * P[k + 1][0].x
+                                     : fmaf(v.m0, P[k + 1][0].x, v.dm0[k] * p0));
+                if (a.with_m0)
+                    store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + K) * a.outputs + rec, p0);
+            }
+            if (a.traj_rec) {
+                float* dst = a.traj_rec + ((train * a.outputs + rec) * NS) * a.atoms + atom;
+#pragma unroll
+                for (int s = 0; s < NS; ++s) dst[s * a.atoms] = P[s][0].x;
+            }
+        }
+        for (int s = 0; s < op_shift3(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+        if (code & OP_SPOIL2) spoil_all<RP, K>(P, M);
+    };
+
     float4 my = make_float4(0.f, 1.f, 1.f, 1.f);  // (sin, cos, E1, E2) of this lane's op
     for (int base = 0; base < a.n_ops; base += kOpChunk) {
         const int count = min(kOpChunk, a.n_ops - base);
+        op_base = base;
         __syncthreads();
         for (int i = threadIdx.x; i < count; i += blockDim.x) {
             s_ops[i] = ops[base + i];
@@ -416,7 +501,6 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
         __syncthreads();
         for (int i = 0; i < count; ++i) {
             const Op op = s_ops[i];
-            const uint32_t code = op.code;
             // Lane q of a voxel evaluates the transcendentals of one of the
             // next L ops; the lanes exchange them by shuffle.
             const int g = i % L;
@@ -430,78 +514,10 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
             tr.y = __shfl_sync(0xffffffffu, my.y, lane - q + g);
             tr.z = __shfl_sync(0xffffffffu, my.z, lane - q + g);
             tr.w = __shfl_sync(0xffffffffu, my.w, lane - q + g);
-            if (lane_traj && !((base + i) & 1)) {
-                float2* dst = lane_traj + int64_t((base + i) >> 1) * op_stride;
-#pragma unroll
-                for (int s = 0; s < NS; ++s)
-#pragma unroll
-                    for (int kk = 0; kk < RP; ++kk) {
-                        dst[(s * 3 + 0) * 32 * RP + kk] = P[s][kk];
-                        dst[(s * 3 + 1) * 32 * RP + kk] = M[s][kk];
-                        dst[(s * 3 + 2) * 32 * RP + kk] = Z[s][kk];
-                    }
-            }
-            float ddt[K], eps1[K], eps2[K], dal[K], dfl[K];
-            op_directions<K, HOT>(a, HOT ? nullptr : &s_dir[0][0], kOpChunk, i, op, v, ddt, eps1,
-                                  eps2, dal, dfl);
-            if (code & OP_RELAX)
-                relax_all<RP, K, HOT>(P, M, Z, tr.z, tr.w, eps1, eps2, q);
-            for (int s = 0; s < op_shift1(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            const int rf = op_rf(code);
-            if (rf == RF_ROTATE) {
-                rotate_all<RP, K, HOT>(P, M, Z, tr.x, tr.y, dal);
-            } else if (rf == RF_INVERT) {
-                invert_all<RP, K, HOT>(Z, v);
-            }
-            for (int s = 0; s < op_shift2(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            if (code & OP_SPOIL1) spoil_all<RP, K>(P, M);
-            if (DIST && (code & OP_RECORD)) {
-                const int64_t rec = op.record;
-                const int first = lane - q;
-                const float p0 = __shfl_sync(0xffffffffu, P[0][0].x, first);
-                float val = v.m0 * p0;  // q = 0: the signal
-                float raw = p0;         // q = K + 2: state 0's recorded F+[0]
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const float d = __shfl_sync(0xffffffffu, P[k + 1][0].x, first);
-                    if (q == k + 1) val = HOT ? v.m0 * d : fmaf(v.m0, d, v.dm0[k] * p0);
-                    if (q == K + 3 + k) raw = d;
-                }
-                if (q == K + 1) val = p0;  // the M0 column
-                if (a.layout == TSG_LAYOUT_PLANES) {
-                    if (row_b != nullptr) {
-                        if (row_a != nullptr) row_a[rec] = 0.f;
-                        row_b[rec] = val;
-                    }
-                } else if (row_a != nullptr) {
-                    reinterpret_cast<float2*>(row_a)[rec] = a.layout == TSG_LAYOUT_COMPLEX
-                                                                ? make_float2(0.f, val)
-                                                                : make_float2(-val, 0.f);
-                }
-                if (rec_row != nullptr) rec_row[rec * NS * a.atoms] = raw;
-            } else if ((code & OP_RECORD) && lane0) {
-                const int64_t rec = op.record;
-                const float p0 = P[0][0].x;
-                if (a.sig_a != nullptr || a.sig_b != nullptr)
-                    store_sample(a.layout, a.sig_a, a.sig_b, row * a.outputs + rec, v.m0 * p0);
-                if (a.jac_a != nullptr || a.jac_b != nullptr) {
-                    const int jc = K + a.with_m0;
-#pragma unroll
-                    for (int k = 0; k < K; ++k)
-                        store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + k) * a.outputs + rec,
-                                     HOT ? v.m0 * P[k + 1][0].x
-                                         : fmaf(v.m0, P[k + 1][0].x, v.dm0[k] * p0));
-                    if (a.with_m0)
-                        store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + K) * a.outputs + rec, p0);
-                }
-                if (a.traj_rec) {
-                    float* dst = a.traj_rec + ((train * a.outputs + rec) * NS) * a.atoms + atom;
-#pragma unroll
-                    for (int s = 0; s < NS; ++s) dst[s * a.atoms] = P[s][0].x;
-                }
-            }
-            for (int s = 0; s < op_shift3(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            if (code & OP_SPOIL2) spoil_all<RP, K>(P, M);
+            if (op.code == kPlainOp)
+                step(std::true_type{}, i, op, tr);
+            else
+                step(std::false_type{}, i, op, tr);
         }
     }
 }
@@ -673,41 +689,11 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     int use_slot = 0, fill_slot = D - 1;
     const float2 neg1 = dup(-1.f);
 
-    for (int o = n_ops - 1; o >= 0; --o) {
+    // One op in reverse; of a plain one (as is an odd op's even one then) the
+    // steps are known when this is compiled.
+    auto step = [&](auto plain, int o, int cur, const Op& op) {
+        const uint32_t code = decltype(plain)::value ? kPlainOp : op.code;
         const bool odd = o & 1;
-        const bool new_pair = odd || o == n_ops - 1;
-        if (new_pair) {
-            if (o % G == G - 1 || o == n_ops - 1) {
-                // The transcendentals of the group of G ops that ends here:
-                // lane q of a voxel evaluates the group's op q (a lone lane
-                // both), so one pass of the warp covers them. (Their last
-                // readers are done.)
-                __syncwarp();
-#pragma unroll
-                for (int e = 0; e < (L < 2 ? 2 : 1); ++e) {
-                    const int oq = o - o % G + q + e;
-                    if (slot < VPW && q < G && oq <= o) {
-                        const Op opq = s_ops[oq];
-                        float si = 0.f, co = 1.f;
-                        if (op_rf(opq.code) == RF_ROTATE) sincosf(opq.flip * v.b1, &si, &co);
-                        s_tring[(oq % G) * VPB + vslot] =
-                            make_float4(si, co, expf(-v.r1 * opq.dt), expf(-v.r2 * opq.dt));
-                    }
-                }
-            }
-            // Orders the lanes' reads of the slot this fetch refills (used by
-            // the last pair) and the transcendentals written above.
-            __syncwarp();
-            if ((o >> 1) - (D - 1) >= 0) fetch((o >> 1) - (D - 1), fill_slot);
-            asm volatile("cp.async.commit_group;\n" ::: "memory");
-            fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
-            asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
-            __syncwarp();  // the seeds another lane copied
-        }
-        const Op op = s_ops[o];
-        const uint32_t code = op.code;
-        const int cur = use_slot;
-        if (!odd) use_slot = use_slot + 1 == D ? 0 : use_slot + 1;
         const float4 tr = s_tring[(o % G) * VPB + vslot];
         const float2* ring = s_ring + cur * (NS * 3 * RP * T) + threadIdx.x * RP;
         const float2* sr = s_sring + (cur * 2 + (o & 1)) * (NS * VPB) + vslot;
@@ -726,18 +712,19 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
         float ddt[K], eps1[K], eps2[K], dal[K], dfl[K];
         if (odd) {
             const Op even = s_ops[o - 1];
+            const uint32_t even_code = decltype(plain)::value ? kPlainOp : even.code;
             const float4 te = s_tring[((o - 1) % G) * VPB + vslot];
             op_directions<K, HOT>(a, dirs, n_ops, o - 1, even, v, ddt, eps1, eps2, dal, dfl);
-            if (even.code & OP_RELAX) relax_all<RP, K, HOT>(P, M, Z, te.z, te.w, eps1, eps2, q);
-            for (int s = 0; s < op_shift1(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            if (op_rf(even.code) == RF_ROTATE)
+            if (even_code & OP_RELAX) relax_all<RP, K, HOT>(P, M, Z, te.z, te.w, eps1, eps2, q);
+            for (int s = 0; s < op_shift1(even_code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (op_rf(even_code) == RF_ROTATE)
                 rotate_all<RP, K, HOT>(P, M, Z, te.x, te.y, dal);
-            else if (op_rf(even.code) == RF_INVERT)
+            else if (op_rf(even_code) == RF_INVERT)
                 invert_all<RP, K, HOT>(Z, v);
-            for (int s = 0; s < op_shift2(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            if (even.code & OP_SPOIL1) spoil_all<RP, K>(P, M);
-            for (int s = 0; s < op_shift3(even.code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
-            if (even.code & OP_SPOIL2) spoil_all<RP, K>(P, M);
+            for (int s = 0; s < op_shift2(even_code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (even_code & OP_SPOIL1) spoil_all<RP, K>(P, M);
+            for (int s = 0; s < op_shift3(even_code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
+            if (even_code & OP_SPOIL2) spoil_all<RP, K>(P, M);
         }
         op_directions<K, HOT>(a, dirs, n_ops, o, op, v, ddt, eps1, eps2, dal, dfl);
         const bool relax = (code & OP_RELAX) != 0;
@@ -771,74 +758,7 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
         float e_flip = 0.f, e_dt = 0.f;  // this lane's curvature of the op
         float ev_flip = 0.f, ev_dt = 0.f;  // value (K == 1)
         const int rf = op_rf(code);
-        if (rf == RF_ROTATE) {
-            const float si = tr.x, co = tr.y;
-            const float2 ch = dup(0.5f * (1.f + co)), sh = dup(0.5f * (1.f - co));
-            const float2 hs = dup(0.5f * si), nhs = dup(-0.5f * si), hc = dup(0.5f * co);
-            const float2 si2 = dup(si), nsi2 = dup(-si), co2 = dup(co), nco2 = dup(-co);
-            float2 ga = dup(0.f);  // dL/da, this lane's part
-            float2 gk[K];          // G_k
-#pragma unroll
-            for (int k = 0; k < K; ++k) gk[k] = dup(0.f);
-#pragma unroll
-            for (int kk = 0; kk < RP; ++kk) {
-                const float2 w = fma2(neg1, M[0][kk], P[0][kk]);
-                const float2 z = Z[0][kk];
-                // R'x as (a, b): rows P, M, Z are (-a, a, b); R''x as (c, e)
-                // with rows (-c, c, e).
-                const float2 ax = fma2(hs, w, mul2(co2, z));
-                const float2 bx = fma2(hc, w, mul2(nsi2, z));
-                const float2 ex = fma2(nhs, w, mul2(nco2, z));
-                const float2 dl = fma2(neg1, pb[0][kk], mb[0][kk]);
-                ga = fma2(dl, ax, fma2(zb[0][kk], bx, ga));
-                float2 U = dup(0.f), V = dup(0.f);
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const float2 d = fma2(neg1, pb[k + 1][kk], mb[k + 1][kk]);
-                    const float2 zbk = zb[k + 1][kk];
-                    const float2 wt = fma2(neg1, M[k + 1][kk], P[k + 1][kk]);
-                    const float2 zt = Z[k + 1][kk];
-                    const float2 at = fma2(hs, wt, mul2(co2, zt));
-                    const float2 bt = fma2(hc, wt, mul2(nsi2, zt));
-                    // G_k = d.ax + zb.bx; H_k = d.at + zb.bt;
-                    // I_k = d.(hc w - si z) + zb.(-hs w - co z) = d.bx + zb.ex.
-                    gk[k] = fma2(d, ax, fma2(zbk, bx, gk[k]));
-                    ga = fma2(d, at, fma2(zbk, bt, ga));
-                    if (!HOT || hot_dir(HOT, k) == 3) {
-                        const float2 al = dup(dal[k]);
-                        ga = fma2(al, fma2(d, bx, mul2(zbk, ex)), ga);
-                        // (R'^T mu_k): P (hs d + hc zb), M -(..), Z (co d - si zb).
-                        U = fma2(al, fma2(hs, d, mul2(hc, zbk)), U);
-                        V = fma2(al, fma2(co2, d, mul2(nsi2, zbk)), V);
-                    }
-                    // mu_k <- R^T mu_k.
-                    const float2 p_ = pb[k + 1][kk], m_ = mb[k + 1][kk];
-                    pb[k + 1][kk] = fma2(ch, p_, fma2(sh, m_, mul2(hs, zbk)));
-                    mb[k + 1][kk] = fma2(sh, p_, fma2(ch, m_, mul2(nhs, zbk)));
-                    zb[k + 1][kk] = fma2(si2, d, mul2(co2, zbk));
-                }
-                const float2 p_ = pb[0][kk], m_ = mb[0][kk], z_ = zb[0][kk];
-                pb[0][kk] = fma2(ch, p_, fma2(sh, m_, fma2(hs, z_, U)));
-                mb[0][kk] = fma2(sh, p_, fma2(ch, m_, fma2(nhs, z_, mul2(neg1, U))));
-                zb[0][kk] = fma2(si2, dl, fma2(co2, z_, V));
-            }
-            const float gsum = ga.x + ga.y;
-            float gf = gsum * v.b1, gb = gsum * op.flip;
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const float g = gk[k].x + gk[k].y;
-                if (HOT) {
-                    if (hot_dir(HOT, k) == 3) gf += g;
-                    continue;
-                }
-                gf = fmaf(g, v.db1[k], gf);
-                gb = fmaf(g, dfl[k], gb);
-                v_b1[k] = fmaf(g, op.flip, v_b1[k]);
-                if (K == 1) ev_flip = g * v.b1;
-            }
-            e_flip = gf;
-            c_b1 += gb;
-        } else if (rf == RF_INVERT) {
+        if (rf == RF_INVERT) {
             const float2 f = dup(-v.eff);
             float2 acc = dup(0.f);
             float2 vk[K];
@@ -865,35 +785,90 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
 #pragma unroll
                 for (int k = 0; k < K; ++k) v_inv[k] -= vk[k].x + vk[k].y;
         }
-        if (relax) {
-            // Q2, Q1 and C2_k, C1_k at the pre-RF point.
-            float2 q2 = dup(0.f), q1 = dup(0.f);
-            float zx0 = 0.f;  // the recovery target's part of lam.(x - e0)
+        // The pulse, in u = F+ + F-, w = F+ - F- (a pulse leaves u and turns
+        // (w, Z), commuting with its generator w -> -2 Z, Z -> w / 2) and
+        // their cotangents U, W = (F+_bar +- F-_bar) / 2; and at the point
+        // before it the relaxation's inner products.
+        const bool rotate = rf == RF_ROTATE;
+        const float si = tr.x, co = tr.y;
+        const float2 half = dup(0.5f), nhalf = dup(-0.5f);
+        const float2 co2 = dup(co), hs = dup(0.5f * si), ns2 = dup(-2.f * si);
+        float2 wz = dup(0.f), zw = dup(0.f);  // of dL/da
+        float2 q2 = dup(0.f), q1 = dup(0.f);
+        float2 gwz[K], gzw[K], c2[K], c1[K];  // of G_k; C2_k and C1_k
 #pragma unroll
-            for (int kk = 0; kk < RP; ++kk) {
-                q2 = fma2(pb[0][kk], P[0][kk], fma2(mb[0][kk], M[0][kk], q2));
-                q1 = fma2(zb[0][kk], Z[0][kk], q1);
+        for (int k = 0; k < K; ++k) gwz[k] = gzw[k] = c2[k] = c1[k] = dup(0.f);
+#pragma unroll
+        for (int kk = 0; kk < RP; ++kk) {
+            const float2 ux = add2(P[0][kk], M[0][kk]), wx = fma2(neg1, M[0][kk], P[0][kk]);
+            const float2 zx = Z[0][kk];
+            float2 more_w = dup(0.f), more_z = dup(0.f);  // K^T mu_k a'_k
+#pragma unroll
+            for (int s = K; s >= 0; --s) {
+                const int k = s - 1;
+                const float2 u = s ? add2(P[s][kk], M[s][kk]) : ux;
+                const float2 w = s ? fma2(neg1, M[s][kk], P[s][kk]) : wx;
+                const float2 z = Z[s][kk];
+                const float2 hp = mul2(half, pb[s][kk]);
+                const float2 U = fma2(half, mb[s][kk], hp);
+                float2 W = fma2(nhalf, mb[s][kk], hp), Zb = zb[s][kk];
+                if (rotate) {
+                    float2 W1 = mul2(co2, W), Z1 = mul2(ns2, W);
+                    if (!s) {
+                        W1 = add2(W1, more_w);
+                        Z1 = add2(Z1, more_z);
+                    }
+                    W = fma2(hs, Zb, W1);
+                    Zb = fma2(co2, Zb, Z1);
+                    wz = fma2(W, z, wz);
+                    zw = fma2(Zb, w, zw);
+                }
+                if (s && (!HOT || hot_dir(HOT, k) == 3) && rotate) {
+                    gwz[k] = fma2(W, zx, gwz[k]);
+                    gzw[k] = fma2(Zb, wx, gzw[k]);
+                    more_w = fma2(dup(0.5f * dal[k]), Zb, more_w);
+                    more_z = fma2(dup(-2.f * dal[k]), W, more_z);
+                }
+                q2 = fma2(U, u, fma2(W, w, q2));
+                q1 = fma2(Zb, z, q1);
+                if (s && (!HOT || hot_dir(HOT, k) == 2)) c2[k] = fma2(U, ux, fma2(W, wx, c2[k]));
+                if (s && (!HOT || hot_dir(HOT, k) == 1)) c1[k] = fma2(Zb, zx, c1[k]);
+                pb[s][kk] = add2(U, W);
+                mb[s][kk] = fma2(neg1, W, U);
+                zb[s][kk] = Zb;
             }
-            if (q == 0) zx0 = zb[0][0].x;
-            float Q2 = q2.x + q2.y, Q1 = q1.x + q1.y - zx0;
+        }
+        if (rotate) {
+            const float gsum = 0.5f * (zw.x + zw.y) - 2.f * (wz.x + wz.y);
+            float gf = gsum * v.b1, gb = gsum * op.flip;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const float g = 0.5f * (gzw[k].x + gzw[k].y) - 2.f * (gwz[k].x + gwz[k].y);
+                if (HOT) {
+                    if (hot_dir(HOT, k) == 3) gf += g;
+                    continue;
+                }
+                gf = fmaf(g, v.db1[k], gf);
+                gb = fmaf(g, dfl[k], gb);
+                v_b1[k] = fmaf(g, op.flip, v_b1[k]);
+                if (K == 1) ev_flip = g * v.b1;
+            }
+            e_flip = gf;
+            c_b1 += gb;
+        }
+        if (relax) {
+            const float Q2 = q2.x + q2.y;
+            float Q1 = q1.x + q1.y;
+            // The recovery target's part of lam.(x - e0).
+            if (q == 0) Q1 -= zb[0][0].x;
             float dtc = 0.f;
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                // C2_k and C1_k: a one-hot direction needs only its own.
+                // A one-hot direction needs only its own.
                 const bool n2 = !HOT || hot_dir(HOT, k) == 2;
                 const bool n1 = !HOT || hot_dir(HOT, k) == 1;
-                float2 c2 = dup(0.f), c1 = dup(0.f), t2 = dup(0.f), t1 = dup(0.f);
-#pragma unroll
-                for (int kk = 0; kk < RP; ++kk) {
-                    if (n2) c2 = fma2(pb[k + 1][kk], P[0][kk], fma2(mb[k + 1][kk], M[0][kk], c2));
-                    if (n1) c1 = fma2(zb[k + 1][kk], Z[0][kk], c1);
-                    t2 = fma2(pb[k + 1][kk], P[k + 1][kk], fma2(mb[k + 1][kk], M[k + 1][kk], t2));
-                    t1 = fma2(zb[k + 1][kk], Z[k + 1][kk], t1);
-                }
-                Q2 += t2.x + t2.y;
-                Q1 += t1.x + t1.y;
-                const float C2 = n2 ? c2.x + c2.y : 0.f;
-                const float C1 = n1 ? c1.x + c1.y - (q == 0 ? zb[k + 1][0].x : 0.f) : 0.f;
+                const float C2 = n2 ? c2[k].x + c2[k].y : 0.f;
+                const float C1 = n1 ? c1[k].x + c1[k].y - (q == 0 ? zb[k + 1][0].x : 0.f) : 0.f;
                 if (HOT) {
                     // r'_k = -w for the unit tangent of T1 (or T2).
                     if (n2) {
@@ -940,22 +915,67 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                 zb[0][kk] = lz;
             }
         }
-        // The op's event partials summed over the warp (a fixed butterfly;
-        // nothing on the state recursion waits for it).
-        float ev[2 * NE2] = {active ? e_flip : 0.f, active ? e_dt : 0.f};
+        // The op's event partials summed over the warp in a fixed order: one
+        // exchange (two for four values) leaves each lane one of the values,
+        // the rest sum it. Nothing on the state recursion waits for it.
+        float f0 = active ? e_flip : 0.f, f1 = active ? e_dt : 0.f;
+        const bool upper = lane & 16, high = lane & 8;
         if constexpr (NE2 == 2) {
-            ev[2] = active ? ev_flip : 0.f;
-            ev[3] = active ? ev_dt : 0.f;
+            float f2 = active ? ev_flip : 0.f, f3 = active ? ev_dt : 0.f;
+            const float x0 = __shfl_xor_sync(0xffffffffu, upper ? f0 : f2, 16);
+            const float x1 = __shfl_xor_sync(0xffffffffu, upper ? f1 : f3, 16);
+            f0 = (upper ? f2 : f0) + x0;
+            f1 = (upper ? f3 : f1) + x1;
+            f0 = (high ? f1 : f0) + __shfl_xor_sync(0xffffffffu, high ? f0 : f1, 8);
+        } else {
+            f0 = (upper ? f1 : f0) + __shfl_xor_sync(0xffffffffu, upper ? f0 : f1, 16);
+            f0 += __shfl_xor_sync(0xffffffffu, f0, 8);
         }
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
+        for (int off = 4; off > 0; off >>= 1) f0 += __shfl_xor_sync(0xffffffffu, f0, off);
+        constexpr int kHolders = 16 / NE2;  // lanes that hold one value
+        if (lane % kHolders == 0)
+            reinterpret_cast<float*>(event_out + int64_t(o) * NE2)[lane / kHolders] = f0;
+    };
+
+    for (int o = n_ops - 1; o >= 0; --o) {
+        const bool odd = o & 1;
+        const bool new_pair = odd || o == n_ops - 1;
+        if (new_pair) {
+            if (o % G == G - 1 || o == n_ops - 1) {
+                // The transcendentals of the group of G ops that ends here:
+                // lane q of a voxel evaluates the group's op q (a lone lane
+                // both), so one pass of the warp covers them. (Their last
+                // readers are done.)
+                __syncwarp();
 #pragma unroll
-            for (int e = 0; e < 2 * NE2; ++e) ev[e] += __shfl_xor_sync(0xffffffffu, ev[e], off);
-        if (lane == 0) {
-#pragma unroll
-            for (int e = 0; e < NE2; ++e)
-                event_out[int64_t(o) * NE2 + e] = make_float2(ev[2 * e], ev[2 * e + 1]);
+                for (int e = 0; e < (L < 2 ? 2 : 1); ++e) {
+                    const int oq = o - o % G + q + e;
+                    if (slot < VPW && q < G && oq <= o) {
+                        const Op opq = s_ops[oq];
+                        float si = 0.f, co = 1.f;
+                        if (op_rf(opq.code) == RF_ROTATE) sincosf(opq.flip * v.b1, &si, &co);
+                        s_tring[(oq % G) * VPB + vslot] =
+                            make_float4(si, co, expf(-v.r1 * opq.dt), expf(-v.r2 * opq.dt));
+                    }
+                }
+            }
+            // Orders the lanes' reads of the slot this fetch refills (used by
+            // the last pair) and the transcendentals written above.
+            __syncwarp();
+            if ((o >> 1) - (D - 1) >= 0) fetch((o >> 1) - (D - 1), fill_slot);
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+            fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
+            asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
+            __syncwarp();  // the seeds another lane copied
         }
+        const Op op = s_ops[o];
+        const int cur = use_slot;
+        if (!odd) use_slot = use_slot + 1 == D ? 0 : use_slot + 1;
+        if (op.code == kPlainOp && (!odd || s_ops[o - 1].code == kPlainOp))
+            step(std::true_type{}, o, cur, op);
+        else
+            step(std::false_type{}, o, cur, op);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
 
