@@ -81,7 +81,7 @@ struct SecondArgs {
     float* jac_b;
     // Trajectory: [train][warp][op / 2][state][plane][lane][RP] float2 (state
     // 0 = x, k + 1 = t_k; warp = atom / (32 / lanes_per_voxel)), and the
-    // recorded F+[0] of each state, [train][output][state][atom].
+    // recorded F+[0] of each state, [train][state][atom][output].
     float2* traj;
     float* traj_rec;
     // Reverse: cotangents of the signal (nullable) and of the derivatives
@@ -357,7 +357,6 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
     const Op* ops = a.ops + train * a.n_ops;
     const int64_t n_all = int64_t(gridDim.y) * a.n_ops;  // ops of all trains, per direction
     const float2* dirs = a.op_dir ? a.op_dir + train * a.n_ops : nullptr;
-    const int64_t row = train * a.atoms + atom;
     // This warp's tile; lanes of a warp past the last voxel store nothing.
     const int64_t n_warps = (a.atoms + VPW - 1) / VPW;
     const int64_t warp_global = int64_t(blockIdx.x) * (blockDim.x >> 5) + warp;
@@ -368,45 +367,64 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
                                   lane * RP
                             : nullptr;
     const bool lane0 = active && q == 0;
-    // Distributed records: with 2K + 3 lanes per voxel or more, lane q of
-    // the voxel writes one output of a record from a pointer set up once
-    // (q = 0 the signal, 1..K the derivative columns, K + 1 the M0 column,
-    // K + 2 + s state s's recorded F+[0] for the reverse), the values coming
-    // from lane 0 by shuffle: one store instruction per record instead of up
-    // to 2K + 3 serial ones in lane 0.
-    constexpr bool DIST = L >= 2 * K + 3;
-    float* row_a = nullptr;    // this lane's output row: plane a, or the complex row
-    float* row_b = nullptr;    // plane b of the planes layout
-    float* rec_row = nullptr;  // this lane's recorded-F+[0] row of the trajectory
-    if constexpr (DIST) {
-        if (active) {
-            float* ba = nullptr;
-            float* bb = nullptr;
-            int64_t off = 0;
-            const int jc = K + a.with_m0;
-            if (q == 0) {
-                if (a.sig_a != nullptr || a.sig_b != nullptr) {
-                    ba = a.sig_a;
-                    bb = a.sig_b;
-                    off = row * a.outputs;
-                }
-            } else if (q <= K || (q == K + 1 && a.with_m0)) {
-                if (a.jac_a != nullptr || a.jac_b != nullptr) {
-                    ba = a.jac_a;
-                    bb = a.jac_b;
-                    off = (row * jc + (q - 1)) * a.outputs;
-                }
-            } else if (q >= K + 2 && q < K + 2 + NS && a.traj_rec != nullptr) {
-                rec_row = a.traj_rec + (train * a.outputs * NS + (q - K - 2)) * a.atoms + atom;
-            }
-            if (a.layout == TSG_LAYOUT_PLANES) {
-                row_a = ba ? ba + off : nullptr;
-                row_b = bb ? bb + off : nullptr;
-            } else if (ba) {
-                row_a = reinterpret_cast<float*>(reinterpret_cast<float2*>(ba) + off);
-            }
+    // Samples: the recorded F+[0] of x and of each t_k wait in shared memory,
+    // EC at a time, and leave as rows (the signal, the derivative columns, the
+    // M0 column, and what the reverse sweep reads of every state). Stored
+    // where they are recorded they were 2 K + 3 partial sectors a voxel and
+    // op, which bound the sweep (1.57 ms; 0.89 ms in rows). With fewer than
+    // four lanes a voxel, a warp's rows are not worth their shared memory.
+    constexpr bool STAGED = L >= 4;
+    constexpr int EC = L >= 8 ? 16 : 8;
+    __shared__ float s_rec[STAGED ? 4 : 1][STAGED ? VPW * NS * (EC + 1) : 1];
+    __shared__ int s_index[4][EC];
+    float* rec_raw = s_rec[STAGED ? warp : 0];
+    int held = 0;
+    const bool with_sig = a.layout == TSG_LAYOUT_PLANES ? a.sig_b != nullptr : a.sig_a != nullptr;
+    const bool with_jac = a.layout == TSG_LAYOUT_PLANES ? a.jac_b != nullptr : a.jac_a != nullptr;
+    const int jac_cols = K + a.with_m0;
+    // One voxel's outputs of one record, from the recorded values raw[state].
+    auto put_record = [&](int64_t voxel, int64_t rec, const float (&raw)[NS], float m0,
+                          const float (&dm0)[K]) {
+        const int64_t out = train * a.atoms + voxel;
+        if (with_sig)
+            store_sample(a.layout, a.sig_a, a.sig_b, out * a.outputs + rec, m0 * raw[0]);
+        if (with_jac) {
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                store_sample(a.layout, a.jac_a, a.jac_b, (out * jac_cols + k) * a.outputs + rec,
+                             HOT ? m0 * raw[k + 1] : fmaf(m0, raw[k + 1], dm0[k] * raw[0]));
+            if (a.with_m0)
+                store_sample(a.layout, a.jac_a, a.jac_b, (out * jac_cols + K) * a.outputs + rec,
+                             raw[0]);
         }
-    }
+        if (a.traj_rec) {
+#pragma unroll
+            for (int s = 0; s < NS; ++s)
+                a.traj_rec[((train * NS + s) * a.atoms + voxel) * a.outputs + rec] = raw[s];
+        }
+    };
+    auto flush = [&]() {
+        __syncwarp();
+        const int col = lane % EC;
+#pragma unroll 1
+        for (int first = 0; first < VPW; first += 32 / EC) {
+            const int vv = first + lane / EC;
+            const int from = min(vv, VPW - 1) * L;
+            const float m0 = __shfl_sync(0xffffffffu, v.m0, from);
+            float dm0[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                dm0[k] = HOT ? 0.f : __shfl_sync(0xffffffffu, v.dm0[k], from);
+            const int64_t voxel = warp_global * VPW + vv;
+            if (vv >= VPW || voxel >= a.atoms || col >= held) continue;
+            float raw[NS];
+#pragma unroll
+            for (int s = 0; s < NS; ++s) raw[s] = rec_raw[(vv * NS + s) * (EC + 1) + col];
+            put_record(voxel, s_index[warp][col], raw, m0, dm0);
+        }
+        __syncwarp();
+        held = 0;
+    };
 
     // One op; of a plain one (kPlainOp, most ops of a fingerprinting train) the
     // steps are known when this is compiled.
@@ -438,49 +456,20 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
         }
         for (int s = 0; s < op_shift2(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
         if (code & OP_SPOIL1) spoil_all<RP, K>(P, M);
-        if (DIST && (code & OP_RECORD)) {
-            const int64_t rec = op.record;
-            const int first = lane - q;
-            const float p0 = __shfl_sync(0xffffffffu, P[0][0].x, first);
-            float val = v.m0 * p0;  // q = 0: the signal
-            float raw = p0;         // q = K + 2: state 0's recorded F+[0]
+        if (code & OP_RECORD) {
+            if constexpr (STAGED) {
+                if (q == 0 && slot < VPW) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const float d = __shfl_sync(0xffffffffu, P[k + 1][0].x, first);
-                if (q == k + 1) val = HOT ? v.m0 * d : fmaf(v.m0, d, v.dm0[k] * p0);
-                if (q == K + 3 + k) raw = d;
-            }
-            if (q == K + 1) val = p0;  // the M0 column
-            if (a.layout == TSG_LAYOUT_PLANES) {
-                if (row_b != nullptr) {
-                    if (row_a != nullptr) row_a[rec] = 0.f;
-                    row_b[rec] = val;
+                    for (int s = 0; s < NS; ++s)
+                        rec_raw[(slot * NS + s) * (EC + 1) + held] = P[s][0].x;
                 }
-            } else if (row_a != nullptr) {
-                reinterpret_cast<float2*>(row_a)[rec] = a.layout == TSG_LAYOUT_COMPLEX
-                                                            ? make_float2(0.f, val)
-                                                            : make_float2(-val, 0.f);
-            }
-            if (rec_row != nullptr) rec_row[rec * NS * a.atoms] = raw;
-        } else if ((code & OP_RECORD) && lane0) {
-            const int64_t rec = op.record;
-            const float p0 = P[0][0].x;
-            if (a.sig_a != nullptr || a.sig_b != nullptr)
-                store_sample(a.layout, a.sig_a, a.sig_b, row * a.outputs + rec, v.m0 * p0);
-            if (a.jac_a != nullptr || a.jac_b != nullptr) {
-                const int jc = K + a.with_m0;
+                if (lane == 0) s_index[warp][held] = op.record;
+                if (++held == EC) flush();
+            } else if (lane0) {
+                float raw[NS];
 #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + k) * a.outputs + rec,
-                                 HOT ? v.m0 * P[k + 1][0].x
-                                     : fmaf(v.m0, P[k + 1][0].x, v.dm0[k] * p0));
-                if (a.with_m0)
-                    store_sample(a.layout, a.jac_a, a.jac_b, (row * jc + K) * a.outputs + rec, p0);
-            }
-            if (a.traj_rec) {
-                float* dst = a.traj_rec + ((train * a.outputs + rec) * NS) * a.atoms + atom;
-#pragma unroll
-                for (int s = 0; s < NS; ++s) dst[s * a.atoms] = P[s][0].x;
+                for (int s = 0; s < NS; ++s) raw[s] = P[s][0].x;
+                put_record(atom, op.record, raw, v.m0, v.dm0);
             }
         }
         for (int s = 0; s < op_shift3(code); ++s) shift_all<RP, L, K>(P, M, q, kill, kill_r);
@@ -520,6 +509,7 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
                 step(std::false_type{}, i, op, tr);
         }
     }
+    if (STAGED && held > 0) flush();
 }
 
 // ---- reverse ---------------------------------------------------------------
@@ -604,7 +594,7 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                                      : nullptr;
     const int jc = K + a.with_m0;
     const float* seed_row = a.seed + (active ? row : 0) * jc * a.outputs * seed_stride;
-    const float* rec_col = a.traj_rec + train * a.outputs * NS * n + ac;
+    const float* rec_row = a.traj_rec + (train * NS * n + ac) * a.outputs;
 
     // This warp's tile (a warp past the last voxel reads tile 0 and keeps
     // nothing of it).
@@ -665,7 +655,7 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                 for (int s = 0; s < NS; ++s)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
                                      sdst + unsigned(s * VPB) * 8u + 4u),
-                                 "l"(rec_col + (r * NS + s) * n), "r"(rec ? 4 : 0)
+                                 "l"(rec_row + s * n * a.outputs + r), "r"(rec ? 4 : 0)
                                  : "memory");
                 const bool have_m = rec && a.with_m0;
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
