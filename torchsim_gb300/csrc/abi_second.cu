@@ -200,17 +200,17 @@ int second_plan(const tsg_program* prog, int64_t atoms, int64_t states, int k, i
     plan->event_bytes = align256(trains * plan->warps_per_train * ops * event_pairs(k, hot) * 8);
     plan->workspace_bytes = plan->dir_bytes + plan->event_bytes +
                             trains * atoms * tissue_values(k, hot) * int64_t(sizeof(float));
-    // The reverse sweep's rings, a slot per pair of ops (states per lane; of
-    // both ops seeds and records per voxel slot), a group's transcendentals,
-    // its ops and op directions.
+    // The reverse sweep's ring (states per lane, a slot per pair of ops), a
+    // group's transcendentals, the records' values and indexes, its ops and op
+    // directions.
     const int T = 32 * kSecondWarps;
     const int RP = best->orders_per_lane / 2;
-    const size_t slots = size_t(vpb), slots4 = (slots + 3) & ~size_t(3);
-    plan->smem = size_t(kSecondRing) *
-                     (sizeof(float2) * size_t((k + 1) * 3 * RP) * T +
-                      2 * (sizeof(float2) * size_t(k + 1) * slots + sizeof(float) * slots4)) +
+    const size_t slots = size_t(vpb), records = size_t(second_records(best->lanes_per_voxel));
+    plan->smem = size_t(kSecondRing) * sizeof(float2) * size_t((k + 1) * 3 * RP) * T +
                  sizeof(float4) * slots * size_t(second_group(best->lanes_per_voxel)) +
-                 sizeof(Op) * size_t(ops) + (event_directions ? sizeof(float2) * size_t(k * ops) : 0);
+                 sizeof(float) * slots * size_t(second_record_items(k, hot)) * records +
+                 sizeof(int) * kSecondWarps * records + sizeof(Op) * size_t(ops) +
+                 (event_directions ? sizeof(float2) * size_t(k * ops) : 0);
     if (plan->smem > 226 * 1024)
         return fail(TSG_ERR_CAPACITY, "the program does not fit in shared memory for the reverse sweep");
     if (plan->blocks > 0x7fffffffLL || trains > 65535) return fail(TSG_ERR_CAPACITY, "launch too large");

@@ -115,6 +115,16 @@ inline int64_t second_trajectory_floats(int64_t trains, int64_t atoms, int64_t o
 // takes two).
 __host__ __device__ constexpr int second_group(int lanes) { return lanes < 2 ? 2 : lanes & ~1; }
 
+// Records held in shared memory per warp (fewer where a warp holds more
+// voxels), and the reverse's values of each: a cotangent per state and M0's
+// curvature, with general directions M0's K derivatives too.
+__host__ __device__ constexpr int second_records(int lanes) {
+    return lanes >= 8 ? 16 : lanes >= 4 ? 8 : 4;
+}
+__host__ __device__ constexpr int second_record_items(int k, int hot) {
+    return k + 2 + (hot ? 0 : k);
+}
+
 inline int64_t second_record_floats(int64_t trains, int64_t atoms, int64_t outputs, int k) {
     return trains * outputs * (k + 1) * atoms;
 }
@@ -374,7 +384,7 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
     // op, which bound the sweep (1.57 ms; 0.89 ms in rows). With fewer than
     // four lanes a voxel, a warp's rows are not worth their shared memory.
     constexpr bool STAGED = L >= 4;
-    constexpr int EC = L >= 8 ? 16 : 8;
+    constexpr int EC = second_records(L);
     __shared__ float s_rec[STAGED ? 4 : 1][STAGED ? VPW * NS * (EC + 1) : 1];
     __shared__ int s_index[4][EC];
     float* rec_raw = s_rec[STAGED ? warp : 0];
@@ -514,11 +524,10 @@ __global__ void __launch_bounds__(128) second_forward_kernel(const SecondArgs a)
 
 // ---- reverse ---------------------------------------------------------------
 
-// Dynamic shared memory, a ring slot per pair of ops: entry states of the even
-// op [D][NS][3][RP][T] float2, transcendentals [G][VPB] float4, of both ops
-// (seed, recorded F+[0]) [D][2][NS][VPB] float2 and the M0 derivative's seed
-// [D][2][VPB4] float, ops [n_ops], per-direction op directions [K][n_ops]
-// float2 (only with event directions).
+// Dynamic shared memory: entry states of the even op [D][NS][3][RP][T] float2
+// (a ring slot per pair of ops), transcendentals [G][VPB] float4, the records'
+// values [W][VPW][NI][EC] float and indexes [W][EC] int, ops [n_ops],
+// per-direction op directions [K][n_ops] float2 (only with event directions).
 template <int RP, int L, int K, int HOT>
 __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const SecondArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -547,16 +556,14 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     const int64_t row = train * n + atom;
     const int vslot = warp * VPW + (slot < VPW ? slot : VPW - 1);
 
-    // Per voxel slot (not per lane): the transcendentals, seeds and
-    // recorded F+[0] one lane of the voxel fetches.
-    constexpr int VPB = W * VPW;
-    constexpr int VPB4 = (VPB + 3) & ~3;
+    constexpr int VPB = W * VPW;  // transcendentals are per voxel slot
+    constexpr int EC = second_records(L), NI = second_record_items(K, HOT);
     float2* s_ring = reinterpret_cast<float2*>(s_raw);                    // [D][NS*3][T][RP]
     constexpr int G = second_group(L);
     float4* s_tring = reinterpret_cast<float4*>(s_ring + D * NS * 3 * RP * T);  // [G][VPB]
-    float2* s_sring = reinterpret_cast<float2*>(s_tring + G * VPB);       // [D][2][NS][VPB]
-    float* s_mring = reinterpret_cast<float*>(s_sring + D * 2 * NS * VPB);  // [D][2][VPB4]
-    Op* s_ops = reinterpret_cast<Op*>(s_mring + D * 2 * VPB4);             // [n_ops]
+    float* s_seed = reinterpret_cast<float*>(s_tring + G * VPB);          // [W][VPW][NI][EC]
+    int* s_index = reinterpret_cast<int*>(s_seed + W * VPW * NI * EC);     // [W][EC]
+    Op* s_ops = reinterpret_cast<Op*>(s_index + W * EC);                   // [n_ops]
     float2* s_dir = reinterpret_cast<float2*>(s_ops + n_ops);              // [K][n_ops]
 
     const Voxel<K> v = load_voxel<K, HOT>(a, ac);
@@ -590,11 +597,62 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
     const bool planes = a.seed_layout == TSG_LAYOUT_PLANES;
     const int seed_stride = planes ? 1 : 2;
     const float seed_sign = planes ? 1.f : -1.f;
-    const float* seed0_row = a.seed0 ? a.seed0 + (active ? row : 0) * a.outputs * seed_stride
-                                     : nullptr;
     const int jc = K + a.with_m0;
-    const float* seed_row = a.seed + (active ? row : 0) * jc * a.outputs * seed_stride;
-    const float* rec_row = a.traj_rec + (train * NS * n + ac) * a.outputs;
+    float* seeds = s_seed + warp * VPW * NI * EC;
+    int* index = s_index + warp * EC;
+    // The next records of the reverse sweep, from op o down, up to EC: their
+    // cotangents of F+[0] of every state and their parts of the M0 sums,
+    // read as rows. (Read one by one where they were used, they were 2 K + 3
+    // copies of four bytes for each voxel and op.)
+    int left = 0, at = 0;
+    auto refill = [&](int o) {
+        __syncwarp();
+        const int j = o - lane;
+        const bool rec = j >= 0 && (s_ops[j].code & OP_RECORD);
+        const unsigned set = __ballot_sync(0xffffffffu, rec);
+        const int rank = __popc(set & ((1u << lane) - 1u));
+        if (rec && rank < EC) index[rank] = s_ops[j].record;
+        left = min(__popc(set), EC);
+        at = 0;
+        __syncwarp();
+        const int col = lane % EC;
+#pragma unroll 1
+        for (int first = 0; first < VPW; first += 32 / EC) {
+            const int vv = first + lane / EC;
+            const int from = min(vv, VPW - 1) * L;
+            const float m0 = __shfl_sync(0xffffffffu, v.m0, from);
+            float dm0[K];
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+                dm0[k] = HOT ? 0.f : __shfl_sync(0xffffffffu, v.dm0[k], from);
+            const int64_t voxel = warp_global * VPW + vv;
+            if (vv >= VPW || voxel >= n || col >= left) continue;
+            const int64_t r = index[col];
+            const int64_t out = train * n + voxel;
+            const float* x = a.traj_rec + (train * NS * n + voxel) * a.outputs + r;
+            const float* g = a.seed + (out * jc * a.outputs + r) * seed_stride;
+            float* dst = seeds + vv * NI * EC + col;
+            const float x0 = x[0];
+            const float g0 = a.seed0 ? seed_sign * a.seed0[(out * a.outputs + r) * seed_stride] : 0.f;
+            // The M0 derivative is F+[0] itself: its seed acts unscaled.
+            float add0 = g0 * m0, m0_sum = g0 * x0;
+            if (a.with_m0)
+                add0 = fmaf(seed_sign, g[int64_t(K) * a.outputs * seed_stride], add0);
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const float gk = seed_sign * g[int64_t(k) * a.outputs * seed_stride];
+                if (!HOT) {
+                    add0 = fmaf(gk, dm0[k], add0);
+                    dst[(NS + 1 + k) * EC] = gk * x0;
+                }
+                dst[(k + 1) * EC] = gk * m0;
+                m0_sum = fmaf(gk, x[(k + 1) * n * a.outputs], m0_sum);
+            }
+            dst[0] = add0;
+            dst[NS * EC] = m0_sum;
+        }
+        __syncwarp();
+    };
 
     // This warp's tile (a warp past the last voxel reads tile 0 and keeps
     // nothing of it).
@@ -606,12 +664,8 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
         lane * RP;
     const unsigned ring_base =
         static_cast<unsigned>(__cvta_generic_to_shared(s_ring + threadIdx.x * RP));
-    const unsigned sring_base = static_cast<unsigned>(__cvta_generic_to_shared(s_sring + vslot));
-    const unsigned mring_base = static_cast<unsigned>(__cvta_generic_to_shared(s_mring + vslot));
 
-    // Pair i (ops 2 i, 2 i + 1) into ring slot rs: the even op's entry states,
-    // and of both ops the seeds and recorded F+[0] (zero unless this lane
-    // records).
+    // Pair i (ops 2 i, 2 i + 1) into ring slot rs: the even op's entry states.
     auto fetch = [&](int i, int rs) {
         const float2* src_op = lane_traj + i * op_stride;
         const unsigned dst_op = ring_base + unsigned(rs * NS * 3 * RP * T) * 8u;
@@ -628,41 +682,6 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst + 8u * kk),
                                  "l"(src + kk)
                                  : "memory");
-            }
-        }
-        // Seeds and recorded F+[0]: lane 0 of each voxel slot copies them
-        // (zeros unless the voxel is live and the op records).
-        if (q == 0 && slot < VPW) {
-#pragma unroll 1
-            for (int h = 0; h < 2; ++h) {
-                const int o = 2 * i + h;
-                if (o >= n_ops) break;
-                const Op op = s_ops[o];
-                const bool rec = lane0 && (op.code & OP_RECORD);
-                const int64_t r = rec ? op.record : 0;
-                const unsigned sdst = sring_base + unsigned((rs * 2 + h) * NS * VPB) * 8u;
-                const bool have0 = rec && seed0_row != nullptr;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sdst),
-                             "l"(have0 ? seed0_row + r * seed_stride : a.seed), "r"(have0 ? 4 : 0)
-                             : "memory");
-    #pragma unroll
-                for (int k = 0; k < K; ++k)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                                     sdst + unsigned((k + 1) * VPB) * 8u),
-                                 "l"(seed_row + (k * a.outputs + r) * seed_stride), "r"(rec ? 4 : 0)
-                                 : "memory");
-    #pragma unroll
-                for (int s = 0; s < NS; ++s)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                                     sdst + unsigned(s * VPB) * 8u + 4u),
-                                 "l"(rec_row + s * n * a.outputs + r), "r"(rec ? 4 : 0)
-                                 : "memory");
-                const bool have_m = rec && a.with_m0;
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(
-                                 mring_base + unsigned((rs * 2 + h) * VPB4) * 4u),
-                             "l"(have_m ? seed_row + (K * a.outputs + r) * seed_stride : a.seed),
-                             "r"(have_m ? 4 : 0)
-                             : "memory");
             }
         }
     };
@@ -686,7 +705,6 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
         const bool odd = o & 1;
         const float4 tr = s_tring[(o % G) * VPB + vslot];
         const float2* ring = s_ring + cur * (NS * 3 * RP * T) + threadIdx.x * RP;
-        const float2* sr = s_sring + (cur * 2 + (o & 1)) * (NS * VPB) + vslot;
 
         // The pre-RF states: entry states (an odd op's by running the even op
         // before it), relaxed and pre-shifted.
@@ -724,23 +742,19 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
         // Reverse of the op's micro-steps after the pulse.
         if (code & OP_SPOIL2) spoil_all<RP, K>(pb, mb);
         for (int s = 0; s < op_shift3(code); ++s) shift_adjoint_all<RP, L, K>(pb, mb, q, kill, kill_r);
-        if ((code & OP_RECORD) && lane0) {
-            const float g0 = seed_sign * sr[0].x;
-            const float x0 = sr[0].y;
-            // The M0 derivative is F+[0] itself: its seed acts unscaled.
-            const float g_m0col = s_mring[(cur * 2 + (o & 1)) * VPB4 + vslot];
-            float add0 = fmaf(g0, v.m0, seed_sign * g_m0col);
-            c_m0 = fmaf(g0, x0, c_m0);
+        if (code & OP_RECORD) {
+            if (left == 0) refill(o);
+            if (lane0) {
+                const float* sv = seeds + slot * NI * EC + at;
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const float gk = seed_sign * sr[(k + 1) * VPB].x;
-                const float tk0 = sr[(k + 1) * VPB].y;
-                if (!HOT) add0 = fmaf(gk, v.dm0[k], add0);
-                pb[k + 1][0].x = fmaf(gk, v.m0, pb[k + 1][0].x);
-                c_m0 = fmaf(gk, tk0, c_m0);
-                if (!HOT) v_m0[k] = fmaf(gk, x0, v_m0[k]);
+                for (int s = 0; s < NS; ++s) pb[s][0].x += sv[s * EC];
+                c_m0 += sv[NS * EC];
+                if (!HOT)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) v_m0[k] += sv[(NS + 1 + k) * EC];
             }
-            pb[0][0].x += add0;
+            ++at;
+            --left;
         }
         if (code & OP_SPOIL1) spoil_all<RP, K>(pb, mb);
         for (int s = 0; s < op_shift2(code); ++s) shift_adjoint_all<RP, L, K>(pb, mb, q, kill, kill_r);
@@ -957,7 +971,7 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
             asm volatile("cp.async.commit_group;\n" ::: "memory");
             fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
             asm volatile("cp.async.wait_group %0;\n" ::"n"(D - 1) : "memory");
-            __syncwarp();  // the seeds another lane copied
+            __syncwarp();  // the transcendentals another lane wrote
         }
         const Op op = s_ops[o];
         const int cur = use_slot;
