@@ -21,7 +21,7 @@
 // Bound: the FMA pipe, with the sine and cosine of each pulse and voxel next.
 // Measured on 96 CPMG protocols of 4 to 64 echoes, 1.5 million voxels: 2.21 ms
 // with the orders spread over lanes, 0.75 ms with every order of one voxel in
-// a lane's pairs, 0.46 ms here.
+// a lane's pairs, 0.46 ms here with sincosf and 0.43 with turn2().
 #include "tsg_internal.h"
 
 namespace tsg {
@@ -35,6 +35,44 @@ __device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+
+// The sines and cosines of two angles without a branch, for |x| <= 2^20:
+// reduction to |r| <= pi/4 by a three-part pi/2 (W. J. Cody and W. Waite,
+// Software Manual for the Elementary Functions, 1980; with fused products the
+// first difference is exact) and the Taylor series to r^9 and r^10, whose
+// remainders there are 2e-9 and 2e-10. At most 1.5 ulp over that range.
+// kTurnLimit bounds a flip in rad and a B1 factor each; a voxel or echo beyond
+// it, or NaN, calls sincosf.
+constexpr float kTurnLimit = 1024.f;
+
+__device__ __forceinline__ bool turns_wild(float x) { return !(fabsf(x) <= kTurnLimit); }
+
+__device__ __forceinline__ void place_turn(int quadrant, float s, float c, float* si, float* co) {
+    const bool swap = quadrant & 1;
+    const float a = swap ? c : s, b = swap ? s : c;
+    *si = __int_as_float(__float_as_int(a) ^ ((quadrant & 2) << 30));
+    *co = __int_as_float(__float_as_int(b) ^ (((quadrant + 1) & 2) << 30));
+}
+
+__device__ __forceinline__ void turn2(float2 x, float2* si, float2* co) {
+    const float2 shifted = fma2(x, dup(0x1.45f306p-1f), dup(12582912.f));  // 2/pi; 1.5 * 2^23
+    const float2 n = add2(shifted, dup(-12582912.f));
+    float2 r = fma2(n, dup(-0x1.921fb6p+0f), x);
+    r = fma2(n, dup(0x1.777a5cp-25f), r);
+    r = fma2(n, dup(0x1.ee59dap-50f), r);
+    const float2 t = mul2(r, r);
+    float2 s = fma2(t, dup(1.f / 362880.f), dup(-1.f / 5040.f));
+    float2 c = fma2(t, dup(-1.f / 3628800.f), dup(1.f / 40320.f));
+    s = fma2(t, s, dup(1.f / 120.f));
+    c = fma2(t, c, dup(-1.f / 720.f));
+    s = fma2(t, s, dup(-1.f / 6.f));
+    c = fma2(t, c, dup(1.f / 24.f));
+    s = fma2(mul2(t, r), s, r);
+    c = fma2(t, c, dup(-0.5f));
+    c = fma2(t, c, dup(1.f));
+    place_turn(__float_as_int(shifted.x), s.x, c.x, &si->x, &co->x);
+    place_turn(__float_as_int(shifted.y), s.y, c.y, &si->y, &co->y);
+}
 
 // Both voxels' sample `held`, voxel-major.
 __device__ __forceinline__ void rec_store(float* rec, int lane, int held, float2 y) {
@@ -54,8 +92,11 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
     const tsg_batch_sequence sq = seqs[u.sequence];
     const Op* train = ops + sq.op_offset;
     const int echoes = sq.op_count >> 1;
-    for (int e = lane; e < echoes; e += 32) s_flip[e] = train[2 * e + 1].flip;
-    __syncwarp();
+    bool far = false;
+    for (int e = lane; e < echoes; e += 32) {
+        s_flip[e] = train[2 * e + 1].flip;
+        far |= turns_wild(s_flip[e]);
+    }
     // This lane's voxels: lane and lane + 32 of the unit.
     const int voxels = min(u.voxel_count, 64);
     const int64_t first = sq.voxel_offset + u.voxel_begin;
@@ -63,6 +104,9 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
     const int64_t vb = first + (lane + 32 < voxels ? lane + 32 : 0);
     const float dt = train[1].dt;
     const float2 b1 = b1v ? make_float2(b1v[va], b1v[vb]) : dup(1.f);
+    // An angle that turn2() does not take.
+    const bool wild = __any_sync(0xffffffffu, far || turns_wild(b1.x) || turns_wild(b1.y));
+    __syncwarp();
     const float2 m0 = m0v ? make_float2(m0v[va], m0v[vb]) : dup(1.f);
     const float2 f1 = make_float2(expf(__fmul_rn(-(1000.f / t1v[va]), dt)),
                                   expf(__fmul_rn(-(1000.f / t1v[vb]), dt)));
@@ -87,8 +131,11 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
     for (int e = 0; e < echoes; ++e) {
         const float2 angle = mul2(dup(s_flip[e]), b1);
         float2 si, co;
-        sincosf(angle.x, &si.x, &co.x);
-        sincosf(angle.y, &si.y, &co.y);
+        turn2(angle, &si, &co);
+        if (wild) {
+            if (turns_wild(s_flip[e]) || turns_wild(b1.x)) sincosf(angle.x, &si.x, &co.x);
+            if (turns_wild(s_flip[e]) || turns_wild(b1.y)) sincosf(angle.y, &si.y, &co.y);
+        }
         const float2 H = h, nH = make_float2(-h.x, -h.y), hco = mul2(h, co), hsi = mul2(h, si);
         const float2 wsi = mul2(w1, si), nsi = make_float2(-wsi.x, -wsi.y), ce = mul2(w1, co);
         const int top = min(min(e, echoes - 1 - e), slots - 1);  // the last order
