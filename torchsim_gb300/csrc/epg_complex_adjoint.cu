@@ -133,15 +133,27 @@ __device__ __forceinline__ void shift_complex_adjoint(float2 (&pr)[RP], float2 (
     }
 }
 
-// An op's two angles in the frame of the last pulse: how far its own pulse
-// turns that frame (0 without one), and its receiver phase in it. (Nothing is
-// transverse before the first pulse, so the first frame is free.)
-__device__ __forceinline__ float2 frame_angles(const Op* ops, const float2* phase, int i) {
-    const bool pulse = op_rf(ops[i].code) == RF_ROTATE;
-    int j = i - 1;
-    while (j >= 0 && op_rf(ops[j].code) != RF_ROTATE) --j;
-    const float last = j >= 0 ? phase[j].x : pulse ? phase[i].x : 0.f;
-    return make_float2(pulse ? phase[i].x - last : 0.f, phase[i].y - (pulse ? phase[i].x : last));
+// Turns staged phases (pulse, receiver) into every op's two angles in the
+// frame of the last pulse: how far its own pulse turns that frame (0 without
+// one), and its receiver phase in it. (Nothing is transverse before the first
+// pulse, so the first frame is free.) One warp does it, 32 ops at a time;
+// `last` and `any` carry the last pulse's phase, and whether there was one,
+// from chunk to chunk.
+__device__ __forceinline__ void frame_angles(const Op* ops, float2* ph, int count, int lane,
+                                             float& last, bool& any) {
+    for (int base = 0; base < count; base += 32) {
+        const int i = base + lane;
+        const float2 x = i < count ? ph[i] : make_float2(0.f, 0.f);
+        const bool pulse = i < count && op_rf(ops[i].code) == RF_ROTATE;
+        const unsigned set = __ballot_sync(0xffffffffu, pulse);
+        const unsigned below = set & ((1u << lane) - 1u);
+        const float near = __shfl_sync(0xffffffffu, x.x, below ? 31 - __clz(below) : 0);
+        const float before = below ? near : any ? last : pulse ? x.x : 0.f;
+        if (i < count) ph[i] = make_float2(pulse ? x.x - before : 0.f, x.y - (pulse ? x.x : before));
+        const float latest = __shfl_sync(0xffffffffu, x.x, set ? 31 - __clz(set) : 0);
+        if (set) last = latest;
+        any |= set != 0;
+    }
 }
 
 // The transcendentals of one op for one voxel: e1, the F+ factor tr + i ti
@@ -227,14 +239,18 @@ __global__ void __launch_bounds__(128) complex_forward_traj_kernel(const Complex
     const int first_lane = lane - q;
     const bool off_axis = a.b0 != nullptr;
     FrameTrig mine;
+    float frame = 0.f;
+    bool framed = false;
 
     for (int base = 0; base < a.n_ops; base += kComplexOpChunk) {
         const int count = min(kComplexOpChunk, a.n_ops - base);
         __syncthreads();
         for (int i = threadIdx.x; i < count; i += blockDim.x) {
             s_ops[i] = ops[base + i];
-            s_ph[i] = frame_angles(ops, phase, base + i);
+            s_ph[i] = phase[base + i];
         }
+        __syncthreads();
+        if (warp == 0) frame_angles(s_ops, s_ph, count, lane, frame, framed);
         __syncthreads();
         for (int i = 0; i < count; ++i) {
             const Op op = s_ops[i];
@@ -394,8 +410,12 @@ __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
         const float2* ph = a.phase + train * n_ops;
         for (int i = threadIdx.x; i < n_ops; i += T) {
             s_ops[i] = ops[i];
-            s_ph[i] = frame_angles(ops, ph, i);
+            s_ph[i] = ph[i];
         }
+        __syncthreads();
+        float frame = 0.f;
+        bool framed = false;
+        if (warp == 0) frame_angles(s_ops, s_ph, n_ops, lane, frame, framed);
         __syncthreads();
     }
 
