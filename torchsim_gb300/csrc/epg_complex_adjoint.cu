@@ -40,6 +40,8 @@
 //            pulse's own changes of w and W.
 #include "epg_complex.cuh"
 
+#include <type_traits>
+
 namespace tsg {
 
 namespace {
@@ -48,6 +50,7 @@ using namespace complex_detail;
 
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 
+constexpr uint32_t kPlainOp = kFastBits | OP_RECORD;
 constexpr int kCxWarps = 2;
 constexpr int kCxRing = 2;
 
@@ -367,7 +370,8 @@ __device__ __forceinline__ float2 dot_acc(const float2 (&y)[RP], const float2 (&
 // Bound: instruction issue; the trajectory's 5 GB there are 0.75 ms. With the
 // general 3x3 pulse (states outside its frame, derivatives by applying their
 // own matrices), seeds read where they are used and two orders per lane it was
-// 2.13 ms; the frame takes 0.30 off, the seeds 0.26, four orders 0.33.
+// 2.13 ms; the frame takes 0.30 off, the seeds 0.26, four orders 0.33 and the
+// plain ops' own copy of the step 0.09 (1.16 ms).
 template <int RP, int L>
 __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
     complex_adjoint_kernel(const ComplexAdjointArgs a) {
@@ -485,15 +489,16 @@ __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
     };
     read_record(n_ops - 1);
 
-    for (int o = n_ops - 1; o >= 0; --o) {
+    // One op in reverse; of a plain one (relaxation, pulse, sample, shift: most
+    // ops of a fingerprinting train) the steps are known when this is compiled.
+    auto step = [&](auto plain, int o, const Op& op) {
         const float2 seed = next_seed, rec0 = next_x0;
         read_record(o - 1);
         if (o - (D - 1) >= 0) fetch(o - (D - 1), fill_slot);
         asm volatile("cp.async.commit_group;\n" ::: "memory");
         fill_slot = fill_slot + 1 == D ? 0 : fill_slot + 1;
-        const Op op = s_ops[o];
         const float2 ph = s_ph[o];
-        const uint32_t code = op.code;
+        const uint32_t code = decltype(plain)::value ? kPlainOp : op.code;
         const int g = (n_ops - 1 - o) % L;
         const int src = first_lane + g;
         if constexpr (L > 1) {
@@ -684,6 +689,13 @@ __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
         for (int off = 4; off > 0; off >>= 1) f0 += __shfl_xor_sync(0xffffffffu, f0, off);
         if ((lane & 7) == 0)
             reinterpret_cast<float*>(event_out + int64_t(o) * 2)[lane >> 3] = f0;
+    };
+    for (int o = n_ops - 1; o >= 0; --o) {
+        const Op op = s_ops[o];
+        if (op.code == kPlainOp)
+            step(std::true_type{}, o, op);
+        else
+            step(std::false_type{}, o, op);
     }
     asm volatile("cp.async.wait_all;\n" ::: "memory");
     float out[7] = {g_t1, g_t2, g_m0, g_b1, g_inv, g_b1p, g_b0};
