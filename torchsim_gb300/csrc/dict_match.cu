@@ -25,14 +25,14 @@
 // complex atoms (Re s, Im s) and (Im s, -Re s) against (Re d, Im d), whose
 // products are the real and imaginary parts of <s, d>.
 //
-// Bound: the tensor pipe (60% active by ncu at 1.94 GHz, and with the scoring
-// left out no more than 1.45 to 1.6 PFLOP/s). Measured, 16,384 voxels x 65,536
-// atoms x 500 samples: 3.62 ms with one CTA per 128 rows in whole waves, 3.24
-// with row tiles in pairs, the last wave split and resident queries, 3.16 with
-// the pair's two SMs on one product, 2.95 (1.46 PFLOP/s) with the candidates
-// inserted a lane's best at a time; 1,024 voxels 2.0 -> 0.22 ms by the split.
-// The rescoring, bound by reading the candidates' atoms, 367 -> 219 us by
-// reading one part of atoms on an axis and four candidates at a time.
+// Bound: the tensor pipe and its power (1.8 to 1.9 PFLOP/s). Measured, 16,384
+// voxels x 65,536 atoms x 500 samples: 3.62 ms with one CTA per 128 rows in
+// whole waves, 3.24 with row tiles in pairs, the last wave split and resident
+// queries, 3.16 with the pair's two SMs on one product, 2.95 with the
+// candidates inserted a lane's best at a time, 2.43 (1.78 PFLOP/s) with one
+// commit for a contraction tile; 1,024 voxels 2.0 -> 0.22 ms by the split. The
+// rescoring, bound by reading the candidates' atoms, 367 -> 219 us by reading
+// one part of atoms on an axis and four candidates at a time.
 //
 // Waits on mbarriers are bounded: a wait that runs out sets the error word
 // and the kernel winds down instead of hanging.
@@ -61,8 +61,13 @@ constexpr int SMEM_B = BN / 2 * BK * 2;  // a CTA's half
 // is past the 128 the memory has; half the atom tile makes it 64 and 32.
 constexpr int kPair = 2;
 // Shared-memory slots: query tiles resident for a whole sweep over the atoms
-// where the contraction has at most kResident tiles, else a short ring; atom
-// tiles in a ring.
+// where the contraction has at most kResident tiles; atom tiles in a ring, a
+// slot holding all parts of a contraction tile and, where they are not
+// resident, its query tile. One wait and one commit then go with all the
+// products of a contraction tile: each tcgen05.commit holds up the products
+// after it, and with one for every part and query tile the pipe stayed 60%
+// active whatever the ring's depth (65,536 voxels x 262,144 atoms x 880
+// samples 84.1 ms, now 67.2; 16,384 x 65,536 x 500 2.95 and 2.43).
 constexpr int kResident = 8;
 constexpr int kMaxA = 8, kMaxB = 10;
 constexpr int kTileBytes = 224 * 1024;  // of both
@@ -161,6 +166,7 @@ struct ScreenWork {
     int parts;    // atom matrices side by side along the contraction (hi, lo)
     int k_step;   // columns from one part to the next
     int na, nb;   // slots
+    int slot;     // bytes of a ring slot in one CTA
     bool resident;
 };
 
@@ -197,7 +203,7 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
     extern __shared__ uint8_t s_raw[];
     uint8_t* a_tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(s_raw) + 1023) & ~uintptr_t(1023));
     uint8_t* b_tiles = a_tiles + w.na * SMEM_A;
-    ScreenShared* sh = reinterpret_cast<ScreenShared*>(b_tiles + w.nb * SMEM_B);
+    ScreenShared* sh = reinterpret_cast<ScreenShared*>(b_tiles + w.nb * w.slot);
     const int warp = threadIdx.x >> 5;
     const int lane = threadIdx.x & 31;
     const int items = screen_items(w);
@@ -244,17 +250,17 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
             // TMA producer.
             // Both CTAs' bytes of a slot land on the first CTA's barrier,
             // which that CTA arms for the sum.
-            auto fetch = [&](const CUtensorMap& map, uint8_t* slot, uint64_t* bar, int bytes, int x,
-                             int y) {
-                const uint32_t own = smem_u32(bar);
+            auto arm = [&](uint64_t* bar, int bytes) {
                 if (rank == 0)
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(own),
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                                  "r"(kPair * bytes)
                                  : "memory");
+            };
+            auto fetch = [&](const CUtensorMap& map, uint8_t* to, uint64_t* bar, int x, int y) {
                 asm volatile(
                     "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global"
-                    ".mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(slot)),
-                    "l"(reinterpret_cast<uint64_t>(&map)), "r"(x), "r"(y), "r"(first_cta(own))
+                    ".mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(to)),
+                    "l"(reinterpret_cast<uint64_t>(&map)), "r"(x), "r"(y), "r"(first_cta(smem_u32(bar)))
                     : "memory");
             };
             int as = 0, bs = 0;
@@ -262,30 +268,36 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
             for (int i = first_item; i < items && !*abort; i += item_step) {
                 const ScreenItem it = screen_item(w, i);
                 for (int n = it.begin; n < it.end && !*abort; ++n) {
-                    for (int kt = 0; kt < w.k_tiles && !*abort; ++kt) {
-                        if (!w.resident || n == it.begin) {
+                    for (int kt = 0; kt < w.k_tiles; ++kt) {
+                        const int row = (it.row_pair * kPair + rank) * BM;
+                        if (w.resident && n == it.begin) {
                             if (!wait_parity(smem_u32(&sh->a_empty[as]), ap)) {
                                 give_up(1);
                                 break;
                             }
-                            fetch(qmap, a_tiles + as * SMEM_A, &sh->a_full[as], SMEM_A, kt * BK,
-                                  (it.row_pair * kPair + rank) * BM);
+                            arm(&sh->a_full[as], SMEM_A);
+                            fetch(qmap, a_tiles + as * SMEM_A, &sh->a_full[as], kt * BK, row);
                             if (++as == w.na) {
                                 as = 0;
                                 ap ^= 1;
                             }
                         }
-                        for (int part = 0; part < w.parts; ++part) {
-                            if (!wait_parity(smem_u32(&sh->b_empty[bs]), bp)) {
-                                give_up(1);
-                                break;
-                            }
-                            fetch(amap, b_tiles + bs * SMEM_B, &sh->b_full[bs], SMEM_B,
+                        if (!wait_parity(smem_u32(&sh->b_empty[bs]), bp)) {
+                            give_up(1);
+                            break;
+                        }
+                        arm(&sh->b_full[bs], w.slot);
+                        uint8_t* to = b_tiles + bs * w.slot;
+                        if (!w.resident) {
+                            fetch(qmap, to, &sh->b_full[bs], kt * BK, row);
+                            to += SMEM_A;
+                        }
+                        for (int part = 0; part < w.parts; ++part)
+                            fetch(amap, to + part * SMEM_B, &sh->b_full[bs],
                                   part * w.k_step + kt * BK, n * BN + rank * (BN / kPair));
-                            if (++bs == w.nb) {
-                                bs = 0;
-                                bp ^= 1;
-                            }
+                        if (++bs == w.nb) {
+                            bs = 0;
+                            bp ^= 1;
                         }
                     }
                 }
@@ -317,7 +329,7 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
                     "h"(kBoth)
                     : "memory");
             };
-            int as = 0, bs = 0;
+            int bs = 0;
             uint32_t ap = 0, bp = 0;
             int t = 0;  // tiles so far: the accumulator is t & 1
             for (int i = first_item; i < items && !*abort; i += item_step) {
@@ -331,27 +343,24 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint32_t d = tmem + uint32_t(b * BN);
                     uint32_t acc = 0;
-                    for (int kt = 0; kt < w.k_tiles && !*abort; ++kt) {
-                        int slot = kt;
-                        if (!w.resident || n == it.begin) {
-                            if (!wait_parity(smem_u32(&sh->a_full[as]), ap)) {
-                                give_up(3);
-                                break;
-                            }
-                            slot = as;
-                            if (++as == w.na) {
-                                as = 0;
-                                ap ^= 1;
-                            }
+                    for (int kt = 0; kt < w.k_tiles; ++kt) {
+                        if (w.resident && n == it.begin &&
+                            !wait_parity(smem_u32(&sh->a_full[kt]), ap)) {
+                            give_up(3);
+                            break;
                         }
-                        const uint32_t a_addr = smem_u32(a_tiles + slot * SMEM_A);
-                        for (int part = 0; part < w.parts; ++part) {
-                            if (!wait_parity(smem_u32(&sh->b_full[bs]), bp)) {
-                                give_up(3);
-                                break;
-                            }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                            const uint32_t b_addr = smem_u32(b_tiles + bs * SMEM_B);
+                        if (!wait_parity(smem_u32(&sh->b_full[bs]), bp)) {
+                            give_up(3);
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                        uint32_t b_addr = smem_u32(b_tiles + bs * w.slot);
+                        uint32_t a_addr = b_addr;
+                        if (w.resident)
+                            a_addr = smem_u32(a_tiles + kt * SMEM_A);
+                        else
+                            b_addr += SMEM_A;
+                        for (int part = 0; part < w.parts; ++part, b_addr += SMEM_B) {
 #pragma unroll
                             for (int j = 0; j < BK / 16; ++j) {
                                 const uint64_t adesc = tile_desc(a_addr + j * 32);
@@ -363,17 +372,18 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
                                     : "memory");
                                 acc = 1;
                             }
-                            commit(&sh->b_empty[bs]);
-                            if (++bs == w.nb) {
-                                bs = 0;
-                                bp ^= 1;
-                            }
                         }
-                        if (!w.resident || n + 1 == it.end) commit(&sh->a_empty[slot]);
+                        commit(&sh->b_empty[bs]);
+                        if (++bs == w.nb) {
+                            bs = 0;
+                            bp ^= 1;
+                        }
+                        if (w.resident && n + 1 == it.end) commit(&sh->a_empty[kt]);
                     }
                     if (*abort) break;
                     commit(&sh->tfull[b]);
                 }
+                ap ^= 1;
             }
         }
     } else {
@@ -802,8 +812,9 @@ ScreenWork plan_screen(int64_t query_rows, int64_t atom_count, int64_t k, int pa
     w.k_step = int(k);
     w.k_tiles = int((k + BK - 1) / BK);
     w.resident = w.k_tiles <= kResident;
-    w.na = w.resident ? w.k_tiles : 4;
-    w.nb = std::min(kMaxB, (kTileBytes - w.na * SMEM_A) / SMEM_B);
+    w.na = w.resident ? w.k_tiles : 0;
+    w.slot = w.parts * SMEM_B + (w.resident ? 0 : SMEM_A);
+    w.nb = std::min(kMaxB, (kTileBytes - w.na * SMEM_A) / w.slot);
     w.full = may_split ? pairs / slots * slots : pairs;
     w.split = pairs - w.full;
     w.pieces = 1;
@@ -849,7 +860,7 @@ int run_screen(const ScreenWork& w, const void* queries, int64_t query_rows, con
     int rc = tile_map(&qmap, queries, query_rows, k, BM);
     if (!rc) rc = tile_map(&amap, atoms, stored_rows, k * w.parts, BN / kPair);
     if (rc) return rc;
-    const size_t smem = 1024 + w.na * SMEM_A + w.nb * SMEM_B + sizeof(ScreenShared);
+    const size_t smem = 1024 + w.na * SMEM_A + w.nb * w.slot + sizeof(ScreenShared);
     TSG_CUDA(cudaFuncSetAttribute(screen_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int grid = kPair * std::min(std::max(1, sms / kPair), screen_items(w));
     screen_kernel<<<unsigned(grid), kThreads, smem, stream>>>(
