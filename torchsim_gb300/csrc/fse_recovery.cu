@@ -24,53 +24,53 @@ __device__ __forceinline__ float2 cmul(float2 a, float2 b) {
     return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 
-// Smith's division: no overflow of the squared denominator.
-__device__ __forceinline__ float2 cdiv(float2 a, float2 b) {
-    if (fabsf(b.x) >= fabsf(b.y)) {
-        const float r = b.y / b.x, d = b.x + b.y * r;
-        return make_float2((a.x + a.y * r) / d, (a.y - a.x * r) / d);
-    }
-    const float r = b.x / b.y, d = b.x * r + b.y;
-    return make_float2((a.x * r + a.y) / d, (a.y * r - a.x) / d);
+// 1 / a by Smith's division: no overflow of the squared magnitude.
+__device__ __forceinline__ float2 creciprocal(float2 a) {
+    const bool wide = fabsf(a.x) >= fabsf(a.y);
+    const float r = wide ? a.y / a.x : a.x / a.y;
+    const float d = 1.f / (wide ? a.x + a.y * r : a.x * r + a.y);
+    return wide ? make_float2(d, -r * d) : make_float2(r * d, -d);
 }
 
+// A warp per row, its lanes along the echoes.
 __global__ void __launch_bounds__(256) fse_recovery_kernel(
     const float2* __restrict__ signal, const float2* __restrict__ jac_in, int64_t rows, int echoes,
-    int columns_in, int columns, RecoveryColumns map, const float* __restrict__ t1v, int64_t t1_step,
-    const float* __restrict__ m0v, int64_t m0_step, float m0_value, float left_ms,
+    int columns_in, int columns, RecoveryColumns map, const float* __restrict__ t1v, int t1_step,
+    const float* __restrict__ m0v, int m0_step, float m0_value, float left_ms,
     float2* __restrict__ out, float2* __restrict__ jac_out) {
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= rows * echoes) return;
-    const int64_t row = i / echoes;
-    const int echo = int(i - row * echoes);
+    const int64_t row = int64_t(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (row >= rows) return;
     const float t1 = t1v[row * t1_step];
     const float m0 = m0v ? m0v[row * m0_step] : m0_value;
     const float rec = expf(-1000.f / t1 * left_ms * 1e-3f);
-    const float2 x = signal[i];
-    const float2 s = make_float2(x.y, -x.x);
-    const float2 denom = make_float2(1.f - rec * s.x, -rec * s.y);
     const float gone = 1.f - rec;
-    const float2 over_m0 = make_float2(s.x * gone, s.y * gone);
-    out[i] = cdiv(make_float2(m0 * over_m0.x, m0 * over_m0.y), denom);
-    if (columns == 0) return;
-    const float2 square = cmul(denom, denom);
-    const float2 slope = cdiv(make_float2(m0 * gone, 0.f), square);
-    for (int c = 0; c < columns; ++c) {
-        float2 y;
-        if (map.source[c] < 0) {
-            y = cdiv(over_m0, denom);
-        } else {
-            const float2 d = jac_in[(row * columns_in + map.source[c]) * echoes + echo];
-            y = cmul(slope, make_float2(d.y, -d.x));
-            if (c == map.t1) {
-                const float2 ms = cmul(make_float2(m0 * s.x, m0 * s.y), make_float2(s.x - 1.f, s.y));
-                const float2 g = cdiv(ms, square);
-                const float k = rec * left_ms / (t1 * t1);
-                y.x += g.x * k;
-                y.y += g.y * k;
+    const float k = rec * left_ms / (t1 * t1);
+    const float2* x_row = signal + row * echoes;
+    const float2* in = jac_in + row * columns_in * echoes;
+    float2* y_row = out + row * echoes;
+    float2* to = jac_out + row * columns * echoes;
+    for (int e = threadIdx.x & 31; e < echoes; e += 32) {
+        const float2 x = x_row[e];
+        const float2 s = make_float2(x.y, -x.x);
+        const float2 inverse = creciprocal(make_float2(1.f - rec * s.x, -rec * s.y));
+        const float2 over_m0 = cmul(make_float2(s.x * gone, s.y * gone), inverse);
+        y_row[e] = make_float2(m0 * over_m0.x, m0 * over_m0.y);
+        if (columns == 0) continue;
+        const float2 slope = cmul(make_float2(m0 * gone * inverse.x, m0 * gone * inverse.y), inverse);
+        for (int c = 0; c < columns; ++c) {
+            float2 y = over_m0;
+            if (map.source[c] >= 0) {
+                const float2 d = in[int64_t(map.source[c]) * echoes + e];
+                y = cmul(slope, make_float2(d.y, -d.x));
+                if (c == map.t1) {
+                    const float2 a = cmul(make_float2(m0 * s.x, m0 * s.y), inverse);
+                    const float2 g = cmul(cmul(a, make_float2(s.x - 1.f, s.y)), inverse);
+                    y.x += g.x * k;
+                    y.y += g.y * k;
+                }
             }
+            to[int64_t(c) * echoes + e] = y;
         }
-        jac_out[(row * columns + c) * echoes + echo] = y;
     }
 }
 
@@ -99,7 +99,7 @@ extern "C" int tsg_fse_recovery(const void* signal, const void* jacobian, int64_
         if (sources[c] >= columns_in || (sources[c] >= 0 && !jacobian))
             return fail(TSG_ERR_ARGUMENT, "column out of range");
     }
-    const int64_t blocks = (rows * echoes + 255) / 256;
+    const int64_t blocks = (rows + 7) / 8;
     if (echoes > 0x7fffffffLL || blocks > 0x7fffffffLL)
         return fail(TSG_ERR_CAPACITY, "launch too large");
     fse_recovery_kernel<<<unsigned(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
