@@ -392,7 +392,7 @@ int tsg_epg_adjoint_complex(const tsg_program* program, const tsg_tissue* tissue
 /* ---- second order: the adjoint of the tangent sweep --------------------- */
 
 /* Sizes for the second-order sweeps along direction_count (1-3) directions:
- * the trajectory (every op's entry state of the signal state and of each
+ * the trajectory (every even op's entry state of the signal state and each
  * tangent, and every recorded F+[0]) and the workspace the caller allocates.
  * event_directions: whether any direction has duration or flip tangents. */
 int tsg_epg_second_plan(const tsg_program* program, int64_t atom_count, int64_t state_count,

@@ -18,10 +18,13 @@
 // directions (J^T g_k, the reference's "value" side) and with respect to the
 // inputs (its "curvature" side, plus J^T g0) follow per micro-step:
 //
-//   rotation by a = flip*b1, a'_k = dflip_k*b1 + flip*db1_k, with the pre-RF
-//   state x, t_k and the post-RF cotangents lam, mu_k:
-//     G_k = mu_k . R'x            (dL/da'_k)
-//     dL/da = lam . R'x + sum_k (mu_k . R't_k + a'_k mu_k . R''x)
+//   rotation R by a = flip*b1, a'_k = dflip_k*b1 + flip*db1_k; R commutes
+//   with its generator K (R' = K R = R K), so with the pre-RF state x, t_k and
+//   the cotangents taken back through the pulse, mu_k = R^T mu_k and lam =
+//   R^T lam + sum_k a'_k K^T mu_k:
+//     G_k = mu_k . K x            (dL/da'_k)
+//     dL/da = lam . K x + sum_k mu_k . K t_k
+//   in w = F+ - F- and Z (F+ + F- stays): K x = (-2 Z, w / 2).
 //   relaxation E = exp(-r dt), eps_k = E'_k / E = -(r'_k dt + r ddt_k),
 //   with the pre-RF states and cotangents (a shift between relaxation and
 //   pulse leaves the inner products unchanged):
@@ -36,14 +39,19 @@
 // lanes' order pairs are 32 * RP consecutive float2, so every store and every
 // load is a whole, aligned line) and every recorded F+[0]; the reverse
 // streams them back through a cp.async ring and runs the even op forward once
-// for the entry state of the odd op after it. Measured at 16,384 voxels x 601
-// ops x 20 orders, T1, T2 and B1: with every op stored the forward spent its
-// time on 10.2 GB of stores (2.21 ms; 1.59 ms with half of them, and the
-// transcendentals shared by a voxel's lanes), while the reverse, which is
-// bound by instruction issue, pays 0.26 ms for the re-run (2.12 to 2.37 ms). Per-event partials are summed over the warp
-// with a fixed butterfly of shuffles after each op; tissue gradients are
-// summed over a voxel's lanes with shuffles. No atomics: results are
+// for the entry state of the odd op after it. Per-event partials are summed
+// over the warp with shuffles in a fixed order after each op; tissue gradients
+// are summed over a voxel's lanes with shuffles. No atomics: results are
 // deterministic.
+//
+// Bound and measured at 16,384 voxels x 601 ops x 20 orders, T1, T2 and B1: the
+// forward by its stores (5.2 GB of trajectory, 0.89 ms; with every op stored
+// and samples stored op by op 2.21 ms), the reverse by instruction issue and
+// latency at 16 warps an SM (1.77 ms). The re-run of the even ops costs the
+// reverse about 0.25 ms and saves the forward about 0.6; the pulses' (u, w)
+// form and the plain ops' own copy of the step take 0.45 off the reverse, the
+// records read as rows 0.17. Held to nine or ten blocks an SM it spills (2.2
+// ms), and four orders per lane take too many registers (2.1 ms).
 #pragma once
 #include "epg_adjoint.cuh"
 #include <type_traits>
