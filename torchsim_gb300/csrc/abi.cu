@@ -132,8 +132,13 @@ const SweepEntry* choose(int mode, int states, int64_t work_items, const tsg_lau
 //   T1, T2  10 states:  2,048 (10,2) 88 / (5,2) 92; 32,768 (5,2) 375 / (1,10) 352
 //   T1, T2  32 states: 32,768 (8,4) 664 / (4,8) 627, at 27 states 709 / 756
 //   T1, T2, B1  20 states: 8,192 (10,2) 212 / (5,4) 229; 24,576 534 / 485
-//   Gauss-Newton 10 states, 880 pulses: 4,096 (5,2) 158 / (1,10) 300;
-//                      16,384 (5,2) 378 / (1,10) 344
+//   Gauss-Newton 10 states, 880 pulses: 4,096 (5,2) 158 / (1,10) 300; 14,592
+//                      (5,2) 282 / (1,10) 343; 15,360 384 / 345; 19,456 424 /
+//                      346; 19,584 424 / 490; 24,320 475 / 499; 26,624 538 / 494
+// The last goes in steps: 19,456 voxels are one warp of (1,10) for each of 608
+// schedulers, and one more warp there starts a second round, while the warps of
+// (5,2) hold 6 voxels each and fill up 14,592 voxels at a time, four to a
+// scheduler.
 struct TrainRule {
     int mode, states, lanes, orders;
     int64_t below;  // voxels x trains
@@ -170,7 +175,8 @@ const TrainRule kTrainRules[] = {
     {MODE_T12BI, 32, 16, 2, 4096},     {MODE_T12BI, 32, 8, 4, kAny},
     {MODE_T12BI, 40, 10, 4, kAny},     {MODE_T12BI, 64, 16, 4, kAny},
     {MODE_T12BI, 128, 32, 4, kAny},
-    {MODE_GN, 10, 5, 2, 12288},        {MODE_GN, 10, 1, 10, kAny},
+    {MODE_GN, 10, 5, 2, 14593},        {MODE_GN, 10, 1, 10, 19457},
+    {MODE_GN, 10, 5, 2, 24321},        {MODE_GN, 10, 1, 10, kAny},
     {MODE_GN, 16, 10, 2, 3072},        {MODE_GN, 16, 4, 4, kAny},
     {MODE_GN, 20, 10, 2, 8192},        {MODE_GN, 20, 2, 10, kAny},
     {MODE_GN, 32, 16, 2, 2048},        {MODE_GN, 32, 8, 4, kAny},
