@@ -276,6 +276,7 @@ __global__ void __launch_bounds__(kTotalThreads)
             s_part[1][threadIdx.x] += s_part[1][threadIdx.x + half];
         }
     }
+    __syncthreads();  // thread 1 writes the total that thread 0 summed
     if (threadIdx.x < 2) out[2 * blockIdx.x + threadIdx.x] = s_part[threadIdx.x][0];
 }
 
