@@ -36,6 +36,12 @@ class NativeError(RuntimeError):
         self.code = code
 
 
+def readable(tensor):
+    """``tensor`` as a kernel reads it through its pointer: contiguous, with a
+    pending conjugation or negation carried out (a copy only where needed)."""
+    return tensor.resolve_conj().resolve_neg().contiguous()
+
+
 class Tissue(ctypes.Structure):
     _fields_ = [(n, ctypes.c_void_p) for n in ("t1_ms", "t2_ms", "m0", "b1", "inversion")]
 

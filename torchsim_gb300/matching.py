@@ -213,7 +213,7 @@ class DictionaryMatcher:
             raise ValueError("dictionary must have shape (atoms, contrasts)")
         if self.top_k > d.shape[0]:
             raise ValueError("top_k must be between one and the atom count")
-        d = d.to(self.device, torch.complex64)
+        d = _native.readable(d.to(self.device, torch.complex64))
         self.dictionary = d
         self.normalized, norm = _normalized(d)
         self.power = norm.square()
@@ -261,7 +261,7 @@ class DictionaryMatcher:
             p = p[:, None] if p.ndim == 1 else p
             if p.ndim != 2 or p.shape[0] != d.shape[0]:
                 raise ValueError("parameters must have shape (atoms, parameters)")
-            self.parameter_values = p
+            self.parameter_values = _native.readable(p)
         return self
 
     def _prepared(self) -> _native.MatchDictionary:
@@ -301,7 +301,7 @@ class DictionaryMatcher:
             params = torch.empty((n, k, prepared.columns), dtype=torch.float32, device=self.device)
         for begin in range(0, n, self.query_chunk_size):
             rows = slice(begin, min(begin + self.query_chunk_size, n))
-            chunk = flat[rows].contiguous()
+            chunk = _native.readable(flat[rows])
             V = chunk.shape[0]
             s_hat, norms = _normalized(chunk)
             s_hat = s_hat.contiguous()
