@@ -462,9 +462,9 @@ def _stream_in_one_kernel(flip_deg: Any, TR_ms: Any, device: torch.device):
         if (tr.dtype != torch.float32 or tr.device != device or tr.numel() not in (1, flip.numel())
                 or tr.ndim > 1):
             return None
-        return flip.contiguous(), tr.contiguous(), 0.0
+        return _native.readable(flip), _native.readable(tr), 0.0
     if isinstance(TR_ms, (int, float)):
-        return flip.contiguous(), None, float(TR_ms)
+        return _native.readable(flip), None, float(TR_ms)
     return None
 
 
@@ -491,8 +491,8 @@ class MrfStream(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, flip, tr, tr_value, ti, template):
-        got = _mrf_stream_kernel(template, flip.detach().contiguous(),
-                                 None if tr is None else tr.detach().contiguous(), tr_value, ti)
+        got = _mrf_stream_kernel(template, _native.readable(flip.detach()),
+                                 None if tr is None else _native.readable(tr.detach()), tr_value, ti)
         ctx.mark_non_differentiable(got[2])
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(flip)
@@ -559,9 +559,9 @@ def _stream_transpose(flip: torch.Tensor, g_flip_ev: torch.Tensor | None,
         return g_flip, g_tr
     if g_flip_ev is None and g_dur_ev is None:
         return None, None
-    ev = [None if g is None else g.to(torch.float32).contiguous() for g in (g_flip_ev, g_dur_ev)]
+    ev = [None if g is None else _native.readable(g.to(torch.float32)) for g in (g_flip_ev, g_dur_ev)]
     out = [None if g is None else torch.empty(n, dtype=torch.float32, device=flip.device) for g in ev]
-    at = flip.detach().contiguous()
+    at = _native.readable(flip.detach())
     _native.check(_native.library().tsg_mrf_stream_vjp(
         at.data_ptr(), n, *[None if t is None else t.data_ptr() for t in (*ev, *out)],
         torch.cuda.current_stream(flip.device).cuda_stream))

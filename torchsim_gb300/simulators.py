@@ -25,7 +25,7 @@ import numpy as np
 import torch
 from torch.autograd import forward_ad
 
-from . import engine
+from . import _native, engine
 from .sequence import (POST_SHIFT, PRE_SHIFT, SHIFT_AFTER, MrfEvents, PackedEvents, fse_events,
                        mrf_events, mrf_gradient_map, mrf_stream_on_device, mrf_stream_with_gradients,
                        played_flip_torch, program_for)
@@ -627,7 +627,8 @@ class FSESimulator(_EpgSimulator):
         t1_column = names.index("T1") if "T1" in names else -1
         return engine.fse_recovery(signal, jacobian,
                                    [-1 if n == "M0" else kernel.index(n) for n in names], t1_column,
-                                   t1.contiguous(), m0.contiguous() if isinstance(m0, torch.Tensor)
+                                   _native.readable(t1),
+                                   _native.readable(m0) if isinstance(m0, torch.Tensor)
                                    else float(m0), left_ms)
 
 
