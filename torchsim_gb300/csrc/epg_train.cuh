@@ -1,6 +1,6 @@
 // The sweep of a plain recorded train: after at most one leading inversion
-// every op is relax, rotate, record, one shift (an MRF repetition), and op i
-// records sample i. Every event stream of the MRF builder with one playing
+// every op is relax, rotate, record, one shift (an MRF repetition; the first may
+// have nothing to relax), and op i records sample i. Every event stream of the MRF builder with one playing
 // compiles to this; other programs run epg_sweep.cuh.
 //
 // Thread mapping and state layout are the general sweep's (one voxel's orders
@@ -157,25 +157,34 @@ __global__ void __launch_bounds__(128, MINB) epg_train_kernel(const SweepArgs a)
         yrow = a.measured + mrow * a.outputs;
     }
 
-    // The coefficients of one op for this lane's voxel, as scalars.
+    // The coefficients of one op for this lane's voxel, as scalars. `still`: an
+    // op that does not wait (a train's first, find_train) leaves the state alone
+    // whatever the relaxation times; the product of its interval with the rate
+    // of a time of zero would be NaN.
     struct Raw {
         float h, hco, nsi, hsi, ce, nb, zb, g1, g2, at;
     };
-    auto evaluate = [&](const float2 op) {
+    auto evaluate = [&](const float2 op, bool still) {
+        const float n1 = still ? 0.f : nr1, n2 = still ? 0.f : nr2;
+        const float d1 = still ? 0.f : w1, d2 = still ? 0.f : w2;
         float si, co;
         sincosf(__fmul_rn(op.y, b1), &si, &co);
-        const float e1 = expf(__fmul_rn(nr1, op.x)), e2 = expf(__fmul_rn(nr2, op.x));
+        const float e1 = expf(__fmul_rn(n1, op.x)), e2 = expf(__fmul_rn(n2, op.x));
         const float h = 0.5f * e2, rec = 1.f - e1;
         return Raw{h, __fmul_rn(h, co), -__fmul_rn(e1, si), __fmul_rn(h, si), __fmul_rn(e1, co),
-                   -__fmul_rn(si, rec), __fmul_rn(co, rec), __fmul_rn(op.x, w1),
-                   __fmul_rn(op.x, w2), op.y};
+                   -__fmul_rn(si, rec), __fmul_rn(co, rec), __fmul_rn(op.x, d1),
+                   __fmul_rn(op.x, d2), op.y};
     };
     // Lane q takes op base + q of a group and leaves its coefficients in
-    // buffer `buf`.
-    auto prepare = [&](int base, int count, int buf) {
+    // buffer `buf`. `start`: op 0 of the group is the train's first. Without a
+    // B1 column the look at the first op alone costs nothing, at every op 1 to
+    // 2% (100,000 voxels x 500 x 32: 703 and 711 us); with one the compiler's
+    // schedule makes it the other way round (100,000 x 500 x 20: every op 1,786
+    // us, the first 1,847, none 1,781).
+    auto prepare = [&](int base, int count, int buf, bool start) {
         const int j = base + q;
         if (holds && q < G && j < count) {
-            const Raw c = evaluate(s_ops[j]);
+            const Raw c = evaluate(s_ops[j], (S::B1 || (start && q == 0)) && s_ops[j].x == 0.f);
             float4* dst = s_coef + ((buf * G + q) * VPW + slot) * Q;
             dst[0] = make_float4(c.h, c.h, c.hco, c.hco);
             dst[1] = make_float4(c.nsi, c.nsi, c.hsi, c.hsi);
@@ -424,11 +433,11 @@ __global__ void __launch_bounds__(128, MINB) epg_train_kernel(const SweepArgs a)
                 return TrainCoef{dup(r.h), dup(-r.h), dup(r.hco), dup(r.nsi), dup(r.hsi), dup(r.ce), r.nb, r.zb,
                                  dup(r.g1), dup(r.g2),  dup(r.at),  dup(-r.at)};
             };
-            Raw next = evaluate(s_ops[0]);
+            Raw next = evaluate(s_ops[0], base == 0 && s_ops[0].x == 0.f);
 #pragma unroll 1
             for (int i = 0; i < count; ++i) {
                 const Raw now = next;
-                next = evaluate(s_ops[min(i + 1, count - 1)]);
+                next = evaluate(s_ops[min(i + 1, count - 1)], false);
                 step(widen(now), held);
                 if (++held == KB || i + 1 == count) {
                     __syncwarp();
@@ -438,12 +447,12 @@ __global__ void __launch_bounds__(128, MINB) epg_train_kernel(const SweepArgs a)
                 }
             }
         } else {
-            prepare(0, count, 0);
+            prepare(0, count, 0, base == 0);
             __syncwarp();
             int buf = 0;
 #pragma unroll 1
             for (int i = 0; i < count; i += G, buf ^= 1) {
-                if (i + G < count) prepare(i + G, count, buf ^ 1);
+                if (i + G < count) prepare(i + G, count, buf ^ 1, false);
                 const int here = min(G, count - i);
                 if (here == G) {
                     TrainCoef c = load(buf, 0);

@@ -115,8 +115,9 @@ int find_train(const HostProgram& program) {
         const Op* ops = program.op.data() + t * program.ops;
         if (first && ops[0].code != uint32_t(RF_INVERT) << OP_RF_SHIFT) return -1;
         for (int64_t i = first; i < program.ops; ++i) {
-            // An op without a relaxation is one of zero duration.
-            if ((ops[i].code | OP_RELAX) != (kFastBits | OP_RECORD)) return -1;
+            // An op without a relaxation is one of zero duration: the first
+            // may be one.
+            if ((ops[i].code | (i == first ? OP_RELAX : 0)) != (kFastBits | OP_RECORD)) return -1;
             if (ops[i].record != i - first) return -1;
         }
     }
