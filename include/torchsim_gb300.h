@@ -361,7 +361,8 @@ int tsg_epg_tangent_complex(const tsg_program* program, const tsg_tissue* tissue
 /* ---- the complex path's first-order adjoint ----------------------------- */
 
 /* Sizes of the complex adjoint's trajectory (every op's entry state: six
- * real planes; and every recorded F+[0]) and workspace. */
+ * real planes; and every recorded F+[0]) and workspace. The trajectory is
+ * 8-byte aligned; one at a 16-byte address is read in wider pieces. */
 int tsg_epg_complex_adjoint_plan(const tsg_program* program, int64_t atom_count,
                                  int64_t state_count, const tsg_launch* launch,
                                  int64_t* trajectory_bytes, int64_t* workspace_bytes);

@@ -372,7 +372,10 @@ __device__ __forceinline__ float2 dot_acc(const float2 (&y)[RP], const float2 (&
 // own matrices), seeds read where they are used and two orders per lane it was
 // 2.13 ms; the frame takes 0.30 off, the seeds 0.26, four orders 0.33 and the
 // plain ops' own copy of the step 0.09 (1.16 ms).
-template <int RP, int L>
+//
+// WIDE: a lane's two pairs are copied as one 16-byte piece, for which the
+// trajectory has to be 16-byte aligned; else pair by pair.
+template <int RP, int L, bool WIDE>
 __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
     complex_adjoint_kernel(const ComplexAdjointArgs a) {
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -437,7 +440,7 @@ __global__ void __launch_bounds__(32 * kCxWarps, RP == 1 ? 10 : 1)
         const unsigned dst = ring_base + unsigned(rs * 6 * T * RP) * 8u;
 #pragma unroll
         for (int p = 0; p < 6; ++p) {
-            if constexpr (RP == 2) {
+            if constexpr (WIDE) {
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(
                                  dst + unsigned(p * T * RP) * 8u),
                              "l"(src + p * plane)
@@ -780,22 +783,25 @@ struct CxEntry {
     int orders_per_lane;
     int lanes_per_voxel;
     void (*forward)(const ComplexAdjointArgs&, dim3, dim3, cudaStream_t);
-    void (*reverse)(const ComplexAdjointArgs&, dim3, dim3, size_t, cudaStream_t);
-    const void* reverse_fn;
+    // The reverse for trajectories of any (8-byte) alignment and of 16 bytes.
+    void (*reverse[2])(const ComplexAdjointArgs&, dim3, dim3, size_t, cudaStream_t);
+    const void* reverse_fn[2];
 };
 
 template <int RP, int L>
 void launch_cx_forward(const ComplexAdjointArgs& a, dim3 g, dim3 b, cudaStream_t s) {
     complex_forward_traj_kernel<RP, L><<<g, b, 0, s>>>(a);
 }
-template <int RP, int L>
+template <int RP, int L, bool WIDE>
 void launch_cx_reverse(const ComplexAdjointArgs& a, dim3 g, dim3 b, size_t smem, cudaStream_t s) {
-    complex_adjoint_kernel<RP, L><<<g, b, smem, s>>>(a);
+    complex_adjoint_kernel<RP, L, WIDE><<<g, b, smem, s>>>(a);
 }
 
-#define TSG_CX_ENTRY(R, L)                                                           \
-    {R, L, &launch_cx_forward<(R) / 2, L>, &launch_cx_reverse<(R) / 2, L>,           \
-     reinterpret_cast<const void*>(&complex_adjoint_kernel<(R) / 2, L>)}
+#define TSG_CX_ENTRY(R, L)                                                                       \
+    {R, L, &launch_cx_forward<(R) / 2, L>,                                                       \
+     {&launch_cx_reverse<(R) / 2, L, false>, &launch_cx_reverse<(R) / 2, L, (R) == 4>},          \
+     {reinterpret_cast<const void*>(&complex_adjoint_kernel<(R) / 2, L, false>),                 \
+      reinterpret_cast<const void*>(&complex_adjoint_kernel<(R) / 2, L, (R) == 4>)}}
 
 const CxEntry kCx[] = {
     TSG_CX_ENTRY(2, 2),  TSG_CX_ENTRY(2, 4),  TSG_CX_ENTRY(2, 5),  TSG_CX_ENTRY(2, 8),
@@ -975,10 +981,11 @@ extern "C" int tsg_epg_adjoint_complex(const tsg_program* program, const tsg_tis
     a.event_partial = reinterpret_cast<float2*>(ws);
     a.tissue_partial = reinterpret_cast<float*>(ws + plan.event_bytes);
     a.warps_per_train = plan.warps_per_train;
+    const int wide = (reinterpret_cast<uintptr_t>(trajectory) & 15) == 0;
     if (plan.smem > 48 * 1024)
-        TSG_CUDA(cudaFuncSetAttribute(plan.reverse->reverse_fn,
+        TSG_CUDA(cudaFuncSetAttribute(plan.reverse->reverse_fn[wide],
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, int(plan.smem)));
-    plan.reverse->reverse(a, dim3(unsigned(plan.blocks), unsigned(program->host.trains)),
+    plan.reverse->reverse[wide](a, dim3(unsigned(plan.blocks), unsigned(program->host.trains)),
                         dim3(32 * kCxWarps), plan.smem, s);
     TSG_CUDA(cudaGetLastError());
     const int64_t ops = program->host.ops;
