@@ -483,6 +483,14 @@ def _mrf_stream_kernel(template: Program, flip: torch.Tensor, tr: torch.Tensor |
     return both[0], both[1], ops
 
 
+def _unmoved(ctx, flip_ev: torch.Tensor, dur_ev: torch.Tensor) -> list[torch.Tensor]:
+    """The event buffers that carry no gradient: of flips where the flips
+    (input 0) are not differentiated, of durations where the TRs (input 1) are
+    not. Left differentiable, each costs the sweep behind it a gradient that
+    nothing takes."""
+    return [ev for ev, moved in zip((flip_ev, dur_ev), ctx.needs_input_grad) if not moved]
+
+
 class MrfStream(torch.autograd.Function):
     """The device-built MRF stream as a function of the flips (deg) and TRs
     (ms): the packed flip and duration buffers, and (not differentiable) the
@@ -493,7 +501,7 @@ class MrfStream(torch.autograd.Function):
     def forward(ctx, flip, tr, tr_value, ti, template):
         got = _mrf_stream_kernel(template, _native.readable(flip.detach()),
                                  None if tr is None else _native.readable(tr.detach()), tr_value, ti)
-        ctx.mark_non_differentiable(got[2])
+        ctx.mark_non_differentiable(got[2], *_unmoved(ctx, got[0], got[1]))
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(flip)
         ctx.tr_shape = None if tr is None else tr.shape
@@ -517,7 +525,9 @@ class MrfEvents(torch.autograd.Function):
         ctx.set_materialize_grads(False)
         ctx.save_for_backward(flip)
         ctx.tr = None if tr is None else (tr.shape, tr.device, tr.dtype)
-        return flip_ev.clone(), dur_ev.clone()
+        got = flip_ev.clone(), dur_ev.clone()
+        ctx.mark_non_differentiable(*_unmoved(ctx, *got))
+        return got
 
     @staticmethod
     def backward(ctx, g_flip_ev, g_dur_ev):
