@@ -601,6 +601,13 @@ int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* state, const fl
                  int64_t voxel_count, int64_t state_count, const void* measured,
                  const tsg_gn_config* config, int32_t* lists, int32_t* counts, double* totals,
                  const tsg_launch* launch, void* stream);
+/* Iterations `first` to `first + iterations - 1` of such a solve, with the
+ * buffers of the whole: a caller that looks at counts in between leaves the
+ * iterations that are no longer needed unqueued. */
+int tsg_gn_solve_part(const tsg_program* program, const tsg_gn_state* state, const float* b1,
+                      int64_t voxel_count, int64_t state_count, const void* measured,
+                      const tsg_gn_config* config, int first, int iterations, int32_t* lists,
+                      int32_t* counts, double* totals, const tsg_launch* launch, void* stream);
 int tsg_gn_total_parts(void);
 /* Natural parameters (voxel_count x 3 floats) of free variables. */
 int tsg_gn_natural(const double* free_variables, int64_t voxel_count, const tsg_gn_config* config,

@@ -172,6 +172,9 @@ SIGNATURES: dict[str, tuple] = {
     "tsg_gn_judge": (_int, [ctypes.POINTER(GNState), _i64, ctypes.POINTER(GNConfig), _vp]),
     "tsg_gn_solve": (_int, [_vp, ctypes.POINTER(GNState), _vp, _i64, _i64, _vp,
                             ctypes.POINTER(GNConfig), _vp, _vp, _vp, ctypes.POINTER(Launch), _vp]),
+    "tsg_gn_solve_part": (_int, [_vp, ctypes.POINTER(GNState), _vp, _i64, _i64, _vp,
+                                 ctypes.POINTER(GNConfig), _int, _int, _vp, _vp, _vp,
+                                 ctypes.POINTER(Launch), _vp]),
     "tsg_gn_total_parts": (_int, []),
     "tsg_gn_natural": (_int, [_vp, _i64, ctypes.POINTER(GNConfig), _vp, _vp]),
     "tsg_match_screen": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),

@@ -332,28 +332,31 @@ extern "C" int tsg_gn_natural(const double* free_variables, int64_t voxel_count,
     return TSG_OK;
 }
 
-// A whole solve queued on the stream: per iteration the step, the evaluation,
-// the judgement with the next voxel list, and the sums. Nothing is read back,
-// so the launches of all iterations are queued at once (a copy of the pool's
-// rows per iteration and one wait each took as long as the sweeps); the grids
-// cover every voxel and blocks past the live ones end at once.
-extern "C" int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* state,
-                            const float* b1, int64_t voxel_count, int64_t state_count,
-                            const void* measured, const tsg_gn_config* config, int32_t* lists,
-                            int32_t* counts, double* totals, const tsg_launch* launch_shape,
-                            void* stream) {
+// A run of a solve's iterations queued on the stream: per iteration the step,
+// the evaluation, the judgement with the next voxel list, and the sums. Nothing
+// is read back, so the launches of all its iterations are queued at once (a copy
+// of the pool's rows per iteration and one wait each took as long as the
+// sweeps); the grids cover every voxel and blocks past the live ones end at
+// once.
+extern "C" int tsg_gn_solve_part(const tsg_program* program, const tsg_gn_state* state,
+                                 const float* b1, int64_t voxel_count, int64_t state_count,
+                                 const void* measured, const tsg_gn_config* config, int first,
+                                 int iterations, int32_t* lists, int32_t* counts, double* totals,
+                                 const tsg_launch* launch_shape, void* stream) {
     if (voxel_count < 0 || !config || (voxel_count > 0 && !valid(state)))
         return fail(TSG_ERR_ARGUMENT, "invalid Gauss-Newton state");
     if (config->max_iterations < 1) return fail(TSG_ERR_ARGUMENT, "max_iterations must be positive");
+    if (first < 0 || iterations < 0 || first > config->max_iterations ||
+        iterations > config->max_iterations + 1 - first)
+        return fail(TSG_ERR_ARGUMENT, "a solve has iterations 0 to max_iterations");
     if (voxel_count > 0x7fffffffLL) return fail(TSG_ERR_CAPACITY, "too many voxels for one solve");
     if (voxel_count == 0) return TSG_OK;
     if (!lists || !counts || !totals) return fail(TSG_ERR_ARGUMENT, "null solve buffer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const unsigned blocks = unsigned((voxel_count + kSolveThreads - 1) / kSolveThreads);
-    const int iterations = config->max_iterations + 1;
-    TSG_CUDA(cudaMemsetAsync(counts, 0, sizeof(int32_t) * iterations, s));
+    TSG_CUDA(cudaMemsetAsync(counts + first, 0, sizeof(int32_t) * iterations, s));
     const tsg_tissue tissue{state->t1, state->t2, state->m0, b1, nullptr};
-    for (int it = 0; it < iterations; ++it) {
+    for (int it = first; it < first + iterations; ++it) {
         VoxelList list{nullptr, nullptr};
         if (it > 0) list = {lists + (it & 1) * voxel_count, counts + it - 1};
         gn_step_kernel<<<blocks, kSolveThreads, 0, s>>>(*state, voxel_count, *config, list);
@@ -369,6 +372,16 @@ extern "C" int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* stat
         TSG_CUDA(cudaGetLastError());
     }
     return TSG_OK;
+}
+
+extern "C" int tsg_gn_solve(const tsg_program* program, const tsg_gn_state* state,
+                            const float* b1, int64_t voxel_count, int64_t state_count,
+                            const void* measured, const tsg_gn_config* config, int32_t* lists,
+                            int32_t* counts, double* totals, const tsg_launch* launch_shape,
+                            void* stream) {
+    return tsg_gn_solve_part(program, state, b1, voxel_count, state_count, measured, config, 0,
+                             config ? config->max_iterations + 1 : 0, lists, counts, totals,
+                             launch_shape, stream);
 }
 
 extern "C" int tsg_gn_total_parts(void) { return kTotalBlocks; }

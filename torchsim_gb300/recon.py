@@ -582,6 +582,11 @@ class ModelOperator(torch.nn.Module):
 
 # ---- the loop -----------------------------------------------------------------
 
+# Iterations of a fused solve queued between two looks at how many voxels are
+# left: above the 21 of the mapping estimator's default loop, so that it waits
+# once. An iteration without voxels is four launches, about 10 us.
+QUEUED_ITERATIONS = 32
+
 
 class GaussNewton:
     """Solve for the maps that explain a measurement by repeated
@@ -690,9 +695,10 @@ class GaussNewton:
                     b1: torch.Tensor | None, config: _native.GNConfig, states: int):
         """The fused device loop: (free variables in T1, T2, M0 order, final
         cost, steps and limit flags per voxel, the summed cost and mean
-        damping after every iteration). Every iteration is queued at once
-        (``tsg_gn_solve``); the one wait is for the counts of live voxels at
-        the end."""
+        damping after every iteration). ``QUEUED_ITERATIONS`` are queued at
+        once (``tsg_gn_solve_part``), then the counts of live voxels read: one
+        wait for a solve of few iterations, and one of many ends soon after
+        its last voxel."""
         device = measured.device
         V = measured.shape[0]
         lib = _native.library()
@@ -722,14 +728,17 @@ class GaussNewton:
             *natural)])
         launch = self.launch if self.launch is not None else pool_shape(program, V, states)
         counts = lists[2 * V:]
-        _native.check(lib.tsg_gn_solve(
-            program.handle, ctypes.byref(state), None if b1 is None else b1.data_ptr(), V, states,
-            measured.data_ptr(), ctypes.byref(config), lists.data_ptr(), counts.data_ptr(),
-            totals.data_ptr(), _native.launch_shape(launch),
-            torch.cuda.current_stream(device).cuda_stream))
-        live = counts.cpu()
-        over = torch.nonzero(live == 0)
-        rounds = int(over[0]) + 1 if over.numel() else rounds
+        for first in range(0, rounds, QUEUED_ITERATIONS):
+            run = min(QUEUED_ITERATIONS, rounds - first)
+            _native.check(lib.tsg_gn_solve_part(
+                program.handle, ctypes.byref(state), None if b1 is None else b1.data_ptr(), V,
+                states, measured.data_ptr(), ctypes.byref(config), first, run, lists.data_ptr(),
+                counts.data_ptr(), totals.data_ptr(), _native.launch_shape(launch),
+                torch.cuda.current_stream(device).cuda_stream))
+            over = torch.nonzero(counts[first:first + run].cpu() == 0)
+            if over.numel():
+                rounds = first + int(over[0]) + 1
+                break
         history, weights = totals[:rounds].sum(1).unbind(-1)
         weights = weights[: rounds - 1] / counts[: rounds - 1]
         return u, cost, steps, flags & 4, history.contiguous(), weights
