@@ -74,14 +74,16 @@ def time_ms(fn: Callable[[], Any], warmup: int = 2, repeats: int = 3) -> float:
 
 def tune(key: str, candidates: Iterable[Any], run: Callable[[Any], Any], *,
          use_cache: bool = True, warmup: int = 2, repeats: int = 3) -> tuple[Any, dict]:
-    """The fastest candidate for ``key`` and the timings measured (ms)."""
+    """The fastest candidate for ``key`` and the timings measured (ms). A
+    cached winner that is not among the candidates is measured anew."""
+    candidates = list(candidates)
     with _lock:
         if use_cache:
-            if key in _memory:
+            if key in _memory and _memory[key] in candidates:
                 return _memory[key], {}
             stored = _load().get(key)
-            if stored is not None:
-                value = tuple(stored) if isinstance(stored, list) else stored
+            value = tuple(stored) if isinstance(stored, list) else stored
+            if value is not None and value in candidates:
                 _memory[key] = value
                 return value, {}
     timings: dict[Any, float] = {}

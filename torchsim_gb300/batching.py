@@ -205,10 +205,18 @@ class SequenceBatch:
         return cands
 
     def tune(self, use_cache: bool = True) -> tuple[tuple[int, int, int], dict]:
-        sig = f"n={len(self.entries)},u={self.updates() // 10**6}M,smax={int(self.states.max())}"
+        """The launch shape for this batch and the timings behind it (ms; none
+        where it was cached). It is the persistent launch's, so the sequences
+        that run there name the workload; a batch without any keeps the first
+        candidate."""
+        rest = ~self.echo
+        if rest.any():
+            u = int((self.voxels * self.outputs * self.states)[rest].sum()) // 10**6
+            sig = f"persistent,n={int(rest.sum())},u={u}M,smax={int(self.states[rest].max())}"
+            candidates = self.candidates()
+        else:
+            sig, candidates = "echo trains", self.candidates()[:1]
         key = autotune.workload_key("batched", workload=sig)
-        # The shape is the persistent launch's: without one any will do.
-        candidates = self.candidates()[:1] if self.echo.all() else self.candidates()
         best, timings = autotune.tune(key, candidates, self.launch, use_cache=use_cache, warmup=1,
                                       repeats=2)
         self.shape = tuple(best)
