@@ -512,7 +512,7 @@ def adjoint_section(torch, device, repeats: int = 5) -> dict:
     # launch shapes and segment lengths.
     fwd_shape, _ = autotune.tune(
         autotune.workload_key("adjoint-forward", states=S, ops=prog.ops, voxels=V),
-        autotune.sweep_shapes(S, engine.FAMILY_SHAPES[0]),
+        autotune.sweep_shapes(S, engine.shapes_for(prog, 0)),
         lambda shape: engine.forward(prog, tissue, S, out=sig, launch=shape), use_cache=False)
     buffers = {}
 

@@ -194,6 +194,10 @@ int tsg_program_plan(const float* duration_s, const int32_t* kind, const float* 
 /* op_count: ops per train; output_count: recorded samples per train. */
 int tsg_program_info(const tsg_program* program, int64_t* train_count, int64_t* op_count,
                      int64_t* output_count, int64_t* event_count);
+/* Whether the program is a plain recorded train (after at most one leading
+ * inversion every op relaxes, rotates, records and shifts once): such programs
+ * take the launch shapes of their own sweep besides the general one's. */
+int tsg_program_recorded_train(const tsg_program* program);
 
 /* Rebinding a compiled program to new event values on the device, with no
  * host round trip (the role of the reference's affine rebinding of packed

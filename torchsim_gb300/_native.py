@@ -124,6 +124,7 @@ SIGNATURES: dict[str, tuple] = {
                                 _i64]),
     "tsg_program_info": (_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64),
                                 ctypes.POINTER(_i64), ctypes.POINTER(_i64)]),
+    "tsg_program_recorded_train": (_int, [_vp]),
     "tsg_program_rebind": (_int, [_vp, _vp, _vp, _vp, _vp]),
     "tsg_program_view": (_int, [_vp, _vp, ctypes.POINTER(_vp)]),
     "tsg_echo_train": (_int, [_vp, _i64]),

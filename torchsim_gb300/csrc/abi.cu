@@ -583,6 +583,10 @@ extern "C" int tsg_program_info(const tsg_program* p, int64_t* trains, int64_t* 
     return TSG_OK;
 }
 
+extern "C" int tsg_program_recorded_train(const tsg_program* p) {
+    return p && p->host.train_first >= 0 ? 1 : 0;
+}
+
 extern "C" int tsg_epg_forward(const tsg_program* program, const tsg_tissue* tissue,
                                int64_t atom_count, int64_t state_count, int layout,
                                float* out_a, float* out_b, const tsg_launch* launch_shape,

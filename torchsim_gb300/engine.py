@@ -438,22 +438,38 @@ def sweep_to_host(program: Program, tissue: TissueMaps, states: int, names: Sequ
 
 
 # (lanes per voxel, orders per lane) instantiated per kernel family, as in the
-# sweep tables of csrc/sweep_*.cu and csrc/train_*.cu (a shape of one table
-# only runs the programs of that table).
+# sweep tables of csrc/sweep_*.cu, which run any program.
 FAMILY_SHAPES = {
     0: [(1, 10), (1, 20), (5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (4, 8), (8, 4), (8, 8),
-        (16, 4), (16, 8), (32, 4), (32, 8), (2, 10), (16, 2), (10, 4), (1, 16), (1, 32), (2, 20)],
+        (16, 4), (16, 8), (32, 4), (32, 8), (2, 10)],
     3: [(1, 10), (5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (4, 8), (8, 4), (8, 8), (16, 4),
-        (32, 4), (16, 2), (10, 4), (1, 16)],
-    7: [(5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (8, 4), (16, 4), (32, 4), (16, 2), (10, 4),
-        (1, 10)],
-    15: [(5, 2), (5, 4), (10, 2), (4, 4), (8, 4), (16, 4), (32, 4), (16, 2), (10, 4)],
+        (32, 4)],
+    7: [(5, 2), (2, 6), (5, 4), (10, 2), (4, 4), (4, 6), (8, 4), (16, 4), (32, 4)],
+    15: [(5, 2), (5, 4), (10, 2), (4, 4), (8, 4), (16, 4), (32, 4)],
+}
+# Further ones of csrc/train_*.cu, which run plain recorded trains only.
+TRAIN_SHAPES = {
+    0: [(16, 2), (10, 4), (1, 16), (1, 32), (2, 20)],
+    3: [(16, 2), (10, 4), (1, 16)],
+    7: [(16, 2), (10, 4), (1, 10)],
+    15: [(16, 2), (10, 4)],
 }
 
 
 # (lanes, orders, min blocks per SM) register-budget variants per family.
 REGISTER_VARIANTS = {7: [(5, 4, 5), (5, 4, 6), (10, 2, 8), (4, 4, 6), (5, 4, 4), (10, 2, 6),
                          (10, 2, 7)]}
+
+
+def recorded_train(program: Program) -> bool:
+    """Whether ``program`` is a plain recorded train (``tsg_program_recorded_train``)."""
+    return bool(_native.library().tsg_program_recorded_train(program.handle))
+
+
+def shapes_for(program: Program, family: int) -> list[tuple[int, int]]:
+    """The (lanes per voxel, orders per lane) of a kernel family that run
+    ``program``."""
+    return FAMILY_SHAPES[family] + (TRAIN_SHAPES[family] if recorded_train(program) else [])
 
 
 def mode_of(names: Sequence[str]) -> int:
@@ -467,7 +483,8 @@ def mode_of(names: Sequence[str]) -> int:
 def tuned_shape(program: Program, tissue: TissueMaps, states: int, names: Sequence[str] = (),
                 sample: int = 32768, use_cache: bool = True) -> tuple[int, int, int]:
     """The autotuner's (lanes, orders, warps) for this sweep, timed on the
-    first ``sample`` voxels and cached per (family, states, ops, outputs)."""
+    first ``sample`` voxels and cached per (family, states, ops, outputs) and
+    sweep (a recorded train's or the general one)."""
     from . import autotune
 
     family = mode_of(names) if names else 0
@@ -475,7 +492,8 @@ def tuned_shape(program: Program, tissue: TissueMaps, states: int, names: Sequen
     sub = TissueMaps(*[None if t is None else t[:n] for t in
                        (tissue.t1, tissue.t2, tissue.m0, tissue.b1, tissue.inv)])
     key = autotune.workload_key("sweep", kernel_family=family, states=states, ops=program.ops,
-                                outputs=program.outputs, sample=n)
+                                outputs=program.outputs, sample=n,
+                                form="train" if recorded_train(program) else "general")
     sig = torch.empty((program.trains * n, program.outputs), dtype=torch.complex64,
                       device=tissue.t1.device)
     jac = torch.empty((program.trains * n, max(1, len(names)), program.outputs),
@@ -487,7 +505,7 @@ def tuned_shape(program: Program, tissue: TissueMaps, states: int, names: Sequen
         else:
             forward(program, sub, states, out=sig, launch=shape)
 
-    cands = autotune.sweep_shapes(states, FAMILY_SHAPES[family])
+    cands = autotune.sweep_shapes(states, shapes_for(program, family))
     cands += [(lanes, orders, 4, mb) for lanes, orders, mb in REGISTER_VARIANTS.get(family, [])
               if lanes * orders >= states]
     best, _ = autotune.tune(key, cands, run, use_cache=use_cache)
