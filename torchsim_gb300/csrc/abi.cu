@@ -185,8 +185,9 @@ const TrainRule kTrainRules[] = {
 };
 
 // The kernel of a plain recorded train, or null where the general sweep runs:
-// a requested shape where it has an instantiation (a requested register budget
-// is the general sweep's and is not looked at), else the rules above.
+// a requested shape where it has an instantiation, else the rules above. A
+// requested register budget is the general sweep's: it makes no difference here,
+// but one that the general sweep does not have is refused there.
 const SweepEntry* choose_train(int mode, int states, int64_t work_items, const tsg_launch* want,
                                int* warps) {
     const Table t = train_table_for(mode);
@@ -200,6 +201,8 @@ const SweepEntry* choose_train(int mode, int states, int64_t work_items, const t
     };
     if (want && (want->lanes_per_voxel > 0 || want->orders_per_lane > 0)) {
         if (want->lanes_per_voxel * want->orders_per_lane < states) return nullptr;
+        int w = 0;
+        if (want->min_blocks_per_sm != 0 && !choose(mode, states, work_items, want, &w)) return nullptr;
         return find(want->lanes_per_voxel, want->orders_per_lane);
     }
     for (const TrainRule& r : kTrainRules)
