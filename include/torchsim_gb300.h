@@ -664,6 +664,9 @@ typedef struct {
 /* Candidate lists a voxel may have: with few voxels the atoms are shared among
  * several CTAs, each of which keeps its own. */
 int tsg_match_lists(int64_t voxels, int64_t atom_count, int64_t k);
+/* Candidate lists of all voxels that tsg_match keeps: one each, and more only
+ * for the voxels whose atoms are shared (at most voxels x tsg_match_lists). */
+int64_t tsg_match_list_rows(int64_t voxels, int64_t atom_count, int64_t k);
 /* The two fp16 rows (k wide, zero-padded) of each normalized complex64 signal. */
 int tsg_match_queries(const void* normalized, int64_t voxels, int64_t samples, int64_t k, float scale,
                       int complex_atoms, void* queries, void* stream);
@@ -674,7 +677,7 @@ int tsg_match_screen_lists(const void* queries, int64_t query_rows, const void* 
                            int* error, void* stream);
 /* A whole match of `voxels` complex64 signals, given as they are and
  * normalized, with the norms: query rows (scratch, 2 voxels x k fp16, 16-byte
- * aligned), screen (scratch lists, as tsg_match_screen_lists), exact FP32
+ * aligned), screen (scratch, tsg_match_list_rows x candidates), exact FP32
  * rescoring, and per voxel the top_k (1..8) scores, atom indices, complex
  * least-squares scales, densities and table rows. */
 int tsg_match(const tsg_match_dictionary* dictionary, const void* signals, const void* normalized,

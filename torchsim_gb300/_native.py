@@ -181,6 +181,7 @@ SIGNATURES: dict[str, tuple] = {
     "tsg_match_screen": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "tsg_match_rescore": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _int, _vp, _vp, _vp]),
     "tsg_match_lists": (_int, [_i64, _i64, _i64]),
+    "tsg_match_list_rows": (_i64, [_i64, _i64, _i64]),
     "tsg_match_queries": (_int, [_vp, _i64, _i64, _i64, ctypes.c_float, _int, _vp, _vp]),
     "tsg_match_screen_lists": (_int, [_vp, _i64, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "tsg_match": (_int, [ctypes.POINTER(MatchDictionary), _vp, _vp, _vp, _i64, _int, _vp, _vp, _vp,

@@ -158,7 +158,11 @@ struct ScreenShared {
 // last `split` row pairs are cut into `pieces` runs of `run` atom tiles each,
 // items in order of the run first, so that CTAs working side by side read the
 // same few atom tiles. Pair c takes items c, c + pairs, ... A piece's
-// candidates go to its own list, merged before the rescoring.
+// candidates go to its own list, merged before the rescoring: piece p's list of
+// voxel v is list p list_step + v. With list_step the voxels of the split row
+// pairs there is one list for every voxel and one more of theirs per further
+// piece (65,536 atoms: 58,496 voxels have one split row pair, in 32 pieces; a
+// list for every voxel and piece took 479 MB there, this takes 16).
 struct ScreenWork {
     int n_tiles;  // atom tiles
     int full, split, pieces, run;
@@ -168,6 +172,7 @@ struct ScreenWork {
     int na, nb;   // slots
     int slot;     // bytes of a ring slot in one CTA
     bool resident;
+    int64_t list_step;
 };
 
 struct ScreenItem {
@@ -482,7 +487,7 @@ __global__ void __cluster_dims__(kPair, 1, 1) __launch_bounds__(kThreads, 1)
             }
             const int64_t row = int64_t(it.row_pair * kPair + rank) * BM + (r & ~1);
             if (row < rows && !*abort) {
-                const int64_t at = (int64_t(it.piece) * (rows >> 1) + (row >> 1)) * kCand +
+                const int64_t at = (int64_t(it.piece) * w.list_step + (row >> 1)) * kCand +
                                    (half * 2 + parity) * kScreen;
 #pragma unroll
                 for (int k = 0; k < kScreen; ++k) {
@@ -625,12 +630,12 @@ template <int AXIS>
 __global__ void rescore_kernel(const float2* __restrict__ signals, const void* __restrict__ atoms,
                                int64_t voxels, int64_t samples, const float* __restrict__ list_score,
                                const int32_t* __restrict__ list_index, int full_pairs, int pieces,
-                               int top_k, float* __restrict__ scores, int64_t* __restrict__ index) {
+                               int64_t list_step, int top_k, float* __restrict__ scores, int64_t* __restrict__ index) {
     const int64_t voxel = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (voxel >= voxels) return;
     const int count = 2 * voxel / (BM * kPair) < full_pairs ? 1 : pieces;
-    int mine = merged_candidate(list_score, list_index, voxel * kCand, voxels * kCand, count, lane);
+    int mine = merged_candidate(list_score, list_index, voxel * kCand, list_step * kCand, count, lane);
     const float2* s = signals + voxel * samples;
     float my_score = -1.f;
     // Four candidates at a time, whose loads overlap and share the signal's.
@@ -817,6 +822,7 @@ ScreenWork plan_screen(int64_t query_rows, int64_t atom_count, int64_t k, int pa
     w.nb = std::min(kMaxB, (kTileBytes - w.na * SMEM_A) / w.slot);
     w.full = may_split ? pairs / slots * slots : pairs;
     w.split = pairs - w.full;
+    w.list_step = std::max<int64_t>(0, query_rows / 2 - int64_t(w.full) * (kPair * BM / 2));
     w.pieces = 1;
     w.run = w.n_tiles;
     double best = 1e300;
@@ -872,10 +878,10 @@ int run_screen(const ScreenWork& w, const void* queries, int64_t query_rows, con
 template <int AXIS>
 void run_rescore(const void* signals, int64_t voxels, const void* atoms, int64_t samples,
                  const float* list_score, const int32_t* list_index, int full_pairs, int pieces,
-                 int top_k, float* scores, int64_t* index, cudaStream_t stream) {
+                 int64_t list_step, int top_k, float* scores, int64_t* index, cudaStream_t stream) {
     rescore_kernel<AXIS><<<unsigned((voxels * 32 + 255) / 256), 256, 0, stream>>>(
         static_cast<const float2*>(signals), atoms, voxels, samples, list_score, list_index,
-        full_pairs, pieces, top_k, scores, index);
+        full_pairs, pieces, list_step, top_k, scores, index);
 }
 
 }  // namespace
@@ -902,7 +908,7 @@ extern "C" int tsg_match_rescore(const void* signals, int64_t voxels, const void
     if (voxels == 0) return TSG_OK;
     if (!signals || !atoms || !candidate_index || !scores || !index)
         return fail(TSG_ERR_ARGUMENT, "null rescoring buffer");
-    run_rescore<0>(signals, voxels, atoms, samples, nullptr, candidate_index, 0, 1, top_k, scores,
+    run_rescore<0>(signals, voxels, atoms, samples, nullptr, candidate_index, 0, 1, 0, top_k, scores,
                    index, static_cast<cudaStream_t>(stream));
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
@@ -928,14 +934,21 @@ extern "C" int tsg_match_screen_lists(const void* queries, int64_t query_rows, c
                                 error);
     if (rc || query_rows == 0) return rc;
     const int sms = match_sms();
-    return run_screen(plan_screen(query_rows, atom_count, k, 2, sms, true), queries, query_rows, atoms,
-                      atom_count, k, list_scores, list_index, error, sms,
+    ScreenWork w = plan_screen(query_rows, atom_count, k, 2, sms, true);
+    w.list_step = query_rows / 2;
+    return run_screen(w, queries, query_rows, atoms, atom_count, k, list_scores, list_index, error, sms,
                       static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tsg_match_lists(int64_t voxels, int64_t atom_count, int64_t k) {
     if (voxels < 1 || atom_count < 1 || k < 1) return 1;
     return plan_screen(2 * voxels, atom_count, k, 2, match_sms(), true).pieces;
+}
+
+extern "C" int64_t tsg_match_list_rows(int64_t voxels, int64_t atom_count, int64_t k) {
+    if (voxels < 1 || atom_count < 1 || k < 1) return 1;
+    const ScreenWork w = plan_screen(2 * voxels, atom_count, k, 2, match_sms(), true);
+    return voxels + (w.pieces - 1) * w.list_step;
 }
 
 extern "C" int tsg_match(const tsg_match_dictionary* d, const void* signals, const void* normalized,
@@ -956,15 +969,16 @@ extern "C" int tsg_match(const tsg_match_dictionary* d, const void* signals, con
         !d->normalized_atoms || !d->dictionary || !d->power || (d->columns > 0 && (!d->table || !parameters)))
         return fail(TSG_ERR_ARGUMENT, "null matching buffer");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int sms = match_sms();
+    const ScreenWork w = plan_screen(2 * voxels, d->atom_count, d->k, 2, sms, true);
     int run = tsg_match_queries(normalized, voxels, d->samples, d->k, d->scale, d->axis == 0, queries, stream);
     if (!run)
-        run = tsg_match_screen_lists(queries, 2 * voxels, d->screen_atoms, d->atom_count, d->k, list_scores,
-                                     list_index, error, stream);
+        run = run_screen(w, queries, 2 * voxels, d->screen_atoms, d->atom_count, d->k, list_scores,
+                         list_index, error, sms, s);
     if (run) return run;
-    const ScreenWork w = plan_screen(2 * voxels, d->atom_count, d->k, 2, match_sms(), true);
     auto rescore = d->axis == 0 ? &run_rescore<0> : (d->axis == 1 ? &run_rescore<1> : &run_rescore<2>);
     rescore(normalized, voxels, d->normalized_atoms, d->samples, list_scores, list_index, w.full,
-            w.pieces, top_k, scores, index, s);
+            w.pieces, w.list_step, top_k, scores, index, s);
     TSG_CUDA(cudaGetLastError());
     const int64_t found = voxels * top_k;
     result_kernel<<<unsigned((found * 32 + 255) / 256), 256, 0, s>>>(

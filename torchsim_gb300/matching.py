@@ -306,9 +306,9 @@ class DictionaryMatcher:
             s_hat, norms = _normalized(chunk)
             s_hat = s_hat.contiguous()
             queries = torch.empty((2 * V, prepared.k), dtype=torch.float16, device=self.device)
-            lists = lib.tsg_match_lists(V, prepared.atom_count, prepared.k)
-            list_s = torch.empty((lists, V, m), dtype=torch.float32, device=self.device)
-            list_i = torch.empty((lists, V, m), dtype=torch.int32, device=self.device)
+            lists = lib.tsg_match_list_rows(V, prepared.atom_count, prepared.k)
+            list_s = torch.empty((lists, m), dtype=torch.float32, device=self.device)
+            list_i = torch.empty((lists, m), dtype=torch.int32, device=self.device)
             _native.check(lib.tsg_match(
                 ctypes.byref(prepared), chunk.data_ptr(), s_hat.data_ptr(), norms.data_ptr(), V, k,
                 queries.data_ptr(), list_s.data_ptr(), list_i.data_ptr(), error.data_ptr(),
