@@ -138,10 +138,12 @@ const SweepEntry* choose(int mode, int states, int64_t work_items, const tsg_lau
 // The last goes in steps: 19,456 voxels are one warp of (1,10) for each of 608
 // schedulers, and one more warp there starts a second round, while the warps of
 // (5,2) hold 6 voxels each and fill up 14,592 voxels at a time, four to a
-// scheduler.
+// scheduler. Those lines are in voxels per scheduler (up to 24, 32 and 40), four
+// to each SM that the device has.
 struct TrainRule {
     int mode, states, lanes, orders;
-    int64_t below;  // voxels x trains
+    int64_t below;      // voxels x trains
+    int per_scheduler;  // if not 0: up to this many for each scheduler instead
 };
 constexpr int64_t kAny = INT64_MAX;
 const TrainRule kTrainRules[] = {
@@ -175,8 +177,8 @@ const TrainRule kTrainRules[] = {
     {MODE_T12BI, 32, 16, 2, 4096},     {MODE_T12BI, 32, 8, 4, kAny},
     {MODE_T12BI, 40, 10, 4, kAny},     {MODE_T12BI, 64, 16, 4, kAny},
     {MODE_T12BI, 128, 32, 4, kAny},
-    {MODE_GN, 10, 5, 2, 14593},        {MODE_GN, 10, 1, 10, 19457},
-    {MODE_GN, 10, 5, 2, 24321},        {MODE_GN, 10, 1, 10, kAny},
+    {MODE_GN, 10, 5, 2, 0, 24},        {MODE_GN, 10, 1, 10, 0, 32},
+    {MODE_GN, 10, 5, 2, 0, 40},        {MODE_GN, 10, 1, 10, kAny},
     {MODE_GN, 16, 10, 2, 3072},        {MODE_GN, 16, 4, 4, kAny},
     {MODE_GN, 20, 10, 2, 8192},        {MODE_GN, 20, 2, 10, kAny},
     {MODE_GN, 32, 16, 2, 2048},        {MODE_GN, 32, 8, 4, kAny},
@@ -205,9 +207,10 @@ const SweepEntry* choose_train(int mode, int states, int64_t work_items, const t
         if (want->min_blocks_per_sm != 0 && !choose(mode, states, work_items, want, &w)) return nullptr;
         return find(want->lanes_per_voxel, want->orders_per_lane);
     }
-    for (const TrainRule& r : kTrainRules)
-        if (r.mode == mode && states <= r.states && work_items < r.below)
-            return find(r.lanes, r.orders);
+    for (const TrainRule& r : kTrainRules) {
+        const int64_t below = r.per_scheduler ? int64_t(4) * sm_count() * r.per_scheduler + 1 : r.below;
+        if (r.mode == mode && states <= r.states && work_items < below) return find(r.lanes, r.orders);
+    }
     return nullptr;
 }
 
