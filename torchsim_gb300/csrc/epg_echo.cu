@@ -22,6 +22,12 @@
 // Measured on 96 CPMG protocols of 4 to 64 echoes, 1.5 million voxels: 2.21 ms
 // with the orders spread over lanes, 0.75 ms with every order of one voxel in
 // a lane's pairs, 0.46 ms here with sincosf and 0.43 with turn2().
+//
+// With few units one warp's chain decides, all chunks of an echo one after the
+// other: there the chunks of two voxels go to eight lanes
+// (epg_echo_few_kernel), with the same arithmetic and so the same bits. (Without
+// it a small batch took longer than with the orders spread over lanes: 33
+// and 21 us for one train of 64 echoes.)
 #include "tsg_internal.h"
 
 namespace tsg {
@@ -200,6 +206,140 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
     }
 }
 
+// The same trains with a chunk of orders per lane: lane q of eight holds orders
+// 4 q to 4 q + 3 of two voxels and evaluates the sines and cosines of every
+// eighth echo; the pair that crosses a chunk's edge moves by shuffle. A block
+// takes eight voxels of a unit. Bound: the chain of one echo, about 0.18 us: 64
+// echoes of 64 voxels 18.4 us with the coefficients and selects on it, 16.4 here.
+constexpr int kFewLanes = kSlots / kChunk;
+constexpr int kFewVoxels = 2 * 32 / kFewLanes;
+
+__global__ void __launch_bounds__(32) epg_echo_few_kernel(
+    const Op* __restrict__ ops, const tsg_batch_sequence* __restrict__ seqs,
+    const tsg_batch_unit* __restrict__ units, const float* __restrict__ t1v,
+    const float* __restrict__ t2v, const float* __restrict__ m0v, const float* __restrict__ b1v,
+    float2* __restrict__ out) {
+    __shared__ float s_flip[2 * kSlots];
+    __shared__ float s_rec[kFewVoxels * (kEchoRecords + 1)];
+    constexpr int kBlocks = 64 / kFewVoxels;  // of a unit
+    const int lane = threadIdx.x;
+    const int q = lane % kFewLanes, pair = lane / kFewLanes;
+    const tsg_batch_unit u = units[blockIdx.x / kBlocks];
+    const int begin = int(blockIdx.x % kBlocks) * kFewVoxels;
+    const int voxels = min(min(u.voxel_count, 64) - begin, kFewVoxels);
+    if (voxels <= 0) return;
+    const tsg_batch_sequence sq = seqs[u.sequence];
+    const Op* train = ops + sq.op_offset;
+    const int echoes = sq.op_count >> 1;
+    for (int e = lane; e < echoes; e += 32) s_flip[e] = train[2 * e + 1].flip;
+    __syncwarp();
+    // This group's voxels: pair and pair + kFewVoxels / 2 of the block.
+    const int64_t first = sq.voxel_offset + u.voxel_begin + begin;
+    const int other = pair + kFewVoxels / 2;
+    const int64_t va = first + (pair < voxels ? pair : 0);
+    const int64_t vb = first + (other < voxels ? other : 0);
+    const float dt = train[1].dt;
+    const float2 b1 = b1v ? make_float2(b1v[va], b1v[vb]) : dup(1.f);
+    const float2 m0 = m0v ? make_float2(m0v[va], m0v[vb]) : dup(1.f);
+    const float2 f1 = make_float2(expf(__fmul_rn(-(1000.f / t1v[va]), dt)),
+                                  expf(__fmul_rn(-(1000.f / t1v[vb]), dt)));
+    const float2 f2 = make_float2(expf(__fmul_rn(-(1000.f / t2v[va]), dt)),
+                                  expf(__fmul_rn(-(1000.f / t2v[vb]), dt)));
+    const float2 m0f2 = mul2(m0, f2);
+    const int slots = sq.states >> 1;
+    // All orders run at every echo: the ones that matter meet only each other.
+    // Masks instead of selects keep the truncation and the last lane's edge off
+    // the predicates.
+    int keep[kChunk];
+#pragma unroll
+    for (int j = 0; j < kChunk; ++j)
+        keep[j] = 2 * slots < echoes && q * kChunk + j + 1 >= slots ? 0 : -1;
+    const int inner = q == kFewLanes - 1 ? 0 : -1;
+    auto masked = [](float2 v, int mask) {
+        return make_float2(__int_as_float(__float_as_int(v.x) & mask),
+                           __int_as_float(__float_as_int(v.y) & mask));
+    };
+
+    float2 P[kChunk], N[kChunk], Z[kChunk];
+#pragma unroll
+    for (int j = 0; j < kChunk; ++j) P[j] = N[j] = Z[j] = dup(0.f);
+    {
+        const float2 a = mul2(dup(train[0].flip), b1);
+        if (q == 0 && slots > 0) P[0] = make_float2(-sinf(a.x), -sinf(a.y));
+    }
+    // The pulse of echo e with the relaxation before it (w1, h) folded in.
+    float2 my_si = dup(0.f), my_co = dup(0.f);
+    float2 hco, hsi, nsi, ce;
+    auto coefficients = [&](int e, float2 w1, float2 h) {
+        const int g = e % kFewLanes;
+        if (g == 0) {
+            const float flip = s_flip[min(e + q, echoes - 1)];
+            const float2 angle = mul2(dup(flip), b1);
+            turn2(angle, &my_si, &my_co);
+            if (turns_wild(flip) || turns_wild(b1.x)) sincosf(angle.x, &my_si.x, &my_co.x);
+            if (turns_wild(flip) || turns_wild(b1.y)) sincosf(angle.y, &my_si.y, &my_co.y);
+        }
+        const float2 si = make_float2(__shfl_sync(0xffffffffu, my_si.x, g, kFewLanes),
+                                      __shfl_sync(0xffffffffu, my_si.y, g, kFewLanes));
+        const float2 co = make_float2(__shfl_sync(0xffffffffu, my_co.x, g, kFewLanes),
+                                      __shfl_sync(0xffffffffu, my_co.y, g, kFewLanes));
+        const float2 wsi = mul2(w1, si);
+        hco = mul2(h, co);
+        hsi = mul2(h, si);
+        nsi = make_float2(-wsi.x, -wsi.y);
+        ce = mul2(w1, co);
+    };
+    float2 h = mul2(dup(0.5f), f2);
+    const float2 w_later = mul2(f1, f1), h_later = mul2(dup(0.5f), mul2(f2, f2));
+    coefficients(0, f1, h);
+    int held = 0;
+#pragma unroll 1
+    for (int e = 0; e < echoes; ++e) {
+        const float2 nH = make_float2(-h.x, -h.y);
+        float2 n[kChunk], p[kChunk];
+#pragma unroll
+        for (int j = 0; j < kChunk; ++j) {
+            const float2 s = make_float2(__fadd_rn(P[j].x, -N[j].x), __fadd_rn(P[j].y, -N[j].y));
+            const float2 d = add2(P[j], N[j]);
+            const float2 B = fma2(hco, d, mul2(nsi, Z[j]));
+            Z[j] = fma2(hsi, d, mul2(ce, Z[j]));
+            n[j] = fma2(nH, s, B);
+            p[j] = masked(fma2(h, s, B), keep[j]);
+        }
+        // -F- moves down, F+ up.
+        const float2 above = make_float2(__shfl_down_sync(0xffffffffu, n[0].x, 1, kFewLanes),
+                                         __shfl_down_sync(0xffffffffu, n[0].y, 1, kFewLanes));
+        const float2 below = make_float2(__shfl_up_sync(0xffffffffu, p[kChunk - 1].x, 1, kFewLanes),
+                                         __shfl_up_sync(0xffffffffu, p[kChunk - 1].y, 1, kFewLanes));
+        // The next echo's coefficients meanwhile.
+        h = h_later;
+        coefficients(e + 1, w_later, h_later);
+        if (q == 0) {
+            const float2 y = mul2(m0f2, n[0]);
+            s_rec[pair * (kEchoRecords + 1) + held] = y.x;
+            s_rec[other * (kEchoRecords + 1) + held] = y.y;
+        }
+        P[0] = q == 0 ? (slots > 0 ? n[0] : dup(0.f)) : below;
+#pragma unroll
+        for (int j = 0; j + 1 < kChunk; ++j) {
+            N[j] = n[j + 1];
+            P[j + 1] = p[j];
+        }
+        N[kChunk - 1] = masked(above, inner);
+        if (++held == kEchoRecords || e + 1 == echoes) {
+            __syncwarp();
+            float2* dst = out + sq.output_offset + int64_t(u.voxel_begin + begin) * sq.outputs +
+                          (e + 1 - held) + lane;
+            if (lane < held)
+                for (int v = 0; v < voxels; ++v)
+                    __stcs(dst + int64_t(v) * sq.outputs,
+                           make_float2(0.f, s_rec[v * (kEchoRecords + 1) + lane]));
+            __syncwarp();
+            held = 0;
+        }
+    }
+}
+
 }  // namespace
 }  // namespace tsg
 
@@ -215,7 +355,13 @@ extern "C" int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* s
     if (tissue->inversion) return fail(TSG_ERR_UNSUPPORTED, "batched sequences take no inversion map");
     if (unit_count > 0x7fffffffLL) return fail(TSG_ERR_CAPACITY, "too many units for one launch");
     if (unit_count == 0) return TSG_OK;
-    epg_echo_kernel<<<unsigned(unit_count), 32, 0, static_cast<cudaStream_t>(stream)>>>(
+    // Up to two units for each SM the chain decides (one 64-echo train of 64
+    // voxels: 16 us with the orders over lanes, 35 without); from three the work
+    // does: at 304 units 29 and 37 us, at 456 39 and 37, at 1,216 94 and 45.
+    constexpr int kFewBlocks = 64 / kFewVoxels;
+    const bool few = unit_count <= int64_t(2) * sm_count();
+    auto kernel = few ? &epg_echo_few_kernel : &epg_echo_kernel;
+    kernel<<<unsigned(unit_count) * (few ? kFewBlocks : 1), 32, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const Op*>(ops), sequences, units, tissue->t1_ms, tissue->t2_ms, tissue->m0,
         tissue->b1, static_cast<float2*>(out));
     TSG_CUDA(cudaGetLastError());
