@@ -522,6 +522,13 @@ int tsg_echo_train(const void* host_ops, int64_t op_count);
 int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* sequences,
                          const tsg_batch_unit* units, int64_t unit_count, const tsg_tissue* tissue,
                          void* out, void* stream);
+/* The same samples with the orders of two voxels over `lanes` (1, 2, 4 or 8)
+ * lanes, four to each, from units of up to 64 / lanes voxels: for few voxels, or
+ * few of each sequence. Every sequence has min(states / 2, (echoes + 1) / 2) <=
+ * 4 lanes. */
+int tsg_epg_echo_few_forward(const void* ops, const tsg_batch_sequence* sequences,
+                             const tsg_batch_unit* units, int64_t unit_count,
+                             const tsg_tissue* tissue, void* out, int lanes, void* stream);
 
 /* ---- Gauss-Newton mapping ---------------------------------------------- */
 

@@ -131,6 +131,8 @@ SIGNATURES: dict[str, tuple] = {
     "tsg_fse_recovery": (_int, [_vp, _vp, _i64, _i64, _int, _int, _vp, _int, _vp, _i64, _vp, _i64,
                                 ctypes.c_float, ctypes.c_float, _vp, _vp, _vp]),
     "tsg_epg_echo_forward": (_int, [_vp, _vp, _vp, _i64, ctypes.POINTER(Tissue), _vp, _vp]),
+    "tsg_epg_echo_few_forward": (_int, [_vp, _vp, _vp, _i64, ctypes.POINTER(Tissue), _vp, _int,
+                                        _vp]),
     "tsg_mrf_stream": (_int, [_vp, _vp, _vp, _i64, ctypes.c_float, _i64, ctypes.c_float,
                               ctypes.c_float, _vp, _vp, _vp, _vp]),
     "tsg_mrf_stream_vjp": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp]),

@@ -8,11 +8,12 @@ to its own problem, with a tail of idle SMs after every small one.
 compiled programs back to back, their tissue back to back, and a list of
 (sequence, voxel tile) units sorted largest first. CPMG trains (the excitation,
 then per echo one refocusing pulse and one sample) run two voxels per lane with
-only the orders that matter at each echo (``tsg_epg_echo_forward``); a single
-launch of the persistent kernel (``tsg_epg_batched_forward``) works through the
-other sequences' units. The launches and the counter reset are captured once in
-a CUDA graph and replayed. The persistent launch's shape (orders per lane, warps per CTA, CTAs per SM) is picked by
-:mod:`torchsim_gb300.autotune`.
+only the orders that matter at each echo (``tsg_epg_echo_forward``), or with the
+orders over lanes where there are few voxels (``tsg_epg_echo_few_forward``); a
+single launch of the persistent kernel (``tsg_epg_batched_forward``) works through
+the other sequences' units. The launches and the counter reset are captured once
+in a CUDA graph and replayed. The persistent launch's shape (orders per lane,
+warps per CTA, CTAs per SM) is picked by :mod:`torchsim_gb300.autotune`.
 """
 
 from __future__ import annotations
@@ -56,6 +57,17 @@ def compile_ops(events: PackedEvents) -> np.ndarray:
 
 # Voxels per unit of the echo kernel: one warp, two voxels per lane.
 ECHO_UNIT = 64
+# Orders that matter which a lane holds of the kernel's form for few voxels. It
+# runs batches of up to ECHO_FEW_UNITS of its units for each SM, where one echo's
+# chain decides, and ones with at most ECHO_FEW_RATIO of them for each of the other
+# form's, where that one's lanes idle or hold orders that no train reaches. Dense
+# units of 64 voxels, us, this form and the other: 64 echoes (eight lanes) 300 units
+# 29 and 37, 1,216 94 and 45; 32 echoes (four) 300 units 12 and 18, 5,000 98 and 90;
+# 16 echoes (two) 5,000 units 37 and 47; 8 echoes (one) 16 and 31. 2,000 trains of
+# 64 echoes of 24 voxels (three units for one) 59 and 86, of 40 (five) 94 and 86.
+ECHO_CHUNK = 4
+ECHO_FEW_UNITS = 16
+ECHO_FEW_RATIO = 3
 
 
 @dataclass
@@ -111,7 +123,7 @@ class SequenceBatch:
         total = int((self.voxels * self.outputs).sum())
         self.out = torch.empty(total, dtype=torch.complex64, device=device)
         self.counter = torch.zeros(1, dtype=torch.int32, device=device)
-        # CPMG trains run two voxels per lane (tsg_epg_echo_forward), the other
+        # CPMG trains run the echo kernel's two forms (_echo_plan), the other
         # sequences the persistent kernel.
         lib = _native.library()
         self.echo = np.array([bool(lib.tsg_echo_train(p.ctypes.data, len(p))) for p in programs], bool)
@@ -163,12 +175,21 @@ class SequenceBatch:
         return self._tables[key]
 
     def _echo_plan(self) -> tuple:
+        """(sequences, units, how many, lanes for the orders of two voxels or 0
+        where a lane holds them all)."""
         if self._echo_tables is None:
+            sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+            orders = np.minimum(self.states // 2, (self.outputs + 1) // 2)
+            lanes = next(n for n in (1, 2, 4, 8) if ECHO_CHUNK * n >= orders[self.echo].max())
+            wide, few = (int((-(-self.voxels[self.echo] // n)).sum())
+                         for n in (ECHO_UNIT, ECHO_UNIT // lanes))
+            if few > max(ECHO_FEW_UNITS * sms, ECHO_FEW_RATIO * wide):
+                lanes = 0
             d_seq = torch.from_numpy(self._sequences(1).view(np.uint8)).to(self.device)
             reached = np.minimum(self.states, self.outputs)
-            units = self._units(self.echo, np.full(len(self.entries), ECHO_UNIT, np.int64),
-                                self.outputs * (reached + 8))
-            self._echo_tables = (d_seq, *units)
+            per_unit = np.full(len(self.entries), ECHO_UNIT // max(lanes, 1), np.int64)
+            units = self._units(self.echo, per_unit, self.outputs * (reached + 8))
+            self._echo_tables = (d_seq, *units, lanes)
         return self._echo_tables
 
     def launch(self, shape: tuple[int, int, int]) -> None:
@@ -182,10 +203,11 @@ class SequenceBatch:
                                 None if self.m0 is None else self.m0.data_ptr(),
                                 None if self.b1 is None else self.b1.data_ptr(), None)
         if self.echo.any():
-            d_seq, d_units, n_units = self._echo_plan()
-            _native.check(lib.tsg_epg_echo_forward(
-                self.d_ops.data_ptr(), d_seq.data_ptr(), d_units.data_ptr(), n_units,
-                ctypes.byref(tissue), self.out.data_ptr(), stream))
+            d_seq, d_units, n_units, lanes = self._echo_plan()
+            args = (self.d_ops.data_ptr(), d_seq.data_ptr(), d_units.data_ptr(), n_units,
+                    ctypes.byref(tissue), self.out.data_ptr())
+            _native.check(lib.tsg_epg_echo_few_forward(*args, lanes, stream) if lanes
+                          else lib.tsg_epg_echo_forward(*args, stream))
         if not self.echo.all():
             d_seq, d_units, n_units = self._plan(orders, warps)
             _native.check(lib.tsg_epg_batched_forward(

@@ -10,16 +10,6 @@
 
 namespace tsg {
 
-int sm_count() {
-    static int count = [] {
-        int dev = 0, n = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        return n > 0 ? n : 1;
-    }();
-    return count;
-}
-
 namespace {
 
 struct Table {
@@ -48,6 +38,16 @@ Table train_table_for(int mode) {
         case MODE_GN: return {kTrainGN, kTrainGNCount};
     }
     return {nullptr, 0};
+}
+
+int sm_count() {
+    static int count = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n > 0 ? n : 1;
+    }();
+    return count;
 }
 
 // Built-in launch heuristic: the fewest padded orders (L*R >= states), then

@@ -24,10 +24,11 @@
 // a lane's pairs, 0.46 ms here with sincosf and 0.43 with turn2().
 //
 // With few units one warp's chain decides, all chunks of an echo one after the
-// other: there the chunks of two voxels go to eight lanes
-// (epg_echo_few_kernel), with the same arithmetic and so the same bits. (Without
-// it a small batch took longer than with the orders spread over lanes: 33
-// and 21 us for one train of 64 echoes.)
+// other, and with few voxels in each unit most lanes idle: there the chunks of
+// two voxels go to lanes of their own (epg_echo_few_kernel), with the same
+// arithmetic and so the same bits. (Without it such a batch took longer than with the
+// orders spread over lanes: one train of 64 echoes 33 and 21 us, 2,000 of them
+// with four voxels each 84 and 47.)
 #include "tsg_internal.h"
 
 namespace tsg {
@@ -206,35 +207,33 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
     }
 }
 
-// The same trains with a chunk of orders per lane: lane q of eight holds orders
-// 4 q to 4 q + 3 of two voxels and evaluates the sines and cosines of every
-// eighth echo; the pair that crosses a chunk's edge moves by shuffle. A block
-// takes eight voxels of a unit. Bound: the chain of one echo, about 0.18 us: 64
-// echoes of 64 voxels 18.4 us with the coefficients and selects on it, 16.4 here.
-constexpr int kFewLanes = kSlots / kChunk;
-constexpr int kFewVoxels = 2 * 32 / kFewLanes;
-
+// The same trains with a chunk of orders per lane: lane q of kFewLanes holds
+// orders 4 q to 4 q + 3 of two voxels and evaluates the sines and cosines of every
+// kFewLanes-th echo; the pair that crosses a chunk's edge moves by shuffle. A unit
+// has up to 64 / kFewLanes voxels. Bound: the chain of one echo, about 0.18 us: 64
+// echoes of 64 voxels 18.4 us with the coefficients and selects on it, 16.4 here;
+// with many units issue, on eight lanes a voxel's echo at twice the instructions
+// of the other kernel. (The lines between the two: torchsim_gb300/batching.py.)
+template <int kFewLanes>
 __global__ void __launch_bounds__(32) epg_echo_few_kernel(
     const Op* __restrict__ ops, const tsg_batch_sequence* __restrict__ seqs,
     const tsg_batch_unit* __restrict__ units, const float* __restrict__ t1v,
     const float* __restrict__ t2v, const float* __restrict__ m0v, const float* __restrict__ b1v,
     float2* __restrict__ out) {
+    constexpr int kFewVoxels = 2 * 32 / kFewLanes;
     __shared__ float s_flip[2 * kSlots];
     __shared__ float s_rec[kFewVoxels * (kEchoRecords + 1)];
-    constexpr int kBlocks = 64 / kFewVoxels;  // of a unit
     const int lane = threadIdx.x;
     const int q = lane % kFewLanes, pair = lane / kFewLanes;
-    const tsg_batch_unit u = units[blockIdx.x / kBlocks];
-    const int begin = int(blockIdx.x % kBlocks) * kFewVoxels;
-    const int voxels = min(min(u.voxel_count, 64) - begin, kFewVoxels);
-    if (voxels <= 0) return;
+    const tsg_batch_unit u = units[blockIdx.x];
+    const int voxels = min(u.voxel_count, kFewVoxels);
     const tsg_batch_sequence sq = seqs[u.sequence];
     const Op* train = ops + sq.op_offset;
     const int echoes = sq.op_count >> 1;
     for (int e = lane; e < echoes; e += 32) s_flip[e] = train[2 * e + 1].flip;
     __syncwarp();
-    // This group's voxels: pair and pair + kFewVoxels / 2 of the block.
-    const int64_t first = sq.voxel_offset + u.voxel_begin + begin;
+    // This group's voxels: pair and pair + kFewVoxels / 2 of the unit.
+    const int64_t first = sq.voxel_offset + u.voxel_begin;
     const int other = pair + kFewVoxels / 2;
     const int64_t va = first + (pair < voxels ? pair : 0);
     const int64_t vb = first + (other < voxels ? other : 0);
@@ -328,7 +327,7 @@ __global__ void __launch_bounds__(32) epg_echo_few_kernel(
         N[kChunk - 1] = masked(above, inner);
         if (++held == kEchoRecords || e + 1 == echoes) {
             __syncwarp();
-            float2* dst = out + sq.output_offset + int64_t(u.voxel_begin + begin) * sq.outputs +
+            float2* dst = out + sq.output_offset + int64_t(u.voxel_begin) * sq.outputs +
                           (e + 1 - held) + lane;
             if (lane < held)
                 for (int v = 0; v < voxels; ++v)
@@ -345,9 +344,11 @@ __global__ void __launch_bounds__(32) epg_echo_few_kernel(
 
 using namespace tsg;
 
-extern "C" int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* sequences,
-                                    const tsg_batch_unit* units, int64_t unit_count,
-                                    const tsg_tissue* tissue, void* out, void* stream) {
+namespace {
+
+int launch_echo(decltype(&epg_echo_kernel) kernel, const void* ops, const tsg_batch_sequence* sequences,
+                const tsg_batch_unit* units, int64_t unit_count, const tsg_tissue* tissue, void* out,
+                void* stream) {
     if (unit_count < 0 || (unit_count > 0 && (!ops || !sequences || !units || !out)))
         return fail(TSG_ERR_ARGUMENT, "null batch buffer");
     if (!tissue || (unit_count > 0 && (!tissue->t1_ms || !tissue->t2_ms)))
@@ -355,17 +356,32 @@ extern "C" int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* s
     if (tissue->inversion) return fail(TSG_ERR_UNSUPPORTED, "batched sequences take no inversion map");
     if (unit_count > 0x7fffffffLL) return fail(TSG_ERR_CAPACITY, "too many units for one launch");
     if (unit_count == 0) return TSG_OK;
-    // Up to two units for each SM the chain decides (one 64-echo train of 64
-    // voxels: 16 us with the orders over lanes, 35 without); from three the work
-    // does: at 304 units 29 and 37 us, at 456 39 and 37, at 1,216 94 and 45.
-    constexpr int kFewBlocks = 64 / kFewVoxels;
-    const bool few = unit_count <= int64_t(2) * sm_count();
-    auto kernel = few ? &epg_echo_few_kernel : &epg_echo_kernel;
-    kernel<<<unsigned(unit_count) * (few ? kFewBlocks : 1), 32, 0, static_cast<cudaStream_t>(stream)>>>(
+    kernel<<<unsigned(unit_count), 32, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const Op*>(ops), sequences, units, tissue->t1_ms, tissue->t2_ms, tissue->m0,
         tissue->b1, static_cast<float2*>(out));
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
+}
+
+}  // namespace
+
+extern "C" int tsg_epg_echo_forward(const void* ops, const tsg_batch_sequence* sequences,
+                                    const tsg_batch_unit* units, int64_t unit_count,
+                                    const tsg_tissue* tissue, void* out, void* stream) {
+    return launch_echo(&epg_echo_kernel, ops, sequences, units, unit_count, tissue, out, stream);
+}
+
+extern "C" int tsg_epg_echo_few_forward(const void* ops, const tsg_batch_sequence* sequences,
+                                        const tsg_batch_unit* units, int64_t unit_count,
+                                        const tsg_tissue* tissue, void* out, int lanes,
+                                        void* stream) {
+    switch (lanes) {
+        case 1: return launch_echo(&epg_echo_few_kernel<1>, ops, sequences, units, unit_count, tissue, out, stream);
+        case 2: return launch_echo(&epg_echo_few_kernel<2>, ops, sequences, units, unit_count, tissue, out, stream);
+        case 4: return launch_echo(&epg_echo_few_kernel<4>, ops, sequences, units, unit_count, tissue, out, stream);
+        case 8: return launch_echo(&epg_echo_few_kernel<8>, ops, sequences, units, unit_count, tissue, out, stream);
+    }
+    return fail(TSG_ERR_ARGUMENT, "1, 2, 4 or 8 lanes for a voxel's orders");
 }
 
 // A train the echo kernel runs: the excitation alone, then per echo the

@@ -227,8 +227,6 @@ extern const int kTrainT12BICount;
 extern const SweepEntry kTrainGN[];
 extern const int kTrainGNCount;
 
-int sm_count();  // of the device the library first ran on
-
 constexpr int kOpChunk = 1024;  // ops staged in shared memory at a time
 
 // Arguments of the checkpointed reverse sweep.
