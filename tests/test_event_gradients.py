@@ -1,5 +1,6 @@
-"""Only the event buffers whose protocol argument is differentiated require a
-gradient: flips that move leave the durations alone, and the other way round."""
+"""Gradients that reach the event buffers of an MRF train: only the buffers whose
+protocol argument is differentiated require one (flips that move leave the
+durations alone, and the other way round), and a second backward is defined."""
 
 from __future__ import annotations
 
@@ -50,3 +51,26 @@ def test_device_built_events(cuda, moved):
     both = grads(("flip", "tr"))
     for name, g in grads(moved).items():
         assert torch.equal(g, both[name])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("device", ["cuda", "cpu"])
+@pytest.mark.parametrize("moved", [("flip",), ("flip", "tr")])
+@pytest.mark.parametrize("route", ["jacobian", "off axis"])
+def test_second_backward_of_a_sweep_that_has_none(cuda, route, moved, device):
+    """The Jacobian's and the complex path's own backward end the graph; what is
+    left of a second derivative is the flips' sign, which does not change."""
+    from torchsim_gb300 import MRFSimulator
+
+    flip, tr = _leaves(device, moved)
+    t1, t2 = torch.linspace(300, 1500, 9, device=cuda), torch.linspace(30, 120, 9, device=cuda)
+    model = MRFSimulator(flip=flip, TR=tr, states=7)
+    if route == "jacobian":
+        out = model.jacobian(("T1", "T2"), T1=t1, T2=t2)[1]
+    else:
+        out = model.simulate(T1=t1, T2=t2, B0=torch.linspace(-20, 20, 9, device=cuda))
+    leaves = [x for x in (flip, tr) if x.requires_grad]
+    first = torch.autograd.grad(out.abs().square().sum(), leaves, create_graph=True)
+    assert first[0].requires_grad and bool(first[0].any())
+    (second,) = torch.autograd.grad(first[0].square().sum(), [flip])
+    assert second.shape == flip.shape and not bool(second.any())

@@ -539,7 +539,7 @@ class MrfEvents(torch.autograd.Function):
         some = g_flip_ev if g_flip_ev is not None else g_dur_ev
         if some is None:
             return (None,) * 4
-        g_flip, g_tr = _stream_transpose(flip.detach().to(some.device), g_flip_ev, g_dur_ev)
+        g_flip, g_tr = _stream_transpose(flip.to(some.device), g_flip_ev, g_dur_ev)
         if g_flip is not None:
             g_flip = g_flip.to(flip.device, flip.dtype)
         if g_tr is not None:
@@ -557,12 +557,15 @@ def _summed_to(g: torch.Tensor | None, shape: torch.Size | None) -> torch.Tensor
 def _stream_transpose(flip: torch.Tensor, g_flip_ev: torch.Tensor | None,
                       g_dur_ev: torch.Tensor | None):
     """Cotangents of the event buffers (None: not wanted) back onto the flips
-    (deg, on the buffers' device) and the per-pulse TRs (ms)."""
+    (deg, on the buffers' device) and the per-pulse TRs (ms). Under
+    ``create_graph`` the result depends on the flips through their sign, as the
+    chain of tensor operations did: a second backward finds its way (of zeros)
+    to them also where the sweep's own backward cannot be differentiated."""
     n = flip.numel()
     if torch.is_grad_enabled():
         g_flip = g_tr = None
         if g_flip_ev is not None:
-            played = g_flip_ev[0, 1::4] * (2.0 * torch.pi) * flip.detach().sgn()
+            played = g_flip_ev[0, 1::4] * (2.0 * torch.pi) * flip.sgn()
             g_flip = torch.deg2rad(played * _HARD_PULSE_AREA)
         if g_dur_ev is not None:
             g_tr = torch.cat((g_dur_ev[0, 5::4] * 1e-3, g_dur_ev.new_zeros(1)))
