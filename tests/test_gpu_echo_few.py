@@ -88,5 +88,5 @@ def test_a_small_batch_is_no_slower_than_the_persistent_kernel(cuda, tmp_path, m
         return min(times)
 
     # 16, 16, 29 and 16 us against 22, 16, 47 and 16; with two voxels per lane 35,
-    # 31, 84 and 27.
-    assert best_us(True) <= 1.25 * best_us(False)
+    # 31, 84 and 27. (Half as long again: timings come in steps of 2 us.)
+    assert best_us(True) <= 1.5 * best_us(False)

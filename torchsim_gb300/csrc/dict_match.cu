@@ -66,8 +66,11 @@ constexpr int kPair = 2;
 // resident, its query tile. One wait and one commit then go with all the
 // products of a contraction tile: each tcgen05.commit holds up the products
 // after it, and with one for every part and query tile the pipe stayed 60%
-// active whatever the ring's depth (65,536 voxels x 262,144 atoms x 880
-// samples 84.1 ms, now 67.2; 16,384 x 65,536 x 500 2.95 and 2.43).
+// active whatever the ring's depth (16,384 voxels x 65,536 atoms x 500 samples
+// 2.95 and 2.43 ms). At whole waves the gain is as large as the power cap lets
+// it: 65,536 x 262,144 x 880 against one CTA per 128 rows 84 and 70 ms after a
+// pause, 88 and 75 back to back, on the MRF dictionary under the benchmark's
+// load 78 and 78 to 79.
 constexpr int kResident = 8;
 constexpr int kMaxA = 8, kMaxB = 10;
 constexpr int kTileBytes = 224 * 1024;  // of both

@@ -367,7 +367,8 @@ __device__ __forceinline__ float2 dot_acc(const float2 (&y)[RP], const float2 (&
 // need: held to 128 registers they spill, 1.24 to 1.43 ms at 16,384 voxels x
 // 601 ops x 20 states.
 //
-// Bound: instruction issue; the trajectory's 5 GB there are 0.75 ms. With the
+// Bound: the latency of an op's chain at two warps a scheduler (0.47 issued a
+// cycle); the trajectory's 5 GB there are 0.75 ms. With the
 // general 3x3 pulse (states outside its frame, derivatives by applying their
 // own matrices), seeds read where they are used and two orders per lane it was
 // 2.13 ms; the frame takes 0.30 off, the seeds 0.26, four orders 0.33 and the

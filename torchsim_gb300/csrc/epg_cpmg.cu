@@ -28,7 +28,8 @@
 // The L lanes share the pulses' sincosf. Samples go to shared memory and leave
 // 16 echoes at a time.
 //
-// Bound: instruction issue, two thirds of it the paired products. Measured at
+// Bound: the latency of an echo's chain at three warps a scheduler (0.51
+// issued a cycle; 55% of the instructions are the paired products). Measured at
 // 65,536 voxels x 48 echoes x 32 states, signal with T1 and T2 columns:
 // 104 us (the complex sweep: 1,220 us); at 8,192 voxels 33 us.
 #include "epg_complex.cuh"

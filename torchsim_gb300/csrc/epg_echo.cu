@@ -47,7 +47,8 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a
 // reduction to |r| <= pi/4 by a three-part pi/2 (W. J. Cody and W. Waite,
 // Software Manual for the Elementary Functions, 1980; with fused products the
 // first difference is exact) and the Taylor series to r^9 and r^10, whose
-// remainders there are 2e-9 and 2e-10. At most 1.5 ulp over that range.
+// remainders there are 2e-9 and 2e-10. Against extended precision its steps are
+// within 1.5 ulp up to 1e5 rad and within 2 ulp over the range.
 // kTurnLimit bounds a flip in rad and a B1 factor each; a voxel or echo beyond
 // it, or NaN, calls sincosf.
 constexpr float kTurnLimit = 1024.f;
@@ -212,8 +213,9 @@ __global__ void __launch_bounds__(32, 8) epg_echo_kernel(
 // kFewLanes-th echo; the pair that crosses a chunk's edge moves by shuffle. A unit
 // has up to 64 / kFewLanes voxels. Bound: the chain of one echo, about 0.18 us: 64
 // echoes of 64 voxels 18.4 us with the coefficients and selects on it, 16.4 here;
-// with many units issue, on eight lanes a voxel's echo at twice the instructions
-// of the other kernel. (The lines between the two: torchsim_gb300/batching.py.)
+// with many units the paired FMAs (47% active, 0.64 issued a cycle), on eight
+// lanes at twice the other kernel's time for a dense unit. (The lines between the
+// two: torchsim_gb300/batching.py.)
 template <int kFewLanes>
 __global__ void __launch_bounds__(32) epg_echo_few_kernel(
     const Op* __restrict__ ops, const tsg_batch_sequence* __restrict__ seqs,

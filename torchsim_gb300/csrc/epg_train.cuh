@@ -24,13 +24,13 @@
 //   op and lane writes an 8-byte piece of a 32-byte sector each time).
 //
 // Bound: with many voxels the FMA pipe and its register ports (ncu, T1/T2/B1
-// at 20 states: FMA pipe 57% active, issue 60%, math-pipe throttle and fixed
+// at 20 states: FMA pipe 61% active, issue 63%, math-pipe throttle and fixed
 // latencies the leading stalls; more warps per SM measured no faster); with
-// few, one op's chain of paired FMAs and one shuffle. Measured against the
+// few, one op's chain of paired FMAs and two shuffles. Measured against the
 // general sweep on the same trains: signal of 1,024 voxels x 880 pulses x 10
 // states 321 -> 61 us, with T1 and T2 568 -> 94 us; 100,000 x 500 x 32 signal
-// 1,256 -> 704 us (41 TFLOP/s of 18 per order and pulse), with T1 and T2
-// 2,166 -> 1,758 us; 262,144 x 880 x 20 with T1, T2 and B1 10.12 -> 7.98 ms
+// 1,256 -> 705 us (41 TFLOP/s of 18 per order and pulse), with T1 and T2
+// 2,166 -> 1,757 us; 262,144 x 880 x 20 with T1, T2 and B1 10.12 -> 7.99 ms
 // (83 TFLOP/s of 144 per order and pulse, above the pipe's 78 because the
 // folded step needs fewer); Gauss-Newton sums of 16,384 x 880 x 10
 // 606 -> 330 us.

@@ -7,15 +7,16 @@ match returns the top-k atoms with their scores, the complex least-squares
 scale (proton density and receive phase), its size and the atoms' parameter
 values.
 
-The search is one tensor-core kernel per chunk of voxels
-(``tsg_match_screen``): fp16 products accumulated in FP32 in tensor memory,
-with the selection of each voxel's best 32 atoms fused into the epilogue, so
-the voxel x atom score matrix never exists. Each atom enters the screen as two
+The search is one call per chunk of voxels (``tsg_match``) around a tensor-core
+screen: fp16 products accumulated in FP32 in tensor memory, with the selection
+of each voxel's best 32 atoms fused into the epilogue, so the voxel x atom score
+matrix never exists (the last voxels share their atoms among idle SMs, with
+further lists of 32 that are merged). Each atom enters the screen as two
 fp16 rows (its value and the rounding remainder), so the screen's scores carry
 the atoms to ~22 bits and only the query's rounding, which shifts near-parallel
 atoms alike, is left. The candidates are then rescored exactly in FP32 against
-the complex signals (``tsg_match_rescore``) and the top k kept, so the screen
-only narrows which atoms are compared exactly.
+the complex signals and the top k kept, so the screen only narrows which atoms
+are compared exactly; the scales, densities and parameters come with them.
 
 Group matching (``groups``) is the reference's option for dictionaries too
 large to search exhaustively (``estimators/_grouped.py``; Cauley, Setsompop,

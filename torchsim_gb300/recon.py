@@ -18,13 +18,14 @@ The same faces are kept here -- :class:`ModelOperator` (``A``, ``A_jvp``,
 -- with two routes under ``minimize``:
 
 * the fused route, for the MRF model of (T1, T2, M0) with B1 known (the
-  mapping workload): the state of every voxel stays on the device
-  (:class:`VoxelPool`), each iteration is three launches -- the FP64 step
-  (``tsg_gn_step``), ONE fused sweep that reduces the model and both tangents
-  straight to the normal equations against the measured samples
-  (``tsg_gn_evaluate``), and the FP64 accept / damping update
-  (``tsg_gn_judge``) -- and finished voxels are compacted away, as the
-  reference's ``_retire`` does (``_gauss_newton.py:759-793``);
+  mapping workload): the state of every voxel stays on the device, each
+  iteration is the FP64 step, ONE fused sweep that reduces the model and both
+  tangents straight to the normal equations against the measured samples, the
+  FP64 accept / damping update with the list of voxels still live (the
+  reference's ``_retire``, ``_gauss_newton.py:759-793``) and the totals -- four
+  launches, of many iterations at once (``tsg_gn_solve_part``). The mapping
+  server runs the same step, sweep and update over a :class:`VoxelPool`, which
+  takes in and compacts away voxels between iterations;
 * the block route, for any other operator: the reference's loop over the
   operator's Jacobian blocks, which come from one fused forward + tangents
   sweep per evaluation, with the damped step solved from the normal equations
