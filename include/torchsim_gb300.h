@@ -231,8 +231,14 @@ int tsg_mrf_stream(const tsg_program* tmpl, const float* flip_deg, const float* 
                    int64_t tr_count, float tr_value, int64_t pulses, float start_s,
                    float first_stamp_us, float* flip_rad, float* duration_s, void* device_ops,
                    void* stream);
+/* The same, and the flips' signs (nullable), one per pulse. */
+int tsg_mrf_stream_signs(const tsg_program* tmpl, const float* flip_deg, const float* tr_ms,
+                         int64_t tr_count, float tr_value, int64_t pulses, float start_s,
+                         float first_stamp_us, float* flip_rad, float* duration_s,
+                         void* device_ops, float* signs, void* stream);
 /* Its transpose: cotangents of the two event buffers (nullable: zero) onto the
- * flips and per-pulse TRs (nullable: not computed). */
+ * flips and per-pulse TRs (nullable: not computed). Of the flips only the signs
+ * are read. */
 int tsg_mrf_stream_vjp(const float* flip_deg, int64_t pulses, const float* flip_cotangent,
                        const float* duration_cotangent, float* flip_gradient, float* tr_gradient,
                        void* stream);

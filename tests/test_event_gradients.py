@@ -1,6 +1,7 @@
 """Gradients that reach the event buffers of an MRF train: only the buffers whose
 protocol argument is differentiated require one (flips that move leave the
-durations alone, and the other way round), and a second backward is defined."""
+durations alone, and the other way round), a second backward is defined, and a
+protocol tensor may change in place once the signal is there."""
 
 from __future__ import annotations
 
@@ -24,7 +25,8 @@ def test_host_built_events(moved):
     flip, tr = _leaves("cpu", moved)
     events = mrf_events(flip.detach(), tr.detach())
     flip_ev, dur_ev = MrfEvents.apply(flip, tr if tr.requires_grad else None,
-                                      torch.from_numpy(events.flip), torch.from_numpy(events.duration))
+                                      torch.from_numpy(events.flip),
+                                      torch.from_numpy(events.duration))[:2]
     assert flip_ev.requires_grad is ("flip" in moved)
     assert dur_ev.requires_grad is ("tr" in moved)
 
@@ -74,3 +76,25 @@ def test_second_backward_of_a_sweep_that_has_none(cuda, route, moved, device):
     assert first[0].requires_grad and bool(first[0].any())
     (second,) = torch.autograd.grad(first[0].square().sum(), [flip])
     assert second.shape == flip.shape and not bool(second.any())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("device", ["cuda", "cpu"])
+@pytest.mark.parametrize("second", [False, True])
+def test_protocol_tensors_change_in_place_after_the_forward(cuda, device, second):
+    from torchsim_gb300 import MRFSimulator
+
+    t1, t2 = torch.linspace(300, 1500, 9, device=cuda), torch.linspace(30, 120, 9, device=cuda)
+
+    def run(change):
+        flip, tr = _leaves(device, ("flip", "tr"))
+        f, r = flip * torch.tensor([1.0, -1.0], device=device).repeat(N // 2), tr * 1.0
+        sig = MRFSimulator(flip=f, TR=r, states=7).simulate(T1=t1, T2=t2)
+        if change:
+            with torch.no_grad():
+                f.mul_(-3.0), r.zero_()
+        got = torch.autograd.grad(sig.real.square().sum(), (flip, tr), create_graph=second)
+        return torch.autograd.grad(sum((g * g).sum() for g in got), (flip, tr)) if second else got
+
+    for a, b in zip(run(True), run(False)):
+        assert bool(b.any()) and torch.equal(a, b)

@@ -135,6 +135,8 @@ SIGNATURES: dict[str, tuple] = {
                                         _vp]),
     "tsg_mrf_stream": (_int, [_vp, _vp, _vp, _i64, ctypes.c_float, _i64, ctypes.c_float,
                               ctypes.c_float, _vp, _vp, _vp, _vp]),
+    "tsg_mrf_stream_signs": (_int, [_vp, _vp, _vp, _i64, ctypes.c_float, _i64, ctypes.c_float,
+                                    ctypes.c_float, _vp, _vp, _vp, _vp, _vp]),
     "tsg_mrf_stream_vjp": (_int, [_vp, _i64, _vp, _vp, _vp, _vp, _vp]),
     "tsg_sequential_sum": (_int, [_vp, _i64, _vp, _vp]),
     "tsg_epg_forward": (_int, [_vp, ctypes.POINTER(Tissue), _i64, _i64, _int, _vp, _vp,

@@ -414,13 +414,16 @@ __global__ void rebind_kernel(const Op* __restrict__ tmpl, const OpSource* __res
 // stamps in microseconds, their differences back to seconds), then the op
 // table (rebind_kernel). Latency-bound: one launch for some twenty
 // elementwise ones, the sum by one thread from shared memory.
+__device__ __forceinline__ float sign_of(float x) { return x > 0.f ? 1.f : (x < 0.f ? -1.f : x); }
+
 constexpr int kStreamChunk = 1024;
 constexpr int kStreamThreads = 256;
 __global__ void __launch_bounds__(kStreamThreads)
     mrf_stream_kernel(const float* __restrict__ flip_deg, const float* __restrict__ tr_ms,
                       int64_t tr_count, float tr_value, int64_t n, float start, float first_stamp,
                       const Op* __restrict__ tmpl, const OpSource* __restrict__ src, int64_t ops,
-                      float* flip_ev, float* dur_ev, Op* __restrict__ out) {
+                      float* flip_ev, float* dur_ev, Op* __restrict__ out,
+                      float* __restrict__ signs) {
     __shared__ float s_cursor[kStreamChunk + 1];  // [0]: the pulse before the chunk
     __shared__ float s_next;
     if (threadIdx.x == 0) {
@@ -451,7 +454,9 @@ __global__ void __launch_bounds__(kStreamThreads)
             const int64_t k = base + i;
             const float now = stamp(k, s_cursor[1 + i]);
             const float before = k == 0 ? 0.f : stamp(k - 1, s_cursor[i]);
-            const float angle = __fmul_rn(flip_deg[k], 0.017453292519943295f);
+            const float deg = flip_deg[k];
+            if (signs != nullptr) signs[k] = sign_of(deg);
+            const float angle = __fmul_rn(deg, 0.017453292519943295f);
             const float played = __fmul_rn(6.283185307179586f, fabsf(__fmul_rn(angle, 0.15915493667125702f)));
             float* d = dur_ev + 1 + 4 * k;
             float* f = flip_ev + 1 + 4 * k;
@@ -482,8 +487,7 @@ __global__ void mrf_stream_vjp_kernel(const float* __restrict__ flip_deg, int64_
     const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (k >= n) return;
     if (g_flip != nullptr) {
-        const float f = flip_deg[k];
-        const float sign = f > 0.f ? 1.f : (f < 0.f ? -1.f : (f == 0.f ? 0.f : f));
+        const float sign = sign_of(flip_deg[k]);
         float g = g_flip_ev != nullptr ? g_flip_ev[1 + 4 * k] : 0.f;
         g = __fmul_rn(__fmul_rn(g, 6.283185307179586f), sign);
         g_flip[k] = __fmul_rn(__fmul_rn(g, 0.15915493667125702f), 0.017453292519943295f);
@@ -543,6 +547,15 @@ extern "C" int tsg_mrf_stream(const tsg_program* tmpl, const float* flip_deg, co
                               int64_t tr_count, float tr_value, int64_t pulses, float start_s,
                               float first_stamp_us, float* flip_rad, float* duration_s,
                               void* device_ops, void* stream) {
+    return tsg_mrf_stream_signs(tmpl, flip_deg, tr_ms, tr_count, tr_value, pulses, start_s,
+                                first_stamp_us, flip_rad, duration_s, device_ops, nullptr, stream);
+}
+
+extern "C" int tsg_mrf_stream_signs(const tsg_program* tmpl, const float* flip_deg,
+                                    const float* tr_ms, int64_t tr_count, float tr_value,
+                                    int64_t pulses, float start_s, float first_stamp_us,
+                                    float* flip_rad, float* duration_s, void* device_ops,
+                                    float* signs, void* stream) {
     if (!tmpl) return fail(TSG_ERR_ARGUMENT, "null program");
     if (pulses < 1 || (tr_count != 0 && tr_count != 1 && tr_count != pulses))
         return fail(TSG_ERR_ARGUMENT, "one TR, or one for each pulse");
@@ -553,7 +566,7 @@ extern "C" int tsg_mrf_stream(const tsg_program* tmpl, const float* flip_deg, co
         return fail(TSG_ERR_ARGUMENT, "null stream buffer");
     mrf_stream_kernel<<<1, kStreamThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         flip_deg, tr_ms, tr_count, tr_value, pulses, start_s, first_stamp_us, tmpl->d_ops, tmpl->d_src,
-        tmpl->host.ops, flip_rad, duration_s, static_cast<Op*>(device_ops));
+        tmpl->host.ops, flip_rad, duration_s, static_cast<Op*>(device_ops), signs);
     TSG_CUDA(cudaGetLastError());
     return TSG_OK;
 }

@@ -470,25 +470,34 @@ def _stream_in_one_kernel(flip_deg: Any, TR_ms: Any, device: torch.device):
 
 def _mrf_stream_kernel(template: Program, flip: torch.Tensor, tr: torch.Tensor | None,
                        tr_value: float, ti: float):
-    """Flip and duration buffers ``(1, events)`` and the rebound op table of
-    :func:`mrf_stream_on_device`, by one kernel."""
+    """Flip and duration buffers ``(1, events)``, the rebound op table of
+    :func:`mrf_stream_on_device` and the flips' signs, by one kernel."""
     n = flip.numel()
     both = torch.empty((2, 1, 1 + 4 * n), dtype=torch.float32, device=flip.device)
+    signs = torch.empty(n, dtype=torch.float32, device=flip.device)
     ops = torch.empty((max(template.ops, 1), 4), dtype=torch.float32, device=flip.device)
-    _native.check(_native.library().tsg_mrf_stream(
+    _native.check(_native.library().tsg_mrf_stream_signs(
         template.handle, flip.data_ptr(), None if tr is None else tr.data_ptr(),
         0 if tr is None else tr.numel(), tr_value, n, float(np.float32(ti)),
         float(np.float32(1e6 * ti)), both[0].data_ptr(), both[1].data_ptr(), ops.data_ptr(),
-        torch.cuda.current_stream(flip.device).cuda_stream))
-    return both[0], both[1], ops
+        signs.data_ptr(), torch.cuda.current_stream(flip.device).cuda_stream))
+    return both[0], both[1], ops, signs
 
 
-def _unmoved(ctx, flip_ev: torch.Tensor, dur_ev: torch.Tensor) -> list[torch.Tensor]:
-    """The event buffers that carry no gradient: of flips where the flips
-    (input 0) are not differentiated, of durations where the TRs (input 1) are
-    not. Left differentiable, each costs the sweep behind it a gradient that
-    nothing takes."""
-    return [ev for ev, moved in zip((flip_ev, dur_ev), ctx.needs_input_grad) if not moved]
+def _keep_signs(ctx, flip_ev: torch.Tensor, dur_ev: torch.Tensor, signs: torch.Tensor,
+                *rest: torch.Tensor) -> None:
+    """What an event function's transpose needs of the flips: their signs, an
+    output of the function so that they are not the caller's tensor (which may
+    change in place before the backward) and still lead back to it. Outputs
+    whose input is not differentiated (the flips, input 0, for the flip buffer
+    and the signs; the TRs, input 1, for the durations) carry no gradient, nor
+    does ``rest``: left differentiable, each would cost the sweep behind it a
+    gradient that nothing takes."""
+    moved = ctx.needs_input_grad
+    still = ([] if moved[0] else [flip_ev, signs]) + ([] if moved[1] else [dur_ev])
+    ctx.mark_non_differentiable(*still, *rest)
+    ctx.set_materialize_grads(False)
+    ctx.save_for_backward(signs)
 
 
 class MrfStream(torch.autograd.Function):
@@ -499,49 +508,40 @@ class MrfStream(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, flip, tr, tr_value, ti, template):
-        got = _mrf_stream_kernel(template, _native.readable(flip.detach()),
-                                 None if tr is None else _native.readable(tr.detach()), tr_value, ti)
-        ctx.mark_non_differentiable(got[2], *_unmoved(ctx, got[0], got[1]))
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(flip)
+        flip_ev, dur_ev, ops, signs = _mrf_stream_kernel(
+            template, _native.readable(flip.detach()),
+            None if tr is None else _native.readable(tr.detach()), tr_value, ti)
+        _keep_signs(ctx, flip_ev, dur_ev, signs, ops)
         ctx.tr_shape = None if tr is None else tr.shape
-        return got
+        return flip_ev, dur_ev, ops, signs
 
     @staticmethod
-    def backward(ctx, g_flip_ev, g_dur_ev, _g_ops):
-        (flip,) = ctx.saved_tensors
-        grads = _stream_transpose(flip, g_flip_ev if ctx.needs_input_grad[0] else None,
-                                  g_dur_ev if ctx.needs_input_grad[1] else None)
-        return grads[0], _summed_to(grads[1], ctx.tr_shape), None, None, None
+    def backward(ctx, g_flip_ev, g_dur_ev, _g_ops, g_signs):
+        (signs,) = ctx.saved_tensors
+        g_flip, g_tr = _stream_transpose(signs, g_flip_ev, g_dur_ev, g_signs)
+        return g_flip, _summed_to(g_tr, ctx.tr_shape), None, None, None
 
 
 class MrfEvents(torch.autograd.Function):
     """The event buffers of a host-built MRF train (one playing), which carry
     the values of the flips (deg) and TRs (ms) already, as a function of
-    these: the buffers as they are, with :class:`MrfStream`'s transpose."""
+    these: the buffers as they are, with :class:`MrfStream`'s transpose. The
+    third output is the transpose's own."""
 
     @staticmethod
     def forward(ctx, flip, tr, flip_ev, dur_ev):
-        ctx.set_materialize_grads(False)
-        ctx.save_for_backward(flip)
-        ctx.tr = None if tr is None else (tr.shape, tr.device, tr.dtype)
-        got = flip_ev.clone(), dur_ev.clone()
-        ctx.mark_non_differentiable(*_unmoved(ctx, *got))
+        ctx.flip, ctx.tr = (None if x is None else (x.shape, x.device, x.dtype) for x in (flip, tr))
+        signs = flip.detach().reshape(-1).to(flip_ev.device).sgn()
+        got = flip_ev.clone(), dur_ev.clone(), signs
+        _keep_signs(ctx, *got)
         return got
 
     @staticmethod
-    def backward(ctx, g_flip_ev, g_dur_ev):
-        (flip,) = ctx.saved_tensors
-        if not ctx.needs_input_grad[0]:
-            g_flip_ev = None
-        if not ctx.needs_input_grad[1]:
-            g_dur_ev = None
-        some = g_flip_ev if g_flip_ev is not None else g_dur_ev
-        if some is None:
-            return (None,) * 4
-        g_flip, g_tr = _stream_transpose(flip.to(some.device), g_flip_ev, g_dur_ev)
+    def backward(ctx, g_flip_ev, g_dur_ev, g_signs):
+        (signs,) = ctx.saved_tensors
+        g_flip, g_tr = _stream_transpose(signs, g_flip_ev, g_dur_ev, g_signs)
         if g_flip is not None:
-            g_flip = g_flip.to(flip.device, flip.dtype)
+            g_flip = g_flip.reshape(ctx.flip[0]).to(ctx.flip[1], ctx.flip[2])
         if g_tr is not None:
             g_tr = _summed_to(g_tr, ctx.tr[0]).to(ctx.tr[1], ctx.tr[2])
         return g_flip, g_tr, None, None
@@ -554,31 +554,33 @@ def _summed_to(g: torch.Tensor | None, shape: torch.Size | None) -> torch.Tensor
     return g.sum().reshape(shape) if shape.numel() == 1 else g.reshape(shape)
 
 
-def _stream_transpose(flip: torch.Tensor, g_flip_ev: torch.Tensor | None,
-                      g_dur_ev: torch.Tensor | None):
+def _stream_transpose(signs: torch.Tensor, g_flip_ev: torch.Tensor | None,
+                      g_dur_ev: torch.Tensor | None, g_signs: torch.Tensor | None):
     """Cotangents of the event buffers (None: not wanted) back onto the flips
     (deg, on the buffers' device) and the per-pulse TRs (ms). Under
-    ``create_graph`` the result depends on the flips through their sign, as the
-    chain of tensor operations did: a second backward finds its way (of zeros)
-    to them also where the sweep's own backward cannot be differentiated."""
-    n = flip.numel()
+    ``create_graph`` the result depends on the flips through their signs, as the
+    chain of tensor operations did: a second backward finds its way (of zeros:
+    ``g_signs`` is worth nothing) to them also where the sweep's own backward
+    cannot be differentiated."""
+    n = signs.numel()
+    g_flip = g_tr = None
     if torch.is_grad_enabled():
-        g_flip = g_tr = None
         if g_flip_ev is not None:
-            played = g_flip_ev[0, 1::4] * (2.0 * torch.pi) * flip.sgn()
+            played = g_flip_ev[0, 1::4] * (2.0 * torch.pi) * signs
             g_flip = torch.deg2rad(played * _HARD_PULSE_AREA)
         if g_dur_ev is not None:
             g_tr = torch.cat((g_dur_ev[0, 5::4] * 1e-3, g_dur_ev.new_zeros(1)))
-        return g_flip, g_tr
-    if g_flip_ev is None and g_dur_ev is None:
-        return None, None
-    ev = [None if g is None else _native.readable(g.to(torch.float32)) for g in (g_flip_ev, g_dur_ev)]
-    out = [None if g is None else torch.empty(n, dtype=torch.float32, device=flip.device) for g in ev]
-    at = _native.readable(flip.detach())
-    _native.check(_native.library().tsg_mrf_stream_vjp(
-        at.data_ptr(), n, *[None if t is None else t.data_ptr() for t in (*ev, *out)],
-        torch.cuda.current_stream(flip.device).cuda_stream))
-    return out
+    elif g_flip_ev is not None or g_dur_ev is not None:
+        ev = [None if g is None else _native.readable(g.to(torch.float32))
+              for g in (g_flip_ev, g_dur_ev)]
+        g_flip, g_tr = (None if g is None else
+                        torch.empty(n, dtype=torch.float32, device=signs.device) for g in ev)
+        _native.check(_native.library().tsg_mrf_stream_vjp(
+            signs.data_ptr(), n, *[None if t is None else t.data_ptr() for t in (*ev, g_flip, g_tr)],
+            torch.cuda.current_stream(signs.device).cuda_stream))
+    if g_flip is None and g_signs is not None:
+        g_flip = torch.zeros_like(signs)
+    return g_flip, g_tr
 
 
 def mrf_stream_with_gradients(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
@@ -591,7 +593,7 @@ def mrf_stream_with_gradients(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
         return None
     ti = float(TI_ms) * 1e-3
     template = _mrf_template(flip_deg.numel(), ti, float(TI_ms), device)
-    flip, duration, ops = MrfStream.apply(
+    flip, duration, ops, _ = MrfStream.apply(
         flip_deg, TR_ms if isinstance(TR_ms, torch.Tensor) else None, plain[2], ti, template)
     return ProgramView(template, ops), flip, duration
 
@@ -608,7 +610,7 @@ def mrf_stream_on_device(flip_deg: torch.Tensor, TR_ms: Any, TI_ms: float,
     one_kernel = _stream_in_one_kernel(flip_deg, TR_ms, device)
     if one_kernel is not None:
         template = _mrf_template(one_kernel[0].numel(), float(TI_ms) * 1e-3, float(TI_ms), device)
-        flip, duration, ops = _mrf_stream_kernel(template, *one_kernel, float(TI_ms) * 1e-3)
+        flip, duration, ops, _ = _mrf_stream_kernel(template, *one_kernel, float(TI_ms) * 1e-3)
         return ProgramView(template, ops), flip, duration
     angles = torch.deg2rad(torch.atleast_1d(flip_deg.detach()).to(device))
     if angles.ndim != 1:

@@ -498,7 +498,7 @@ class MRFSimulator(_EpgSimulator):
             # Reverse mode alone: one transpose instead of a chain of
             # elementwise operations. (The flips are read for their sign.)
             at = flip if _tracked(flip) else flip_ev.new_zeros(n)
-            flip_ev, dur_ev = MrfEvents.apply(at, tr if _tracked(tr) else None, flip_ev, dur_ev)
+            flip_ev, dur_ev, _ = MrfEvents.apply(at, tr if _tracked(tr) else None, flip_ev, dur_ev)
             return flip_ev, dur_ev, phase_ev
         with torch._C._DisableFuncTorch():
             where = _gradient_map_on(n, repetitions, dev)
