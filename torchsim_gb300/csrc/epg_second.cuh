@@ -640,7 +640,20 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
             const float* x = a.traj_rec + (train * NS * n + voxel) * a.outputs + r;
             const float* g = a.seed + (out * jc * a.outputs + r) * seed_stride;
             float* dst = seeds + vv * NI * EC + col;
-            const float x0 = x[0];
+            // With one or two directions all loads come first, so that they are
+            // one wait (3,000 voxels x 300 x 6 states, T1 and T2: 376 and 302 us);
+            // with three the compiler does better where they are used (16,384 x
+            // 300 x 20: 899 and 917 us).
+            constexpr bool kFirst = K < 3;
+            float xs[NS], gs[K];
+            if constexpr (kFirst) {
+#pragma unroll
+                for (int s = 0; s < NS; ++s) xs[s] = x[s * n * a.outputs];
+#pragma unroll
+                for (int k = 0; k < K; ++k) gs[k] = g[int64_t(k) * a.outputs * seed_stride];
+            }
+            auto recorded = [&](int s) { return kFirst ? xs[s] : x[s * n * a.outputs]; };
+            const float x0 = recorded(0);
             const float g0 = a.seed0 ? seed_sign * a.seed0[(out * a.outputs + r) * seed_stride] : 0.f;
             // The M0 derivative is F+[0] itself: its seed acts unscaled.
             float add0 = g0 * m0, m0_sum = g0 * x0;
@@ -648,13 +661,13 @@ __global__ void __launch_bounds__(32 * kSecondWarps) second_reverse_kernel(const
                 add0 = fmaf(seed_sign, g[int64_t(K) * a.outputs * seed_stride], add0);
 #pragma unroll
             for (int k = 0; k < K; ++k) {
-                const float gk = seed_sign * g[int64_t(k) * a.outputs * seed_stride];
+                const float gk = seed_sign * (kFirst ? gs[k] : g[int64_t(k) * a.outputs * seed_stride]);
                 if (!HOT) {
                     add0 = fmaf(gk, dm0[k], add0);
                     dst[(NS + 1 + k) * EC] = gk * x0;
                 }
                 dst[(k + 1) * EC] = gk * m0;
-                m0_sum = fmaf(gk, x[(k + 1) * n * a.outputs], m0_sum);
+                m0_sum = fmaf(gk, recorded(k + 1), m0_sum);
             }
             dst[0] = add0;
             dst[NS * EC] = m0_sum;
